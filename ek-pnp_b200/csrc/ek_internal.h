@@ -186,6 +186,9 @@ cudaError_t make_pop_tensor_map(int storage, const void *pops, int nxp, int ny, 
 cudaError_t launch_step_tma(const Chan &c, int storage, const void *map, const void *src, void *dst, double *fields,
                             bool first, bool explicit_e, bool moments, int sbuf, int *err, long long wait_cycles,
                             cudaStream_t s);
+// map_out: a CUtensorMap over a row-major BF16 matrix (ld elements a row, 16-byte
+// aligned rows), boxes of box_rows x box_cols with 128-byte swizzle.
+cudaError_t make_matrix_tensor_map(const void *p, int rows, int cols, int ld, int box_rows, int box_cols, void *map_out);
 inline size_t pop_elem_bytes(int storage) { return storage == EK_STORE_F64 ? 8 : (storage == EK_STORE_F32 ? 4 : 2); }
 
 // ---- Poisson (ek_poisson.cu) ----

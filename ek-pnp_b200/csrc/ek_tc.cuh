@@ -1,13 +1,12 @@
 // ek_tc.cuh -- sm_100a tensor-core primitives (tcgen05 with TMEM
 // accumulators) and CTA-local mbarriers, as inline PTX.
 //
-// Shared-memory operands use the canonical K-major layout without swizzle:
-// the tile is cut into "core matrices" of 8 rows x 16 bytes (8 bf16), each
-// stored as 128 contiguous bytes (row r at byte 16 r).  In a tile of R rows
-// and KC columns the core matrix of row group g and column group c sits at
-// byte (g * KC/8 + c) * 128, so neighbours along K are 128 bytes apart (the
-// descriptor's leading-dimension byte offset) and neighbours along M/N are
-// KC/8 * 128 bytes apart (the stride-dimension byte offset).
+// Shared-memory operands use the K-major layout with 128-byte swizzle, as TMA
+// writes it: rows of 64 bf16 (128 bytes), 8 rows to a 1024-byte atom whose
+// 16-byte vectors are XOR-ed with the row's index mod 8; atoms follow one
+// another along M/N (the descriptor's stride-dimension byte offset, 1024).
+// The 16 K-elements of one MMA are 32 bytes along the row, reached by moving
+// the descriptor's start address.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -20,6 +19,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)_
 // ---- mbarrier -------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+// The phase's one arrival, and the bytes that TMA copies will add to it.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
@@ -59,9 +62,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Generic-proxy shared-memory writes -> visible to the tensor cores.
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 // 32 lanes x 8 consecutive 32-bit columns: thread t of the warp gets lane
 // (taddr lane + t), columns taddr.col .. +7.  The wait is in the same
 // statement so no use of the registers can move above it.
@@ -78,14 +78,16 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float v[8]) {
 }
 
 // ---- MMA ------------------------------------------------------------------
-// Shared-memory matrix descriptor: start address, leading- and stride-
-// dimension byte offsets (all >> 4), descriptor version 1 (bits 46-47), no
-// swizzle (layout type 0, bits 61-63), base offset 0.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+// Shared-memory matrix descriptor: start address and stride-dimension byte
+// offset (both >> 4; the leading-dimension offset is not used by a tile one
+// swizzle row wide), descriptor version 1 (bits 46-47), 128-byte swizzle
+// (layout type 2, bits 61-63), base offset 0 (atoms 1024-byte aligned).
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
     uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
     d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
     return d;
 }
 // Instruction descriptor of kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16
