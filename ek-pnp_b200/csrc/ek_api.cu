@@ -472,7 +472,9 @@ int ek_create(const ek_params *p, ek_ctx **out) {
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { free_ctx(c); return cuda_fail(e, "stream create"); }
     c->own_stream = true;
-    c->nxp = round_up(p->nx, 32);
+    // rows start 128-byte aligned in FP32, but those of the narrowest channels: a
+    // row of 16 columns padded to 32 would double the memory its nodes take
+    c->nxp = p->nx <= 16 ? 16 : round_up(p->nx, 32);
     c->plane = (size_t)p->ny * c->nxp;
     c->n = p->ny - 2;
     c->mp = round_up(p->nx / 2 + 1, 16);
@@ -528,7 +530,6 @@ int ek_create(const ek_params *p, ek_ctx **out) {
     if (e == cudaSuccess) e = launch_rates(*p, c->rates_dev, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&c->rates, c->rates_dev, sizeof(Rates), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e == cudaSuccess) e = poisson_set_smem_limits();
     if (e != cudaSuccess) { free_ctx(c); return cuda_fail(e, "context set-up"); }
     if (p->storage != EK_STORE_F64) {
         c->tma_ok = make_pop_tensor_map(p->storage, c->pops[0], c->nxp, p->ny, &c->tmaps[0]) == cudaSuccess &&
@@ -572,6 +573,8 @@ int ek_create(const ek_params *p, ek_ctx **out) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) { free_ctx(c); return cuda_fail(e, "FP32 Poisson set-up"); }
     }
+    e = poisson_set_smem_limits(c->pp);
+    if (e != cudaSuccess) { free_ctx(c); return cuda_fail(e, "context set-up"); }
     refresh_chan(c);
     int rcl = upload_lift(c);
     if (rcl != EK_OK) { free_ctx(c); return rcl; }
@@ -856,20 +859,24 @@ int ek_step(ek_ctx *c, int32_t nsteps) {
     const bool every = (c->p.flags & EK_FLAG_MOMENTS_EVERY_STEP) != 0;
     int rcs = split_if_stale(c);
     if (rcs != EK_OK) return rcs;
+    const bool small = (size_t)c->p.nx * c->p.ny <= PDL_NODES && !(c->p.flags & EK_FLAG_EXPLICIT_E);
+    bool rebased = false;  // the step before ended with a re-basing of the populations
     for (int32_t i = 0; i < nsteps; ++i) {
         const bool ee = c->explicit_e_once || (c->p.flags & EK_FLAG_EXPLICIT_E);
         const bool rebase = shifted(c) && c->rebase_every > 0 && (c->steps + 1) % c->rebase_every == 0;
         const bool mom = every || (i == nsteps - 1 && c->last_moments) || rebase;
+        const int chain = !small ? CHAIN_NONE : (i == 0 || rebased ? CHAIN_FIRST : CHAIN_NEXT);
+        rebased = rebase;
         int rc0 = timed(c, 0, "LBM step kernel", [&] {
             if (c->p.storage == EK_STORE_F64)
                 return launch_step_f64(c->chan, (const double *)c->pops[c->cur], (double *)c->pops[c->cur ^ 1],
-                                       c->fields, c->state_pre, ee, mom, c->stream);
+                                       c->fields, c->state_pre, ee, mom, chain, c->stream);
             if (use_tma(c))
                 return launch_step_tma(c->chan, c->p.storage, &c->tmaps[c->cur], c->pops[c->cur],
                                        c->pops[c->cur ^ 1], c->fields, c->state_pre, ee, mom, c->cur, c->err_dev,
                                        c->wait_cycles, c->stream);
             return launch_step_shifted(c->chan, c->p.storage, c->pops[c->cur], c->pops[c->cur ^ 1], c->fields,
-                                       c->state_pre, ee, mom, c->cur, c->stream);
+                                       c->state_pre, ee, mom, c->cur, chain, c->stream);
         });
         if (rc0 != EK_OK) return rc0;
         c->cur ^= 1;

@@ -44,7 +44,7 @@ constexpr int REFS_TPB = 256;
 
 // ---- kernels ---------------------------------------------------------------
 
-// Persistent LBM kernel over the tile list; TXB threads = tile width x rows.
+// Persistent LBM kernel over the tile list; TXB threads = half a tile's width x rows.
 // MINB: blocks per SM the register allocation must allow (the block shapes,
 // kShapes below, pair a width with it).
 // Tiles are handed out from a queue, TILE_CHUNK consecutive tiles (same
@@ -63,27 +63,35 @@ batch_lbm(const ChanF *__restrict__ chans, const S *const *__restrict__ src, S *
     __shared__ ChanF ks;
     __shared__ int claim;
     int cur = -1;
-    for (;;) {
-        if (threadIdx.x == 0) claim = atomicAdd(queue, TILE_CHUNK);
-        __syncthreads();
-        const int t0 = claim;
-        if (t0 >= ntiles) break;  // the same for every thread of the block
+    if (threadIdx.x == 0) claim = atomicAdd(queue, TILE_CHUNK);
+    __syncthreads();
+    int t0 = claim;
+    while (t0 < ntiles) {  // the same for every thread of the block
         const int t1 = min(ntiles, t0 + TILE_CHUNK);
+        int next = 0;
+        if (threadIdx.x == 0) next = atomicAdd(queue, TILE_CHUNK);  // the next claim, while this one is worked on
+        int4 tl = tiles[t0];  // {channel, y0, x0, width}
         for (int t = t0; t < t1; ++t) {
-            const int4 tl = tiles[t];  // {channel, y0, x0, width}
+            const int4 after = t + 1 < t1 ? tiles[t + 1] : tl;
             if (tl.x != cur) {
                 __syncthreads();
-                if (threadIdx.x == 0) ks = chans[tl.x];
+                // every thread copies its share of the channel's constants
+                for (int i = threadIdx.x; i < (int)(sizeof(ChanF) / 4); i += TXB)
+                    ((uint32_t *)&ks)[i] = __ldg((const uint32_t *)&chans[tl.x] + i);
                 __syncthreads();
                 cur = tl.x;
             }
-            const int r = threadIdx.x / tl.w;
-            const int x = tl.z + (threadIdx.x - r * tl.w), y = tl.y + r;
-            if (r < TXB / tl.w && x < ks.nx && y < ks.ny)
-                // 32-bit indexing: batched channels are at most 4096 x 8194 (ek_batch_create)
-                node_shifted<S, FIRST, EE, uint32_t>(ks, src[cur], dst[cur], fields[cur], x, y, mom, sbuf);
+            // two columns a thread (the width is even: nx a power of two from 16 on)
+            const int half = tl.w >> 1, r = threadIdx.x / half;
+            const int x = tl.z + 2 * (threadIdx.x - r * half), y = tl.y + r;
+            if (r < TXB / half && x < ks.nx && y < ks.ny)
+                node_shifted<S, FIRST, EE, float2>(ks, src[cur], dst[cur], fields[cur], x, y, mom, sbuf, false);
+            tl = after;
         }
-        __syncthreads();  // every thread has read `claim` before thread 0 claims again
+        __syncthreads();  // every thread has read `claim`
+        if (threadIdx.x == 0) claim = next;
+        __syncthreads();
+        t0 = claim;
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -112,11 +120,14 @@ batch_rebase(const ChanF *__restrict__ chans, S *const *__restrict__ pops, float
              const int4 *__restrict__ tiles) {
     const int4 tl = tiles[blockIdx.x];
     const ChanF &k = chans[tl.x];
-    const int r = threadIdx.x / tl.w;
-    const int x = tl.z + (threadIdx.x - r * tl.w), y = tl.y + r;
-    if (r >= TXB / tl.w || x >= k.nx || y >= k.ny) return;  // each node of the tile once
+    const int half = tl.w >> 1, r = threadIdx.x / half;
+    const int x = tl.z + 2 * (threadIdx.x - r * half), y = tl.y + r;
+    if (r >= TXB / half || x >= k.nx || y >= k.ny) return;  // each pair of the tile once
     S *base = pops[tl.x] + (size_t)y * k.nxp + x;
-    for (int pl = 0; pl < 27; ++pl) rebase_dev<S>(base + (size_t)pl * k.plane, pl, k.ny, y, k.kref, spare[tl.x]);
+    for (int pl = 0; pl < 27; ++pl) {
+        rebase_dev<S>(base + (size_t)pl * k.plane, pl, k.ny, y, k.kref, spare[tl.x]);
+        rebase_dev<S>(base + (size_t)pl * k.plane + 1, pl, k.ny, y, k.kref, spare[tl.x]);
+    }
 }
 
 // The spare rows become the current ones: item {channel, row}, 3 species.
@@ -152,16 +163,14 @@ cudaError_t lbm_t(const ChanF *chans, const void *src, void *dst, double *const 
 }
 
 // Block shapes of the batched LBM kernel: threads, the widest tile (a tile is
-// min(width, nx) columns by threads / that many rows) and the blocks per SM
-// that the register allocation must allow.  At 72 registers (7 blocks of 128,
-// 14 of 64) the batched node update spills a little; 10 blocks of 64, 5 of
-// 128 and 3 of 256 do not.  Narrower tiles than threads give 2-D tiles whose
-// rows share their pulled neighbours in L1.
+// min(width, nx) columns, two a thread, by as many rows as the threads make)
+// and the blocks per SM that the register allocation must allow: 512 threads
+// of 128 registers, which the update of two nodes takes without spilling.
 struct Shape {
     int threads, width, minb;
 };
-constexpr Shape kShapes[EK_BATCH_SHAPES] = {{64, 64, 10},   {128, 128, 5}, {128, 128, 7},
-                                             {256, 256, 3}, {256, 64, 3},  {256, 128, 3}};
+constexpr Shape kShapes[EK_BATCH_SHAPES] = {{64, 64, 8},   {128, 128, 4}, {128, 256, 4},
+                                             {256, 256, 2}, {256, 64, 2},  {256, 512, 2}};
 
 #define EK_SHAPE_CASES(F) F(0) F(1) F(2) F(3) F(4) F(5)
 static_assert(EK_BATCH_SHAPES == 6, "one case per shape");
@@ -244,7 +253,7 @@ struct ek_batch {
     int ntiles = 0, shape = 1, txb = 128, grid = 0;  // kShapes[shape], txb = its threads
     int *d_queue = nullptr;          // LBM tile queue: next tile, finished blocks (zero between launches)
     int2 *d_pairs = nullptr;         // Poisson row-pair items
-    int npairs = 0;
+    int npairs = 0, row_block = 256;  // items, threads of a block (batch_row_block)
     int3 *d_modes = nullptr;         // Poisson x-mode items
     int nmodes = 0;
     int2 *d_rows = nullptr;          // {channel, row} of every row
@@ -291,7 +300,7 @@ void release_graph(ek_batch *b) {
     b->graph_cur = -1;
 }
 
-// LBM tiles of a block shape: min(width, nx) columns by threads / that many
+// LBM tiles of a block shape: min(width, nx) columns by 2 threads / that many
 // rows; the grid is one wave.
 int build_tiles(ek_batch *b, int shape) {
     if (shape < 0 || shape >= EK_BATCH_SHAPES) return ek::ctx_fail(EK_ERR_INVALID, "no such block shape");
@@ -301,7 +310,7 @@ int build_tiles(ek_batch *b, int shape) {
         if (!b->active[i]) continue;
         const ek_params &p = b->ch[i]->p;
         const int w = std::min(kShapes[shape].width, p.nx);
-        const int rows = txb / w;
+        const int rows = 2 * txb / w;
         for (int y = 0; y < p.ny; y += rows)
             for (int x0 = 0; x0 < p.nx; x0 += w) tiles.push_back(make_int4((int)i, y, x0, w));
     }
@@ -342,6 +351,9 @@ int build_tables(ek_batch *b) {
     b->poisson_f32 = f32;
     if (!f32)
         return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batched channels run the FP32 Poisson form (EK_OPT_POISSON 0 or 2)");
+    int nx_max = 0;
+    for (ek_ctx *c : b->ch) nx_max = std::max(nx_max, (int)c->p.nx);
+    b->row_block = batch_row_block(nx_max);
     size_t field_bytes = 0;  // right-hand side + psi (FP32 planes) of the stepping channels
     for (size_t i = 0; i < b->ch.size(); ++i)
         if (b->active[i]) field_bytes += 2 * b->ch[i]->plane * sizeof(float);
@@ -363,7 +375,7 @@ int build_tables(ek_batch *b) {
         kq.push_back(make_int4(c->kq[0], c->kq[1], c->kq[2], 0));
         const int nx = c->p.nx, n = c->pp.n;
         if (b->active[i]) {
-            const int per = 256 / (nx >> 4);
+            const int per = b->row_block / (nx >> 4);
             for (int q = 0; q < (n + 1) / 2; q += per) pairs.push_back(make_int2((int)i, q));
             const int M = poisson_tridiag_modes(n);
             // the zero mode in FP64 (an item with 0 modes per block); modes 1.. in FP32
@@ -413,11 +425,11 @@ int launch_step(ek_batch *b, bool first, bool ee, bool mom) {
                         : lbm_s<float>(b->shape, b->d_chanf, src, dst, b->d_fields, b->d_tiles, b->ntiles,
                                        b->d_queue, b->grid, first, ee, mom, b->cur, b->stream);
     EK_BCUDA(e, "batch LBM kernel");
-    EK_BCUDA(batch_poisson(0, b->d_plans, b->d_chan, b->d_fields, b->d_pairs, b->npairs, false, b->stream),
+    EK_BCUDA(batch_poisson(0, b->d_plans, b->d_chan, b->d_fields, b->d_pairs, b->npairs, b->row_block, false, b->stream),
              "batch rows");
     EK_BCUDA(batch_tridiag_f32(b->d_plans, b->d_modes, b->nmodes, b->stream), "batch modes");
     // the FP64 psi planes follow on the steps that write the moments
-    EK_BCUDA(batch_poisson(2, b->d_plans, b->d_chan, b->d_fields, b->d_pairs, b->npairs, mom, b->stream),
+    EK_BCUDA(batch_poisson(2, b->d_plans, b->d_chan, b->d_fields, b->d_pairs, b->npairs, b->row_block, mom, b->stream),
              "batch rows");
     b->launches += launches_per_step(b);
     b->cur ^= 1;
@@ -511,7 +523,6 @@ int ek_batch_create(const ek_params *params, int32_t count, ek_batch **out) {
             return ek::ctx_fail(EK_ERR_INVALID, "all channels of a batch need one storage mode");
         if (p.storage != EK_STORE_F32 && p.storage != EK_STORE_F16)
             return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batches use FP32 or FP16 storage");
-        static_assert(index32_fits((size_t)4096 * 8194), "batched channels use 32-bit indexing");
         if (!pow2(p.nx) || p.nx < 16 || p.nx > 4096)
             return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batched channels need nx a power of two in [16, 4096]");
         if (p.flags & EK_FLAG_EXPLICIT_E) return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batches derive E from psi");
@@ -541,6 +552,7 @@ int ek_batch_create(const ek_params *params, int32_t count, ek_batch **out) {
         b->nodes += (int64_t)params[i].nx * params[i].ny;
     }
     int rc = build_tables(b);
+    if (rc == EK_OK && (e = batch_set_smem_limits(b->row_block)) != cudaSuccess) rc = cuda_err(e, "row kernels");
     if (rc == EK_OK) rc = build_tiles(b, 1);
     if (rc != EK_OK) {
         ek_batch_destroy(b);

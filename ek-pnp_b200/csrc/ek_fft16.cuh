@@ -1,5 +1,6 @@
-// ek_fft32.cuh -- FP32 complex transforms of 2^K points held by 2^(K-4)
-// threads (16 points a thread), for the row passes of the FP32 Poisson form.
+// ek_fft16.cuh -- complex transforms of 2^K points held by 2^(K-4) threads (16
+// points a thread), FP32 (float2) and FP64 (double2), for the row passes of
+// the Poisson solve.
 //
 // Forward: decimation in frequency, radix-16 passes from the top index bit
 // down (bits [b, b+4), b = K-4, K-8, ...), then one radix-2^(K mod 4) pass on
@@ -16,20 +17,31 @@
 // XOR, so an element's address is its group base's address XOR a
 // compile-time constant.  Every pass writes back onto the slots its group
 // read, so one barrier per pass suffices.
-// The pass twiddles come from per-pass tables laid out f-major, kb-minor:
-// the 32 lanes of a warp read consecutive entries.
+// FP32 sums of complex values are packed instructions (one issue slot for
+// both parts).  FP32 pass twiddles come from per-pass tables laid out f-major,
+// kb-minor (the 32 lanes of a warp read consecutive entries); FP64 ones from
+// the table of nx-th roots.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace ek {
-namespace fft32 {
+namespace fft16 {
 
-__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
-constexpr float C1 = 0.92387953251128674f;  // cos(pi/8)
-constexpr float S1 = 0.38268343236508977f;  // sin(pi/8)
-constexpr float R2 = 0.70710678118654752f;  // cos(pi/4)
+template <typename C> struct RealOf;
+template <> struct RealOf<float2> { using type = float; };
+template <> struct RealOf<double2> { using type = double; };
+template <typename C> using Real = typename RealOf<C>::type;
+__device__ __forceinline__ float2 mk(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 mk(double a, double b) { return make_double2(a, b); }
+
+constexpr double C1 = 0.92387953251128674;  // cos(pi/8)
+constexpr double S1 = 0.38268343236508977;  // sin(pi/8)
+constexpr double R2 = 0.70710678118654752;  // cos(pi/4)
 
 __host__ __device__ constexpr int brev4(int f) { return ((f & 1) << 3) | ((f & 2) << 1) | ((f & 4) >> 1) | ((f & 8) >> 3); }
 __host__ __device__ constexpr int brevq(int f, int q) { return brev4(f) >> (4 - q); }
@@ -39,56 +51,52 @@ __host__ __device__ constexpr int lin(int v) { return v ^ (((v >> 4) ^ (v >> 8))
 __device__ __forceinline__ int swz_base(int i, int p) { return i ^ (((i >> 4) ^ (i >> 8) ^ p) & 15); }
 
 // z * exp(-/+ 2 pi i m/16) (forward: minus), m a compile-time constant
-template <bool INV, int M>
-__device__ __forceinline__ float2 w16(float2 z) {
+template <bool INV, int M, typename C>
+__device__ __forceinline__ C w16(C z) {
+    using R = Real<C>;
     constexpr int m = M & 15;
     if constexpr (m == 0) {
         return z;
     } else if constexpr (m == 8) {
-        return make_float2(-z.x, -z.y);
+        return mk(-z.x, -z.y);
     } else if constexpr (m == 4 || m == 12) {
         // forward m = 4: -i z; m = 12: +i z; inverse the other way round
         constexpr bool minus_i = (m == 4) != INV;
-        return minus_i ? make_float2(z.y, -z.x) : make_float2(-z.y, z.x);
+        return minus_i ? mk(z.y, -z.x) : mk(-z.y, z.x);
     } else if constexpr ((m & 1) == 0) {
         // (c + i s) with |c| = |s| = cos(pi/4)
-        constexpr float c = (m == 2 || m == 14) ? R2 : -R2;
-        constexpr float s0 = (m == 2 || m == 6) ? -R2 : R2;  // forward imaginary part
-        constexpr float s = INV ? -s0 : s0;
+        constexpr R c = (R)((m == 2 || m == 14) ? R2 : -R2);
+        constexpr R s0 = (R)((m == 2 || m == 6) ? -R2 : R2);  // forward imaginary part
+        constexpr R s = INV ? -s0 : s0;
         constexpr bool same = (c > 0) == (s > 0);
         // z (c + i s) = (c z.x - s z.y, s z.x + c z.y)
-        if constexpr (same) return make_float2(c * (z.x - z.y), c * (z.x + z.y));
-        else return make_float2(c * (z.x + z.y), c * (z.y - z.x));
+        if constexpr (same) return mk(c * (z.x - z.y), c * (z.x + z.y));
+        else return mk(c * (z.x + z.y), c * (z.y - z.x));
     } else {
-        constexpr float cs[8] = {1.0f, C1, R2, S1, 0.0f, -S1, -R2, -C1};   // cos(pi j/8), j < 8
-        constexpr float sn[8] = {0.0f, S1, R2, C1, 1.0f, C1, R2, S1};      // sin(pi j/8), j < 8
-        constexpr float c = m < 8 ? cs[m] : -cs[m - 8];
-        constexpr float s0 = m < 8 ? -sn[m] : sn[m - 8];  // forward: -sin(pi m/8)
-        constexpr float s = INV ? -s0 : s0;
-        return make_float2(z.x * c - z.y * s, z.x * s + z.y * c);
+        constexpr double cs[8] = {1.0, C1, R2, S1, 0.0, -S1, -R2, -C1};   // cos(pi j/8), j < 8
+        constexpr double sn[8] = {0.0, S1, R2, C1, 1.0, C1, R2, S1};      // sin(pi j/8), j < 8
+        constexpr R c = (R)(m < 8 ? cs[m] : -cs[m - 8]);
+        constexpr R s0 = (R)(m < 8 ? -sn[m] : sn[m - 8]);  // forward: -sin(pi m/8)
+        constexpr R s = INV ? -s0 : s0;
+        return mk(z.x * c - z.y * s, z.x * s + z.y * c);
     }
 }
 
 // 4-point DFT in place: (a, b, c, d) -> (X0, X1, X2, X3)
-template <bool INV>
-__device__ __forceinline__ void dft4(float2 &a, float2 &b, float2 &c, float2 &d) {
-    const float2 s0 = a + c, d0 = a - c, s1 = b + d, d1 = b - d;
-    const float2 id1 = make_float2(-d1.y, d1.x);  // i d1
+template <bool INV, typename C>
+__device__ __forceinline__ void dft4(C &a, C &b, C &c, C &d) {
+    const C s0 = a + c, d0 = a - c, s1 = b + d, d1 = b - d;
     a = s0 + s1;
     c = s0 - s1;
-    if (INV) {
-        b = d0 + id1;
-        d = d0 - id1;
-    } else {
-        b = d0 - id1;
-        d = d0 + id1;
-    }
+    const C plus = mk(d0.x - d1.y, d0.y + d1.x), minus = mk(d0.x + d1.y, d0.y - d1.x);  // d0 +- i d1
+    b = INV ? plus : minus;
+    d = INV ? minus : plus;
 }
 
 // 16-point DFT in place; output f sits at x[out16(f)]
 __host__ __device__ constexpr int out16(int f) { return 4 * (f & 3) + (f >> 2); }
-template <bool INV>
-__device__ __forceinline__ void dft16(float2 (&x)[16]) {
+template <bool INV, typename C>
+__device__ __forceinline__ void dft16(C (&x)[16]) {
     // n = n1 + 4 n2, f = 4 f1 + f2: 4-point DFTs over n2, twiddles W16^(n1 f2),
     // 4-point DFTs over n1
 #pragma unroll
@@ -108,10 +116,10 @@ __device__ __forceinline__ void dft16(float2 (&x)[16]) {
 
 // 2^Q-point DFT (Q = 1..3) in place on x[o .. o + 2^Q); output f at x[o + outq<Q>(f)]
 template <int Q> __host__ __device__ constexpr int outq(int f) { return Q == 3 ? 2 * (f & 3) + (f >> 2) : f; }
-template <bool INV, int Q>
-__device__ __forceinline__ void dftq(float2 *x) {
+template <bool INV, int Q, typename C>
+__device__ __forceinline__ void dftq(C *x) {
     if constexpr (Q == 1) {
-        const float2 a = x[0], b = x[1];
+        const C a = x[0], b = x[1];
         x[0] = a + b;
         x[1] = a - b;
     } else if constexpr (Q == 2) {
@@ -126,7 +134,7 @@ __device__ __forceinline__ void dftq(float2 *x) {
         x[7] = w16<INV, 6>(x[7]);
 #pragma unroll
         for (int f2 = 0; f2 < 4; ++f2) {
-            const float2 a = x[2 * f2], b = x[2 * f2 + 1];
+            const C a = x[2 * f2], b = x[2 * f2 + 1];
             x[2 * f2] = a + b;
             x[2 * f2 + 1] = a - b;
         }
@@ -165,11 +173,20 @@ __device__ __forceinline__ float2 ldtw(const float2 *p) {
     return v;
 }
 
-__device__ __forceinline__ float2 mulw(float2 a, float2 w) {
-    return make_float2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+template <typename C> __device__ __forceinline__ C mulw(C a, C w) {
+    return mk(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
 }
-__device__ __forceinline__ float2 mulw_conj(float2 a, float2 w) {
-    return make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
+template <typename C> __device__ __forceinline__ C mulw_conj(C a, C w) {
+    return mk(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
+}
+
+// Twiddle exp(-2 pi i kb f / 2^(b+4)) of full pass I (b = Shape::bit(I)):
+// FP32 from the pass tables, FP64 from the nx-th roots.
+template <int K, int I> __device__ __forceinline__ float2 pass_tw(const float2 *__restrict__ t, int f, int kb) {
+    return ldtw(t + Shape<K>::off(I) + ((f - 1) << Shape<K>::bit(I)) + kb);
+}
+template <int K, int I> __device__ __forceinline__ double2 pass_tw(const double2 *__restrict__ t, int f, int kb) {
+    return __ldg(t + ((kb * f) << (K - 4 - Shape<K>::bit(I))));
 }
 
 // Thread t's group of full pass I: first element and in-group offset kb.
@@ -181,25 +198,24 @@ __device__ __forceinline__ void group(int t, int &base, int &kb) {
 }
 
 // Forward full pass I on x (its group's elements, v = 0..15), result into s.
-template <int K, int I>
-__device__ __forceinline__ void fwd_pass_store(float2 (&x)[16], float2 *s, int t, int p,
-                                               const float2 *__restrict__ twp) {
+template <int K, int I, typename C>
+__device__ __forceinline__ void fwd_pass_store(C (&x)[16], C *s, int t, int p,
+                                               const C *__restrict__ twp) {
     constexpr int b = Shape<K>::bit(I);
     int base, kb;
     group<K, I>(t, base, kb);
     dft16<false>(x);
     const int sb = swz_base(base, p);
     if constexpr (b > 0) {
-        const float2 *tp = twp + Shape<K>::off(I) + kb;
 #pragma unroll
-        for (int f = 1; f < 16; ++f) x[out16(f)] = mulw(x[out16(f)], ldtw(tp + ((f - 1) << b)));
+        for (int f = 1; f < 16; ++f) x[out16(f)] = mulw(x[out16(f)], pass_tw<K, I>(twp, f, kb));
     }
 #pragma unroll
     for (int f = 0; f < 16; ++f) s[sb ^ lin(brev4(f) << b)] = x[out16(f)];
 }
 
-template <int K, int I>
-__device__ __forceinline__ void fwd_pass_load(float2 (&x)[16], const float2 *s, int t, int p) {
+template <int K, int I, typename C>
+__device__ __forceinline__ void fwd_pass_load(C (&x)[16], const C *s, int t, int p) {
     constexpr int b = Shape<K>::bit(I);
     int base, kb;
     group<K, I>(t, base, kb);
@@ -209,10 +225,10 @@ __device__ __forceinline__ void fwd_pass_load(float2 (&x)[16], const float2 *s, 
 }
 
 // Forward passes 2..NF and the partial pass, after pass 1 stored into s.
-template <int K, int I>
-__device__ __forceinline__ void fwd_rest(float2 *s, int t, int p, const float2 *__restrict__ twp) {
+template <int K, int I, typename C>
+__device__ __forceinline__ void fwd_rest(C *s, int t, int p, const C *__restrict__ twp) {
     if constexpr (I <= Shape<K>::NF) {
-        float2 x[16];
+        C x[16];
         fwd_pass_load<K, I>(x, s, t, p);  // a pass writes back onto its group's own slots
         fwd_pass_store<K, I>(x, s, t, p, twp);
         __syncthreads();
@@ -220,7 +236,7 @@ __device__ __forceinline__ void fwd_rest(float2 *s, int t, int p, const float2 *
     } else if constexpr (Shape<K>::Q > 0) {
         constexpr int Q = Shape<K>::Q, R = 1 << Q;
         const int sb = swz_base(t << 4, p);
-        float2 x[16];
+        C x[16];
 #pragma unroll
         for (int v = 0; v < 16; ++v) x[v] = s[sb ^ v];
 #pragma unroll
@@ -235,28 +251,27 @@ __device__ __forceinline__ void fwd_rest(float2 *s, int t, int p, const float2 *
 
 // Inverse full pass I: conjugate twiddles, inverse DFT; x ends in natural
 // order of v (element base | v << b).
-template <int K, int I>
-__device__ __forceinline__ void inv_pass_load(float2 (&x)[16], const float2 *s, int t, int p,
-                                              const float2 *__restrict__ twp) {
+template <int K, int I, typename C>
+__device__ __forceinline__ void inv_pass_load(C (&x)[16], const C *s, int t, int p,
+                                              const C *__restrict__ twp) {
     constexpr int b = Shape<K>::bit(I);
     int base, kb;
     group<K, I>(t, base, kb);
     const int sb = swz_base(base, p);
-    float2 z[16];
+    C z[16];
 #pragma unroll
     for (int f = 0; f < 16; ++f) z[f] = s[sb ^ lin(brev4(f) << b)];
     if constexpr (b > 0) {
-        const float2 *tp = twp + Shape<K>::off(I) + kb;
 #pragma unroll
-        for (int f = 1; f < 16; ++f) z[f] = mulw_conj(z[f], ldtw(tp + ((f - 1) << b)));
+        for (int f = 1; f < 16; ++f) z[f] = mulw_conj(z[f], pass_tw<K, I>(twp, f, kb));
     }
     dft16<true>(z);
 #pragma unroll
     for (int v = 0; v < 16; ++v) x[v] = z[out16(v)];
 }
 
-template <int K, int I>
-__device__ __forceinline__ void inv_pass_store(const float2 (&x)[16], float2 *s, int t, int p) {
+template <int K, int I, typename C>
+__device__ __forceinline__ void inv_pass_store(const C (&x)[16], C *s, int t, int p) {
     constexpr int b = Shape<K>::bit(I);
     int base, kb;
     group<K, I>(t, base, kb);
@@ -267,10 +282,10 @@ __device__ __forceinline__ void inv_pass_store(const float2 (&x)[16], float2 *s,
 
 // Inverse passes NF..2 (after the partial pass); pass 1 is left to the caller,
 // which takes its output from registers.
-template <int K, int I>
-__device__ __forceinline__ void inv_full(float2 *s, int t, int p, const float2 *__restrict__ twp) {
+template <int K, int I, typename C>
+__device__ __forceinline__ void inv_full(C *s, int t, int p, const C *__restrict__ twp) {
     if constexpr (I >= 2) {
-        float2 x[16];
+        C x[16];
         inv_pass_load<K, I>(x, s, t, p, twp);
         inv_pass_store<K, I>(x, s, t, p);
         __syncthreads();
@@ -278,12 +293,12 @@ __device__ __forceinline__ void inv_full(float2 *s, int t, int p, const float2 *
     }
 }
 
-template <int K>
-__device__ __forceinline__ void inv_partial(float2 *s, int t, int p) {
+template <int K, typename C>
+__device__ __forceinline__ void inv_partial(C *s, int t, int p) {
     if constexpr (Shape<K>::Q > 0) {
         constexpr int Q = Shape<K>::Q, R = 1 << Q;
         const int sb = swz_base(t << 4, p);
-        float2 x[16];
+        C x[16];
 #pragma unroll
         for (int j = 0; j < 16; j += R)
 #pragma unroll
@@ -291,7 +306,7 @@ __device__ __forceinline__ void inv_partial(float2 *s, int t, int p) {
 #pragma unroll
         for (int j = 0; j < 16; j += R) {
             dftq<true, Q>(x + j);
-            float2 y[R];
+            C y[R];
 #pragma unroll
             for (int v = 0; v < R; ++v) y[v] = x[j + outq<Q>(v)];
 #pragma unroll
@@ -301,5 +316,5 @@ __device__ __forceinline__ void inv_partial(float2 *s, int t, int p) {
     }
 }
 
-}  // namespace fft32
+}  // namespace fft16
 }  // namespace ek

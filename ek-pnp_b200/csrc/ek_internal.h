@@ -72,6 +72,32 @@ __device__ __forceinline__ void st_field_f(float *p, float v, bool keep) {
     *p = v;
 }
 
+__device__ __forceinline__ void st_field_f4(float *p, float4 v, bool keep) {
+#if defined(__CUDA_ARCH__)
+    if (keep) {
+        unsigned long long pol;
+        asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+        asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z),
+                     "f"(v.w), "l"(pol)
+                     : "memory");
+        return;
+    }
+#endif
+    *(float4 *)p = v;
+}
+
+__device__ __forceinline__ void st_field_f2(float *p, float2 v, bool keep) {
+#if defined(__CUDA_ARCH__)
+    if (keep) {
+        unsigned long long pol;
+        asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+        asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(v.x), "f"(v.y), "l"(pol) : "memory");
+        return;
+    }
+#endif
+    *(float2 *)p = v;
+}
+
 template <typename... Exp, typename... Act>
 cudaError_t launch_pdl(void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
     cudaLaunchConfig_t cfg = {};
@@ -86,6 +112,23 @@ cudaError_t launch_pdl(void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem,
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Act>(args)...);
 }
+
+// launch_pdl, or an ordinary launch where pdl is false.
+template <typename... Exp, typename... Act>
+cudaError_t launch_maybe_pdl(bool pdl, void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
+    if (pdl) return launch_pdl(kern, grid, block, smem, s, std::forward<Act>(args)...);
+    kern<<<grid, block, smem, s>>>(std::forward<Act>(args)...);
+    return cudaGetLastError();
+}
+// Channels of at most this many nodes: every kernel of a step is about one
+// wave of blocks, and the step a chain of launch latencies.
+constexpr size_t PDL_NODES = (size_t)1 << 18;
+// The LBM kernel of a step: by itself (many waves of blocks); of a small
+// channel, letting pass A be scheduled early; the same, itself scheduled while
+// the kernel before drains.  CHAIN_NEXT gathers its populations before the wait
+// for that kernel, so it is only for a step right after another one's Poisson
+// solve (the populations were written three kernels earlier).
+enum StepChain { CHAIN_NONE = 0, CHAIN_FIRST = 1, CHAIN_NEXT = 2 };
 
 // D2Q9 velocity set in the reference numbering:  6 2 5 / 3 0 1 / 7 4 8
 __host__ __device__ constexpr int cxd(int d) {
@@ -144,8 +187,9 @@ enum Field { F_RHO = 0, F_UX, F_UY, F_CP, F_CN, F_PSI, F_EX, F_EY, F_RHS, F_COUN
 cudaError_t launch_rates(const ek_params &p, Rates *dev_out, cudaStream_t s);
 cudaError_t launch_init_f64(const Chan &c, double *pops, const double *fields, bool explicit_e,
                             cudaStream_t s);
+// chain: how the step's kernel is launched (StepChain)
 cudaError_t launch_step_f64(const Chan &c, const double *src, double *dst, double *fields,
-                            bool first, bool explicit_e, bool moments, cudaStream_t s);
+                            bool first, bool explicit_e, bool moments, int chain, cudaStream_t s);
 cudaError_t launch_efield_f64(const Chan &c, double *fields, cudaStream_t s);
 cudaError_t launch_rhs_from_moments_f64(const Chan &c, double *fields, cudaStream_t s);
 
@@ -164,7 +208,7 @@ cudaError_t launch_pb_newton(const Chan &c, double dy, double g, double a, const
 // sbuf: index (0/1) of the population buffer that src is (it names the wall
 // ions' frames); buf: the buffer that pops is.
 cudaError_t launch_step_shifted(const Chan &c, int storage, const void *src, void *dst, double *fields,
-                                bool first, bool explicit_e, bool moments, int sbuf, cudaStream_t s);
+                                bool first, bool explicit_e, bool moments, int sbuf, int chain, cudaStream_t s);
 cudaError_t launch_init_shifted(const Chan &c, int storage, void *pops, const double *fields, bool explicit_e,
                                 int buf, cudaStream_t s);
 // Wall frames of the ions from the fields' wall rows (initialisation; buf is
@@ -260,10 +304,11 @@ cudaError_t poisson_tridiag_f32(const PoissonPlan &pp, cudaStream_t s);
 cudaError_t batch_tridiag_f32(const PoissonPlan *plans, const void *items, int nitems, cudaStream_t s);
 // Batched Poisson passes of the FP32 form over many channels (ek_batch.cu
 // builds the items): pass 0/2 items int2 {channel, first row pair}
-// (256-thread blocks, each 256/(nx/16) row pairs; power-of-two nx from 16 to
-// 4096); pass 1 is batch_tridiag_f32.  write_f64 as poisson_pass_f32.
+// (each block/(nx/16) row pairs; power-of-two nx from 16 to 4096); pass 1 is batch_tridiag_f32.  write_f64 as poisson_pass_f32.
+// block: the threads a block, batch_row_block of the widest channel.
 cudaError_t batch_poisson(int pass, const PoissonPlan *plans, const Chan *chans, double *const *fields,
-                          const void *items, int nitems, bool write_f64, cudaStream_t s);
+                          const void *items, int nitems, int block, bool write_f64, cudaStream_t s);
+int batch_row_block(int nx_max);
 int poisson_tridiag_modes(int n);
 // Steady-state residual sums (ek_residual.cu): per channel 8 FP64 sums,
 // (q - q_snap)^2 then q^2 for q in (ux, c+, c-, psi); the snapshot is updated.
@@ -277,6 +322,9 @@ cudaError_t launch_batch_residual(const Chan *chans, double *const *fields, doub
                                   cudaStream_t s);
 // Record an error message for ek_last_error() (ek_api.cu).
 void set_last_error(const char *msg);
-cudaError_t poisson_set_smem_limits();
+// Shared-memory attributes of the row kernels: of one plan's length (its sizes and
+// specf set), of a batch's.
+cudaError_t poisson_set_smem_limits(const PoissonPlan &pp);
+cudaError_t batch_set_smem_limits(int block);
 
 }  // namespace ek

@@ -71,24 +71,20 @@ ChanF make_chanf(const Chan &c) {
 namespace {
 
 constexpr int TPB = 128;
-// Blocks per SM the register allocation must allow.  Unconstrained the node
-// update takes 108 registers (4 blocks of 4 warps per SM); at 7 blocks (72
-// registers, no spills) the kernel hides more of the HBM latency: 0.169 ms
-// against 0.219 ms per launch on 4096x1024 FP32 (B200; 6 blocks 0.183, 8
-// blocks with 16-byte spills 0.181).
+// Blocks per SM the register allocation must allow: 4 blocks of 128 threads,
+// 128 registers, which the update of two nodes a thread takes without
+// spilling; 512 threads then have 54 loads of populations in flight each.
 #ifndef EK_LBM_MIN_BLOCKS
-#define EK_LBM_MIN_BLOCKS 7
+#define EK_LBM_MIN_BLOCKS 4
 #endif
 
-// I: the index type of the node update (uint32_t when every offset into the
-// population and field planes fits 32 bits, see own9s).
-template <typename S, bool FIRST, bool EE, typename I>
+template <typename S, bool FIRST, bool EE>
 __global__ void __launch_bounds__(TPB, EK_LBM_MIN_BLOCKS)
 step_shifted(const ChanF k, const S *__restrict__ src, S *__restrict__ dst, double *__restrict__ fields, bool mom,
-             int sbuf) {
-    const int x = blockIdx.x * TPB + threadIdx.x;
-    if (x >= k.nx) return;
-    node_shifted<S, FIRST, EE, I>(k, src, dst, fields, x, blockIdx.y, mom, sbuf);
+             int sbuf, bool wait) {
+    const int x = 2 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= k.nx || y >= k.ny) return;
+    node_shifted<S, FIRST, EE, float2>(k, src, dst, fields, x, y, mom, sbuf, wait);
 }
 
 template <typename S>
@@ -111,27 +107,22 @@ __global__ void __launch_bounds__(256) wall_delta(const ChanF k, const float *__
     if (i < 4 * k.nx) wall_delta_dev(k, kwall, wdelta, i);
 }
 
-template <typename S, typename I>
-cudaError_t step_indexed(const ChanF &k, const void *src, void *dst, double *fields, bool first, bool ee,
-                         bool mom, int sbuf, cudaStream_t s) {
-    const dim3 g((k.nx + TPB - 1) / TPB, k.ny);
-    const S *a = (const S *)src;
-    S *b = (S *)dst;
-    if (first) {
-        if (ee) step_shifted<S, true, true, I><<<g, TPB, 0, s>>>(k, a, b, fields, mom, sbuf);
-        else step_shifted<S, true, false, I><<<g, TPB, 0, s>>>(k, a, b, fields, mom, sbuf);
-    } else {
-        if (ee) step_shifted<S, false, true, I><<<g, TPB, 0, s>>>(k, a, b, fields, mom, sbuf);
-        else step_shifted<S, false, false, I><<<g, TPB, 0, s>>>(k, a, b, fields, mom, sbuf);
-    }
-    return cudaGetLastError();
-}
-
 template <typename S>
 cudaError_t step_typed(const ChanF &k, const void *src, void *dst, double *fields, bool first, bool ee,
-                       bool mom, int sbuf, cudaStream_t s) {
-    if (index32_fits(k.plane)) return step_indexed<S, uint32_t>(k, src, dst, fields, first, ee, mom, sbuf, s);
-    return step_indexed<S, size_t>(k, src, dst, fields, first, ee, mom, sbuf, s);
+                       bool mom, int sbuf, int chain, cudaStream_t s) {
+    // a thread takes two columns; blocks of narrow channels take several rows
+    int tx = 8;
+    while (tx < TPB && 2 * tx < k.nx) tx *= 2;
+    const dim3 t(tx, TPB / tx), g(((k.nx + 1) / 2 + tx - 1) / tx, (k.ny + TPB / tx - 1) / (TPB / tx));
+    const S *a = (const S *)src;
+    S *b = (S *)dst;
+    const bool wait = chain != CHAIN_NONE, pdl = chain == CHAIN_NEXT;
+    if (first) {
+        if (ee) return launch_maybe_pdl(pdl, step_shifted<S, true, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+        return launch_maybe_pdl(pdl, step_shifted<S, true, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+    }
+    if (ee) return launch_maybe_pdl(pdl, step_shifted<S, false, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+    return launch_maybe_pdl(pdl, step_shifted<S, false, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
 }
 
 __global__ void __launch_bounds__(256) row_refs(const Chan c, const double *__restrict__ fields, int qf, int qp,
@@ -227,10 +218,11 @@ cudaError_t launch_rebase(const Chan &c, int storage, void *pops, const float *k
 }
 
 cudaError_t launch_step_shifted(const Chan &c, int storage, const void *src, void *dst, double *fields,
-                                bool first, bool explicit_e, bool moments, int sbuf, cudaStream_t s) {
+                                bool first, bool explicit_e, bool moments, int sbuf, int chain, cudaStream_t s) {
     const ChanF k = make_chanf(c);
-    if (storage == EK_STORE_F16) return step_typed<__half>(k, src, dst, fields, first, explicit_e, moments, sbuf, s);
-    return step_typed<float>(k, src, dst, fields, first, explicit_e, moments, sbuf, s);
+    if (storage == EK_STORE_F16)
+        return step_typed<__half>(k, src, dst, fields, first, explicit_e, moments, sbuf, chain, s);
+    return step_typed<float>(k, src, dst, fields, first, explicit_e, moments, sbuf, chain, s);
 }
 
 cudaError_t launch_init_shifted(const Chan &c, int storage, void *pops, const double *fields, bool explicit_e,

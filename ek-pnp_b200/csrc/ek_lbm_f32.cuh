@@ -101,93 +101,207 @@ template <> __device__ __forceinline__ void st_pop<__half>(__half *p, float v) {
 
 constexpr float W0F = 4.0f / 9.0f, WSF = 1.0f / 9.0f, WDF = 1.0f / 36.0f;
 
-// Index arithmetic of the node update in type I: size_t in general,
-// uint32_t where every offset into the 27 population planes and the 9 field
-// planes fits 32 bits (27 plane < 2^32), which spares the 64-bit address
-// arithmetic of every access.
-// Whether the 32-bit index form covers a channel of `plane` elements a plane.
-__host__ __device__ constexpr bool index32_fits(size_t plane) { return plane < ((size_t)1 << 32) / 27; }
+// ---- arithmetic of one node or of two neighbouring nodes -------------------
+// V = float updates one node a thread, V = float2 the nodes x and x + 1 (x
+// even) with the packed FP32 instructions of sm_100 (one issue slot for both).
+// Every operation is an explicit round-to-nearest intrinsic, so that nothing
+// is left to the compiler's choice of fused multiply-adds: the forms of the
+// step (two nodes a thread, the batch, the TMA-fed one) give the same bits.
+// No inexact product is an operand of vadd (vfma instead): packed, the sum of a
+// product was seen to round once (ptxas 12.9), where the scalar one rounds twice.
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+template <typename V> __device__ __forceinline__ V bc(float v);
+template <> __device__ __forceinline__ float bc<float>(float v) { return v; }
+template <> __device__ __forceinline__ float2 bc<float2>(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float vrcp(float a) { return 1.0f / a; }
+__device__ __forceinline__ float2 vrcp(float2 a) { return make_float2(1.0f / a.x, 1.0f / a.y); }
+// a + k b, a k for a scalar k
+template <typename V> __device__ __forceinline__ V vaxpy(float k, V b, V a) { return vfma(bc<V>(k), b, a); }
+template <typename V> __device__ __forceinline__ V vscale(float k, V a) { return vmul(bc<V>(k), a); }
+template <typename V> struct Width;
+template <> struct Width<float> { static constexpr int n = 1; };
+template <> struct Width<float2> { static constexpr int n = 2; };
 
-template <typename S, typename I = size_t>
-__device__ __forceinline__ void own9s(const S *__restrict__ b, I pl, I o, float p[9]) {
-#pragma unroll
-    for (int d = 0; d < 9; ++d) p[d] = ld_pop<S>(b + ((I)d * pl + o));
+// Columns of a thread's nodes: x, and where its pulls and differences look --
+// xm left of the first node, xr right of the first (the second node itself,
+// or 0 where the second lies past the last column), xp right of the last.
+struct Cols {
+    int x, xm, xr, xp;
+    bool two;  // the second node exists (nx odd: the last thread of a row has one)
+};
+template <typename V> __device__ __forceinline__ Cols make_cols(int x, int nx);
+template <> __device__ __forceinline__ Cols make_cols<float>(int x, int nx) {
+    const int xp = x + 1 == nx ? 0 : x + 1;
+    return {x, x == 0 ? nx - 1 : x - 1, xp, xp, false};
+}
+template <> __device__ __forceinline__ Cols make_cols<float2>(int x, int nx) {
+    return {x, x == 0 ? nx - 1 : x - 1, x + 1 == nx ? 0 : x + 1, x + 2 >= nx ? x + 2 - nx : x + 2, x + 1 < nx};
 }
 
-template <typename S, typename I = size_t>
-__device__ __forceinline__ void pull9s(const S *__restrict__ b, I pl, int nxp, int x, int y, int xm,
-                                       int xp, int ym, int yp, float p[9]) {
-    const I r0 = (I)y * (I)nxp, rm = (I)ym * (I)nxp, rp = (I)yp * (I)nxp;
-    p[0] = ld_pop<S>(b + (r0 + (I)x));
-    p[1] = ld_pop<S>(b + (1 * pl + r0 + (I)xm));
-    p[2] = ld_pop<S>(b + (2 * pl + rm + (I)x));
-    p[3] = ld_pop<S>(b + (3 * pl + r0 + (I)xp));
-    p[4] = ld_pop<S>(b + (4 * pl + rp + (I)x));
-    p[5] = ld_pop<S>(b + (5 * pl + rm + (I)xm));
-    p[6] = ld_pop<S>(b + (6 * pl + rm + (I)xp));
-    p[7] = ld_pop<S>(b + (7 * pl + rp + (I)xp));
-    p[8] = ld_pop<S>(b + (8 * pl + rp + (I)xm));
+// Addresses: a plane's base pointer is the same for the whole block, and an
+// element's byte offset inside a plane fits 32 bits for every channel this
+// library takes (at most 8192 x 65535 elements of 8 bytes), so an access is a
+// uniform 64-bit base plus a 32-bit offset.  Offsets of the four columns in a row:
+struct RowAt {
+    uint32_t x, xm, xr, xp;  // elements
+};
+__device__ __forceinline__ RowAt row_at(const Cols &c, int y, int nxp) {
+    const uint32_t r = (uint32_t)y * (uint32_t)nxp;
+    return {r + (uint32_t)c.x, r + (uint32_t)c.xm, r + (uint32_t)c.xr, r + (uint32_t)c.xp};
+}
+template <typename T> __device__ __forceinline__ T *at(T *base, uint32_t e) {
+    return (T *)((char *)base + (size_t)(e * (uint32_t)sizeof(T)));
+}
+template <typename T> __device__ __forceinline__ const T *at(const T *base, uint32_t e) {
+    return (const T *)((const char *)base + (size_t)(e * (uint32_t)sizeof(T)));
+}
+
+// Values of a plane's row at the thread's own columns (rows start 64-byte
+// aligned and are padded to a multiple of 32 elements, so the pair is one
+// access), at their left neighbours and at their right ones.
+template <typename V, typename S> struct Row;
+template <typename S> struct Row<float, S> {
+    static __device__ __forceinline__ float own(const S *p, const RowAt &r) { return ld_pop<S>(at(p, r.x)); }
+    static __device__ __forceinline__ float left(const S *p, const RowAt &r) { return ld_pop<S>(at(p, r.xm)); }
+    static __device__ __forceinline__ float right(const S *p, const RowAt &r) { return ld_pop<S>(at(p, r.xp)); }
+    static __device__ __forceinline__ void put(S *p, const RowAt &r, float v) { st_pop<S>(at(p, r.x), v); }
+};
+__device__ __forceinline__ float2 ld_pair(const float *p) { return __ldg((const float2 *)p); }
+__device__ __forceinline__ float2 ld_pair(const __half *p) { return __half22float2(__ldg((const __half2 *)p)); }
+__device__ __forceinline__ void st_pair(float *p, float2 v) { *(float2 *)p = v; }
+__device__ __forceinline__ void st_pair(__half *p, float2 v) { *(__half2 *)p = __float22half2_rn(v); }
+template <typename S> struct Row<float2, S> {
+    static __device__ __forceinline__ float2 own(const S *p, const RowAt &r) { return ld_pair(at(p, r.x)); }
+    static __device__ __forceinline__ float2 left(const S *p, const RowAt &r) {
+        return make_float2(ld_pop<S>(at(p, r.xm)), ld_pop<S>(at(p, r.x)));
+    }
+    static __device__ __forceinline__ float2 right(const S *p, const RowAt &r) {
+        return make_float2(ld_pop<S>(at(p, r.xr)), ld_pop<S>(at(p, r.xp)));
+    }
+    static __device__ __forceinline__ void put(S *p, const RowAt &r, float2 v) { st_pair(at(p, r.x), v); }
+};
+// Per-x arrays without padding (wall frames, lifting): element by element.
+template <typename V> struct PerX;
+template <> struct PerX<float> {
+    static __device__ __forceinline__ float own(const float *a, const Cols &c) { return __ldg(a + c.x); }
+    static __device__ __forceinline__ float left(const float *a, const Cols &c) { return __ldg(a + c.xm); }
+    static __device__ __forceinline__ float right(const float *a, const Cols &c) { return __ldg(a + c.xp); }
+};
+template <> struct PerX<float2> {
+    static __device__ __forceinline__ float2 own(const float *a, const Cols &c) {
+        return make_float2(__ldg(a + c.x), __ldg(a + (c.two ? c.x + 1 : c.x)));
+    }
+    static __device__ __forceinline__ float2 left(const float *a, const Cols &c) {
+        return make_float2(__ldg(a + c.xm), __ldg(a + c.x));
+    }
+    static __device__ __forceinline__ float2 right(const float *a, const Cols &c) {
+        return make_float2(__ldg(a + c.xr), __ldg(a + c.xp));
+    }
+};
+// Moments to a plane of doubles; ref: a reference density added in FP64.
+__device__ __forceinline__ void st_moment(double *p, const Cols &, const RowAt &r, float ref, float v) {
+    *at(p, r.x) = (double)ref + (double)v;
+}
+__device__ __forceinline__ void st_moment(double *p, const Cols &c, const RowAt &r, float2 ref, float2 v) {
+    *at(p, r.x) = (double)ref.x + (double)v.x;
+    if (c.two) *at(p, r.x + 1) = (double)ref.y + (double)v.y;
+}
+__device__ __forceinline__ float ld_f64(const double *p, const Cols &, const RowAt &r, float) { return (float)*at(p, r.x); }
+__device__ __forceinline__ float2 ld_f64(const double *p, const Cols &c, const RowAt &r, float2) {
+    return make_float2((float)*at(p, r.x), (float)*at(p, r.x + (c.two ? 1u : 0u)));
+}
+__device__ __forceinline__ void st_rhs(float *p, const RowAt &r, float v, bool keep) { st_field_f(at(p, r.x), v, keep); }
+__device__ __forceinline__ void st_rhs(float *p, const RowAt &r, float2 v, bool keep) { st_field_f2(at(p, r.x), v, keep); }
+
+template <typename V, typename S>
+__device__ __forceinline__ void own9s(const S *__restrict__ b, size_t pl, const RowAt &r, V p[9]) {
+#pragma unroll
+    for (int d = 0; d < 9; ++d) p[d] = Row<V, S>::own(b + d * pl, r);
+}
+
+// Pull: direction d arrives from (x - cx_d, y - cy_d); r0, rm, rp: the row
+// itself, the one below and the one above.
+template <typename V, typename S>
+__device__ __forceinline__ void pull9s(const S *__restrict__ b, size_t pl, const RowAt &r0, const RowAt &rm,
+                                       const RowAt &rp, V p[9]) {
+    using R = Row<V, S>;
+    p[0] = R::own(b, r0);
+    p[1] = R::left(b + 1 * pl, r0);
+    p[2] = R::own(b + 2 * pl, rm);
+    p[3] = R::right(b + 3 * pl, r0);
+    p[4] = R::own(b + 4 * pl, rp);
+    p[5] = R::left(b + 5 * pl, rm);
+    p[6] = R::right(b + 6 * pl, rm);
+    p[7] = R::right(b + 7 * pl, rp);
+    p[8] = R::left(b + 8 * pl, rp);
 }
 
 // Change of frame of pulled populations to the puller's row reference:
 // directions 2, 5, 6 came from row y-1 (dm = kref[y-1] - kref[y]), 4, 7, 8
 // from row y+1 (dp = kref[y+1] - kref[y]); 36 w = 4 (straight), 1 (diagonal).
-__device__ __forceinline__ void reframe_dn(float p[9], float dm) {
-    p[2] += 4.0f * dm;
-    p[5] += dm;
-    p[6] += dm;
+template <typename V> __device__ __forceinline__ void reframe_dn(V p[9], float dm) {
+    p[2] = vadd(p[2], bc<V>(4.0f * dm));
+    p[5] = vadd(p[5], bc<V>(dm));
+    p[6] = vadd(p[6], bc<V>(dm));
 }
-__device__ __forceinline__ void reframe_up(float p[9], float dp) {
-    p[4] += 4.0f * dp;
-    p[7] += dp;
-    p[8] += dp;
+template <typename V> __device__ __forceinline__ void reframe_up(V p[9], float dp) {
+    p[4] = vadd(p[4], bc<V>(4.0f * dp));
+    p[7] = vadd(p[7], bc<V>(dp));
+    p[8] = vadd(p[8], bc<V>(dp));
 }
-__device__ __forceinline__ void reframe(float p[9], float dm, float dp) {
+template <typename V> __device__ __forceinline__ void reframe(V p[9], float dm, float dp) {
     reframe_dn(p, dm);
     reframe_up(p, dp);
 }
 // Pulls from a wall row, whose ion values sit in per-x frames kw(x'):
 // lower wall (puller y = 1): 2 from x, 5 from x-1, 6 from x+1;
 // upper wall (puller y = ny-2): 4 from x, 7 from x+1, 8 from x-1.
-__device__ __forceinline__ void reframe_dn_wall(float p[9], float kx, float kxm, float kxp, float k0) {
-    p[2] += 4.0f * (kx - k0);
-    p[5] += kxm - k0;
-    p[6] += kxp - k0;
+template <typename V> __device__ __forceinline__ void reframe_dn_wall(V p[9], const float *kw, const Cols &c, V k0) {
+    p[2] = vaxpy(4.0f, vsub(PerX<V>::own(kw, c), k0), p[2]);
+    p[5] = vadd(p[5], vsub(PerX<V>::left(kw, c), k0));
+    p[6] = vadd(p[6], vsub(PerX<V>::right(kw, c), k0));
 }
-__device__ __forceinline__ void reframe_up_wall(float p[9], float kx, float kxm, float kxp, float k0) {
-    p[4] += 4.0f * (kx - k0);
-    p[7] += kxp - k0;
-    p[8] += kxm - k0;
+template <typename V> __device__ __forceinline__ void reframe_up_wall(V p[9], const float *kw, const Cols &c, V k0) {
+    p[4] = vaxpy(4.0f, vsub(PerX<V>::own(kw, c), k0), p[4]);
+    p[7] = vadd(p[7], vsub(PerX<V>::right(kw, c), k0));
+    p[8] = vadd(p[8], vsub(PerX<V>::left(kw, c), k0));
 }
 
 // Ion anti-bounce-back in deviations: d_ibar = -q_i + 2 w_i (c_wall - R).
-__device__ __forceinline__ void ion_wall_dev(const float q[9], float dcw, float p[9]) {
-    const float m0 = 2.0f * W0F * dcw, ms = 2.0f * WSF * dcw, md = 2.0f * WDF * dcw;
-    p[0] = -q[0] + m0;
-    p[3] = -q[1] + ms;
-    p[4] = -q[2] + ms;
-    p[1] = -q[3] + ms;
-    p[2] = -q[4] + ms;
-    p[7] = -q[5] + md;
-    p[8] = -q[6] + md;
-    p[5] = -q[7] + md;
-    p[6] = -q[8] + md;
+template <typename V> __device__ __forceinline__ void ion_wall_dev(const V q[9], V dcw, V p[9]) {
+    const V m0 = vscale(2.0f * W0F, dcw), ms = vscale(2.0f * WSF, dcw), md = vscale(2.0f * WDF, dcw);
+    p[0] = vsub(m0, q[0]);
+    p[3] = vsub(ms, q[1]);
+    p[4] = vsub(ms, q[2]);
+    p[1] = vsub(ms, q[3]);
+    p[2] = vsub(ms, q[4]);
+    p[7] = vsub(md, q[5]);
+    p[8] = vsub(md, q[6]);
+    p[5] = vsub(md, q[7]);
+    p[6] = vsub(md, q[8]);
 }
 
 // Moments with opposite directions paired first.  In the double layer the
 // y-opposite populations carry large, nearly opposite parts (the force-
 // balanced y-flux); adding those partners first cancels them exactly
 // (Sterbenz), so the small remaining sums round at their own scale.
-__device__ __forceinline__ float sum9f(const float t[9]) {
-    return (t[0] + (t[1] + t[3])) + ((t[2] + t[4]) + ((t[5] + t[7]) + (t[6] + t[8])));
+template <typename V> __device__ __forceinline__ V sum9f(const V t[9]) {
+    return vadd(vadd(t[0], vadd(t[1], t[3])), vadd(vadd(t[2], t[4]), vadd(vadd(t[5], t[7]), vadd(t[6], t[8]))));
 }
 // x-momentum: t5 - t6 and t8 - t7 pair values streamed from one row (same
 // y-part), so each difference is exact when the y-part dominates.
-__device__ __forceinline__ float momx(const float t[9]) {
-    return (t[1] - t[3]) + ((t[5] - t[6]) + (t[8] - t[7]));
+template <typename V> __device__ __forceinline__ V momx(const V t[9]) {
+    return vadd(vsub(t[1], t[3]), vadd(vsub(t[5], t[6]), vsub(t[8], t[7])));
 }
-__device__ __forceinline__ float momy(const float t[9]) {
-    return (t[2] - t[4]) + ((t[5] + t[6]) - (t[7] + t[8]));
+template <typename V> __device__ __forceinline__ V momy(const V t[9]) {
+    return vadd(vsub(t[2], t[4]), vsub(vadd(t[5], t[6]), vadd(t[7], t[8])));
 }
 
 // v/36 by multiplication with the rounded 1/36: the momentum-carrying parts
@@ -220,75 +334,79 @@ __device__ __forceinline__ float div36(float v) { return v * (1.0f / 36.0f); }
 //    force source sm cfl dt F is split the same way.
 // Ions (not FLUID) relax their flux to 4 dens c/36 per pair unit: the ion
 // flux is not conserved, so no factor accumulates.
-template <bool FORCE, bool FLUID>
-__device__ __forceinline__ void trt_f32(float d[9], float ddens, float dens, float ux, float uy, float usq_rest,
-                                        float wp, float wm, const ChanF &k, float fx, float fy, float px, float py) {
-    const float vsq = ux * ux + uy * uy;
-    const float usq = k.hinvcs2 * vsq;
-    const float base = ddens - dens * usq;
-    const float cx = ux * k.kcu, cy = uy * k.kcu;
-    // symmetric equilibria: straight pairs, diagonal mass and xy moments, rest remainder
-    const float seq13 = WSF * (base + dens * (0.5f * cx * cx));
-    const float seq24 = WSF * (base + dens * (0.5f * cy * cy));
-    const float seq_s = (base + dens * (0.5f * (cx * cx + cy * cy))) * (1.0f / 9.0f);
-    const float seq_q = dens * (cx * cy) * (1.0f / 9.0f);
-    const float e0 = (ddens - ((2.0f * seq13 + 2.0f * seq24) + seq_s)) + W0F * dens * (k.hinvcs2 * (vsq - usq_rest));
+// Pairs are carried doubled (d1 + d3, d1 - d3), which is exact.
+template <bool FORCE, bool FLUID, typename V>
+__device__ __forceinline__ void trt_f32(V d[9], V ddens, V dens, V ux, V uy, bool rest_fluid, V usq_fluid, float wp,
+                                        float wm, const ChanF &k, V fx, V fy, V px, V py) {
+    const V vsq = vfma(ux, ux, vmul(uy, uy));
+    const V base = vfma(vscale(-k.hinvcs2, vsq), dens, ddens);
+    const V cx = vscale(k.kcu, ux), cy = vscale(k.kcu, uy);
+    const V qx = vmul(dens, cx), qy = vmul(dens, cy);
+    // symmetric equilibria: straight pairs (doubled), diagonal mass and xy
+    // moments, rest remainder
+    const V b9 = vscale(WSF, base), ax = vscale(1.0f / 9.0f, qx), ay = vscale(1.0f / 9.0f, qy);
+    const V xx = vmul(ax, cx), yy = vmul(ay, cy);
+    const V seq13 = vaxpy(2.0f, b9, xx), seq24 = vaxpy(2.0f, b9, yy);
+    const V seq_s = vaxpy(0.5f, xx, vaxpy(0.5f, yy, b9));
+    const V seq_q = vmul(ax, cy);
+    V e0 = vsub(ddens, vadd(vadd(seq13, seq24), seq_s));
+    if (rest_fluid) e0 = vfma(vscale(W0F * k.hinvcs2, dens), vsub(vsq, usq_fluid), e0);
     // antisymmetric equilibria (half-pair units: a13 = (d1 - d3)/2, X = d5 - d6 - d7 + d8)
-    float aq13, aqx, aq24, aqy;
+    V aq13, aqx, aq24, aqy;
     if (FLUID) {
-        aq13 = px * (1.0f / 3.0f);
-        aqx = px - 2.0f * aq13;
-        aq24 = py * (1.0f / 3.0f);
-        aqy = py - 2.0f * aq24;
+        aq13 = vscale(1.0f / 3.0f, px);
+        aqx = vaxpy(-2.0f, aq13, px);
+        aq24 = vscale(1.0f / 3.0f, py);
+        aqy = vaxpy(-2.0f, aq24, py);
     } else {
-        aq13 = aqx = 4.0f * div36(dens * cx);
-        aq24 = aqy = 4.0f * div36(dens * cy);
+        aq13 = aqx = ax;
+        aq24 = aqy = ay;
     }
-    float d0 = d[0] - wp * (d[0] - e0);
-    float s13 = 0.5f * (d[1] + d[3]), a13 = 0.5f * (d[1] - d[3]);
-    float s24 = 0.5f * (d[2] + d[4]), a24 = 0.5f * (d[2] - d[4]);
-    s13 = s13 - wp * (s13 - seq13);
-    a13 = a13 - wm * (a13 - aq13);
-    s24 = s24 - wp * (s24 - seq24);
-    a24 = a24 - wm * (a24 - aq24);
-    const float A = d[5] - d[6], B = d[8] - d[7];  // x-differences of values from one row
-    const float C = d[5] + d[6], D = d[7] + d[8];
-    float X = A + B, Q = A - B, Y = C - D, S = C + D;
-    S = S - wp * (S - seq_s);
-    Q = Q - wp * (Q - seq_q);
-    X = X - wm * (X - aqx);
-    Y = Y - wm * (Y - aqy);
+    const V nwp = bc<V>(-wp), nwm = bc<V>(-wm);
+    V d0 = vfma(nwp, vsub(d[0], e0), d[0]);
+    V s13 = vadd(d[1], d[3]), a13 = vsub(d[1], d[3]);
+    V s24 = vadd(d[2], d[4]), a24 = vsub(d[2], d[4]);
+    s13 = vfma(nwp, vsub(s13, seq13), s13);
+    a13 = vfma(nwm, vaxpy(-2.0f, aq13, a13), a13);
+    s24 = vfma(nwp, vsub(s24, seq24), s24);
+    a24 = vfma(nwm, vaxpy(-2.0f, aq24, a24), a24);
+    const V A = vsub(d[5], d[6]), B = vsub(d[8], d[7]);  // x-differences of values from one row
+    const V C = vadd(d[5], d[6]), D = vadd(d[7], d[8]);
+    V X = vadd(A, B), Q = vsub(A, B), Y = vsub(C, D), S = vadd(C, D);
+    S = vfma(nwp, vsub(S, seq_s), S);
+    Q = vfma(nwp, vsub(Q, seq_q), Q);
+    X = vfma(nwm, vsub(X, aqx), X);
+    Y = vfma(nwm, vsub(Y, aqy), Y);
     if (FORCE) {
-        const float uF = k.inv_cs2 * (ux * fx + uy * fy);
-        const float cfx = fx * k.gF, cfy = fy * k.gF;
-        const float sp = k.sp * k.dt;
+        const V nuF = vscale(-k.inv_cs2, vfma(ux, fx, vmul(uy, fy)));
+        const V cfx = vscale(k.gF, fx), cfy = vscale(k.gF, fy);
+        const float sp9 = k.sp * k.dt * WSF;
         // symmetric (mass-free) part: the rest takes the remainder
-        const float g13 = sp * (WSF * (cx * cfx - uF)), g24 = sp * (WSF * (cy * cfy - uF));
-        const float gs = sp * ((cx * cfx + cy * cfy - uF) * (1.0f / 9.0f));
-        const float gq = sp * ((cx * cfy + cy * cfx) * (1.0f / 9.0f));
-        d0 -= (2.0f * g13 + 2.0f * g24) + gs;
-        s13 += g13;
-        s24 += g24;
-        S += gs;
-        Q += gq;
+        const V t13 = vfma(cx, cfx, nuF), t24 = vfma(cy, cfy, nuF), ts = vfma(cx, cfx, t24);
+        d0 = vaxpy(-sp9, vaxpy(2.0f, vadd(t13, t24), ts), d0);
+        s13 = vaxpy(2.0f * sp9, t13, s13);
+        s24 = vaxpy(2.0f * sp9, t24, s24);
+        S = vaxpy(sp9, ts, S);
+        Q = vaxpy(sp9, vfma(cx, cfy, vmul(cy, cfx)), Q);
         // momentum: sm cfl dt F, a third to each straight half-pair unit
-        const float fsx = k.srcF * fx, fsy = k.srcF * fy;
-        const float q13 = fsx * (1.0f / 3.0f), q24 = fsy * (1.0f / 3.0f);
-        a13 += q13;
-        a24 += q24;
-        X += fsx - 2.0f * q13;
-        Y += fsy - 2.0f * q24;
+        const V fsx = vscale(k.srcF, fx), fsy = vscale(k.srcF, fy);
+        const V q13 = vscale(1.0f / 3.0f, fsx), q24 = vscale(1.0f / 3.0f, fsy);
+        a13 = vaxpy(2.0f, q13, a13);
+        a24 = vaxpy(2.0f, q24, a24);
+        X = vadd(X, vaxpy(-2.0f, q13, fsx));
+        Y = vadd(Y, vaxpy(-2.0f, q24, fsy));
     }
-    const float P = S + Y, M = S - Y, U = Q + X, V = Q - X;
+    const V h13 = vscale(0.5f, s13), h24 = vscale(0.5f, s24);
+    const V P = vscale(0.25f, vadd(S, Y)), M = vscale(0.25f, vsub(S, Y)), U = vadd(Q, X), W = vsub(Q, X);
     d[0] = d0;
-    d[1] = s13 + a13;
-    d[3] = s13 - a13;
-    d[2] = s24 + a24;
-    d[4] = s24 - a24;
-    d[5] = 0.25f * (P + U);
-    d[6] = 0.25f * (P - U);
-    d[7] = 0.25f * (M + V);
-    d[8] = 0.25f * (M - V);
+    d[1] = vaxpy(0.5f, a13, h13);
+    d[3] = vaxpy(-0.5f, a13, h13);
+    d[2] = vaxpy(0.5f, a24, h24);
+    d[4] = vaxpy(-0.5f, a24, h24);
+    d[5] = vaxpy(0.25f, U, P);
+    d[6] = vaxpy(-0.25f, U, P);
+    d[7] = vaxpy(0.25f, W, M);
+    d[8] = vaxpy(-0.25f, W, M);
 }
 
 // Central-difference E of the shifted forms (the stencil of gpu_efield and
@@ -307,212 +425,212 @@ __device__ __forceinline__ void efield_shifted(const ChanF &k, const double *__r
 // FP32 fluctuations alone, Ey from the FP64 difference of the two row means
 // (the zero mode, rounded once) plus that of the fluctuations.  Stencil of
 // gpu_efield / gpu_bc (poisson.cu:145-174).
-template <typename I = size_t>
-__device__ __forceinline__ void efield_f32(const ChanF &k, int x, int y, int xm, int xp, float *ex, float *ey) {
-    const I r = (I)y * (I)k.nxp;
-    *ex = (__ldg(k.psif + (r + (I)xm)) - __ldg(k.psif + (r + (I)xp))) * k.half_inv_dxf;
+template <typename V>
+__device__ __forceinline__ void efield_f32(const ChanF &k, const Cols &c, int y, V *ex, V *ex_tot, V *ey) {
+    using R = Row<V, float>;
+    const RowAt r = row_at(c, y, k.nxp);
+    const V dx = vsub(R::left(k.psif, r), R::right(k.psif, r));
+    *ex = vscale(k.half_inv_dxf, dx);
+    *ex_tot = vaxpy(k.half_inv_dxf, dx, bc<V>(k.ext_xf));
     const int yc = y == 0 ? 1 : (y == k.ny - 1 ? k.ny - 2 : y);
     const float eym = (float)((__ldg(k.psim + yc - 1) - __ldg(k.psim + yc + 1)) * k.half_inv_dy);
-    *ey = eym + (__ldg(k.psif + ((I)(yc - 1) * (I)k.nxp + (I)x)) - __ldg(k.psif + ((I)(yc + 1) * (I)k.nxp + (I)x))) *
-                    k.half_inv_dyf;
+    const V dn = R::own(k.psif, row_at(c, yc - 1, k.nxp)), up = R::own(k.psif, row_at(c, yc + 1, k.nxp));
+    *ey = vaxpy(k.half_inv_dyf, vsub(dn, up), bc<V>(eym));
 }
 
-// One node of one step.  src/dst: 27 population planes (species-major);
-// fields: the channel's 9 FP64 field planes.
-// Raw populations of one node, as stored: FIRST -> the node's own
-// (pre-collision) values; otherwise the fluid pulled from the neighbours and
-// the ions pulled (interior rows) or the node's own values (wall rows).
-template <typename S, bool FIRST, typename I = size_t>
-__device__ __forceinline__ void gather_global(const ChanF &k, const S *__restrict__ src, int x, int y, float f[9],
-                                              float h[9], float t[9]) {
-    const I pl = (I)k.plane;
-    const int nxp = k.nxp;
-    const I o = (I)y * (I)nxp + (I)x;
-    const bool wall = y == 0 || y == k.ny - 1;
-    const int xm = x == 0 ? k.nx - 1 : x - 1, xp = x + 1 == k.nx ? 0 : x + 1;
-    const int ym = y == 0 ? k.ny - 1 : y - 1, yp = y + 1 == k.ny ? 0 : y + 1;
+// One step of a thread's node or pair of nodes.  src/dst: 27 population
+// planes (species-major); fields: the channel's 9 FP64 field planes.
+// Raw populations, as stored: FIRST -> the nodes' own (pre-collision) values;
+// otherwise the fluid pulled from the neighbours and the ions pulled (interior
+// rows) or the nodes' own values (wall rows).
+template <typename S, bool FIRST, typename V>
+__device__ __forceinline__ void gather_global(const ChanF &k, const S *__restrict__ src, const Cols &c, int y, V f[9],
+                                              V h[9], V t[9]) {
+    const size_t pl = k.plane;
+    const RowAt r0 = row_at(c, y, k.nxp);
     const S *sf = src, *sh = src + 9 * pl, *st = src + 18 * pl;
     if (FIRST) {
-        own9s<S, I>(sf, pl, o, f);
-        own9s<S, I>(sh, pl, o, h);
-        own9s<S, I>(st, pl, o, t);
+        own9s<V, S>(sf, pl, r0, f);
+        own9s<V, S>(sh, pl, r0, h);
+        own9s<V, S>(st, pl, r0, t);
     } else {
-        pull9s<S, I>(sf, pl, nxp, x, y, xm, xp, ym, yp, f);
-        if (wall) {
-            own9s<S, I>(sh, pl, o, h);
-            own9s<S, I>(st, pl, o, t);
+        const RowAt rm = row_at(c, y == 0 ? k.ny - 1 : y - 1, k.nxp), rp = row_at(c, y + 1 == k.ny ? 0 : y + 1, k.nxp);
+        pull9s<V, S>(sf, pl, r0, rm, rp, f);
+        if (y == 0 || y == k.ny - 1) {
+            own9s<V, S>(sh, pl, r0, h);
+            own9s<V, S>(st, pl, r0, t);
         } else {
-            pull9s<S, I>(sh, pl, nxp, x, y, xm, xp, ym, yp, h);
-            pull9s<S, I>(st, pl, nxp, x, y, xm, xp, ym, yp, t);
+            pull9s<V, S>(sh, pl, r0, rm, rp, h);
+            pull9s<V, S>(st, pl, r0, rm, rp, t);
         }
     }
 }
 
-// Collision, walls and stores of one node from its raw populations (see
-// gather_global); src is read only for the lower wall's row-1 pull.  sbuf:
-// index (0/1) of the population buffer that src is, which names the wall
+// Collision, walls and stores of a thread's nodes from their raw populations
+// (see gather_global); src is read only for the lower wall's row-1 pull.
+// sbuf: index (0/1) of the population buffer that src is, which names the wall
 // nodes' ion frames of the values read (sbuf) and written (sbuf ^ 1).
-// `moments` is a run-time flag on purpose: as a template parameter it gave
-// two instantiations that the compiler fused into multiply-adds differently,
-// so a step that wrote the moments could round differently from one that
-// did not.  One body with predicated stores keeps every step's arithmetic
-// independent of how the steps are split into calls.
-template <typename S, bool FIRST, bool EXPLICIT_E, typename I = size_t>
-__device__ __forceinline__ void collide_shifted(const ChanF &k, float f[9], float h[9], float t[9],
-                                                const S *__restrict__ src, S *__restrict__ dst,
-                                                double *__restrict__ fields, int x, int y, bool moments, int sbuf) {
-    const I pl = (I)k.plane;
-    const int nxp = k.nxp;
-    const I o = (I)y * (I)nxp + (I)x;
-    const bool lo = y == 0, hi = y == k.ny - 1, wall = lo || hi;
-    const int xm = x == 0 ? k.nx - 1 : x - 1, xp = x + 1 == k.nx ? 0 : x + 1;
-    const int ym = y == 0 ? k.ny - 1 : y - 1, yp = y + 1 == k.ny ? 0 : y + 1;
-    const S *sf = src;
-    const int ny = k.ny;
-    // frames (/36) of this node's values: the fluid and interior ions use the
+// `moments` is a run-time flag, so that every step's arithmetic is independent
+// of how the steps are split into calls.
+template <typename S, bool FIRST, bool EXPLICIT_E, typename V>
+__device__ __forceinline__ void collide_shifted(const ChanF &k, V f[9], V h[9], V t[9], const S *__restrict__ src,
+                                                S *__restrict__ dst, double *__restrict__ fields, const Cols &c, int y,
+                                                bool moments, int sbuf) {
+    using R = Row<V, S>;
+    const size_t pl = k.plane;
+    const int nxp = k.nxp, ny = k.ny;
+    const RowAt r0 = row_at(c, y, nxp);
+    const bool lo = y == 0, hi = y == ny - 1, wall = lo || hi;
+    const int ym = y == 0 ? ny - 1 : y - 1, yp = y + 1 == ny ? 0 : y + 1;
+    const int nx = k.nx;
+    // frames (/36) of these nodes' values: the fluid and interior ions use the
     // row references, the wall nodes' ions the per-x frame of the output buffer
     const float kf0 = __ldg(k.kref + y);
-    float kh0, kt0;
+    auto kw = [&](int buf, int s, int w) { return k.kwall + (size_t)((buf * 2 + s) * 2 + w) * nx; };
+    V kh0, kt0;
     if (wall) {
         const int w = lo ? 0 : 1;
-        kh0 = kwall_at(k, sbuf ^ 1, 0, w, x);
-        kt0 = kwall_at(k, sbuf ^ 1, 1, w, x);
+        kh0 = PerX<V>::own(kw(sbuf ^ 1, 0, w), c);
+        kt0 = PerX<V>::own(kw(sbuf ^ 1, 1, w), c);
     } else {
-        kh0 = __ldg(k.kref + ny + y);
-        kt0 = __ldg(k.kref + 2 * ny + y);
+        kh0 = bc<V>(__ldg(k.kref + ny + y));
+        kt0 = bc<V>(__ldg(k.kref + 2 * ny + y));
     }
-    const float Rf = 36.0f * kf0, Rh = 36.0f * kh0, Rt = 36.0f * kt0;  // exact: 36 K 2^-q < 2^22 2^-q
+    const float Rf = 36.0f * kf0;
+    const V Rh = vscale(36.0f, kh0), Rt = vscale(36.0f, kt0);  // exact: 36 K 2^-q < 2^22 2^-q
     if (!FIRST) reframe(f, __ldg(k.kref + ym) - kf0, __ldg(k.kref + yp) - kf0);
     if (wall) {
         // anti-bounce-back (gpu_bc_charge) from the stored frame into the
         // other: an exact reflection plus w_i times the frame defect; the
         // first step too, whose stored values init_node_shifted reflected
         const int w = lo ? 0 : 1;
-        float q[9];
+        V q[9];
 #pragma unroll
         for (int d = 0; d < 9; ++d) q[d] = h[d];
-        ion_wall_dev(q, wdelta_at(k, 0, w, x), h);
+        ion_wall_dev(q, PerX<V>::own(k.wdelta + (size_t)w * nx, c), h);
 #pragma unroll
         for (int d = 0; d < 9; ++d) q[d] = t[d];
-        ion_wall_dev(q, wdelta_at(k, 1, w, x), t);
+        ion_wall_dev(q, PerX<V>::own(k.wdelta + (size_t)(2 + w) * nx, c), t);
     } else if (!FIRST) {
         if (y == 1) {
-            reframe_dn_wall(h, kwall_at(k, sbuf, 0, 0, x), kwall_at(k, sbuf, 0, 0, xm), kwall_at(k, sbuf, 0, 0, xp), kh0);
-            reframe_dn_wall(t, kwall_at(k, sbuf, 1, 0, x), kwall_at(k, sbuf, 1, 0, xm), kwall_at(k, sbuf, 1, 0, xp), kt0);
+            reframe_dn_wall(h, kw(sbuf, 0, 0), c, kh0);
+            reframe_dn_wall(t, kw(sbuf, 1, 0), c, kt0);
         } else {
-            reframe_dn(h, __ldg(k.kref + ny + ym) - kh0);
-            reframe_dn(t, __ldg(k.kref + 2 * ny + ym) - kt0);
+            reframe_dn(h, __ldg(k.kref + ny + ym) - __ldg(k.kref + ny + y));
+            reframe_dn(t, __ldg(k.kref + 2 * ny + ym) - __ldg(k.kref + 2 * ny + y));
         }
         if (y == ny - 2) {
-            reframe_up_wall(h, kwall_at(k, sbuf, 0, 1, x), kwall_at(k, sbuf, 0, 1, xm), kwall_at(k, sbuf, 0, 1, xp), kh0);
-            reframe_up_wall(t, kwall_at(k, sbuf, 1, 1, x), kwall_at(k, sbuf, 1, 1, xm), kwall_at(k, sbuf, 1, 1, xp), kt0);
+            reframe_up_wall(h, kw(sbuf, 0, 1), c, kh0);
+            reframe_up_wall(t, kw(sbuf, 1, 1), c, kt0);
         } else {
-            reframe_up(h, __ldg(k.kref + ny + yp) - kh0);
-            reframe_up(t, __ldg(k.kref + 2 * ny + yp) - kt0);
+            reframe_up(h, __ldg(k.kref + ny + yp) - __ldg(k.kref + ny + y));
+            reframe_up(t, __ldg(k.kref + 2 * ny + yp) - __ldg(k.kref + 2 * ny + y));
         }
     }
-    const float drho = sum9f(f), dcp = sum9f(h), dcn = sum9f(t);
-    const float rho = Rf + drho;
-    float ex, ey;
+    const V drho = sum9f(f), dcp = sum9f(h), dcn = sum9f(t);
+    const V rho = vadd(bc<V>(Rf), drho);
+    V ex, ex_tot, ey;  // ex_tot: with the applied field
     if (EXPLICIT_E) {
-        ex = (float)fields[F_EX * pl + o];
-        ey = (float)fields[F_EY * pl + o];
+        ex = ld_f64(fields + F_EX * pl, c, r0, V{});
+        ey = ld_f64(fields + F_EY * pl, c, r0, V{});
+        ex_tot = vadd(ex, bc<V>(k.ext_xf));
     } else {
-        efield_f32<I>(k, x, y, xm, xp, &ex, &ey);
+        efield_f32<V>(k, c, y, &ex, &ex_tot, &ey);
     }
-    float fx = 0.0f, fy = 0.0f;
-    const float dq = dcp - dcn;
-    const float qnet = (Rh - Rt) + dq;  // c+ - c-
-    if (k.flags & EK_FLAG_FORCE) {
-        const float q = k.f_chargef * qnet;
-        fx = q * (ex + k.ext_xf) + k.exff;
-        fy = q * ey;
+    V fx = bc<V>(0.0f), fy = bc<V>(0.0f);
+    const V dq = vsub(dcp, dcn);
+    const bool force = (k.flags & EK_FLAG_FORCE) != 0;
+    if (force) {
+        const V q = vscale(k.f_chargef, vadd(vsub(Rh, Rt), dq));  // f_charge (c+ - c-)
+        fx = vfma(q, ex_tot, bc<V>(k.exff));
+        fy = vmul(q, ey);
     }
-    const float rrho = 1.0f / rho;
-    float ux = (momx(f) * k.inv_cfl + fx * k.half_dt) * rrho;
-    float uy = (momy(f) * k.inv_cfl + fy * k.half_dt) * rrho;
+    const V rrho = vrcp(rho);
+    const V mx = momx(f), my = momy(f);
+    V ux = vmul(vaxpy(k.half_dt, fx, vscale(k.inv_cfl, mx)), rrho);
+    V uy = vmul(vaxpy(k.half_dt, fy, vscale(k.inv_cfl, my)), rrho);
     if (lo) {
-        float m[9];
-        const I o1 = (I)nxp + (I)x;
+        V m[9];
         const float kf1 = __ldg(k.kref + 1);
         if (FIRST) {
-            own9s<S, I>(sf, pl, o1, m);
+            own9s<V, S>(src, pl, row_at(c, 1, nxp), m);
         } else {
-            pull9s<S, I>(sf, pl, nxp, x, 1, xm, xp, 0, 2, m);
+            pull9s<V, S>(src, pl, row_at(c, 1, nxp), r0, row_at(c, 2, nxp), m);
             reframe(m, __ldg(k.kref + 0) - kf1, __ldg(k.kref + 2) - kf1);
         }
-        const float rrho1 = 1.0f / (36.0f * kf1 + sum9f(m));
-        ux = -(momx(m) * k.inv_cfl + fx * k.half_dt) * rrho1;
-        uy = -(momy(m) * k.inv_cfl + fy * k.half_dt) * rrho1;
+        const V rrho1 = vrcp(vadd(bc<V>(36.0f * kf1), sum9f(m)));
+        ux = vmul(vaxpy(-k.half_dt, fx, vscale(-k.inv_cfl, momx(m))), rrho1);
+        uy = vmul(vaxpy(-k.half_dt, fy, vscale(-k.inv_cfl, momy(m))), rrho1);
     }
     if (moments) {
-        fields[(I)F_RHO * pl + o] = (double)Rf + (double)drho;
-        fields[(I)F_UX * pl + o] = ux;
-        fields[(I)F_UY * pl + o] = uy;
-        fields[(I)F_CP * pl + o] = (double)Rh + (double)dcp;
-        fields[(I)F_CN * pl + o] = (double)Rt + (double)dcn;
+        const V none = bc<V>(0.0f);
+        st_moment(fields + F_RHO * pl, c, r0, bc<V>(Rf), drho);
+        st_moment(fields + F_UX * pl, c, r0, none, ux);
+        st_moment(fields + F_UY * pl, c, r0, none, uy);
+        st_moment(fields + F_CP * pl, c, r0, Rh, dcp);
+        st_moment(fields + F_CN * pl, c, r0, Rt, dcn);
     }
     // right-hand side without its FP64 row constant (rhs_q (R+ - R-) and the
     // lifting's x-mean, added by the row pass), with the lifting's x-fluctuation
     if (!wall) {
-        float v = k.rhs_qf * dq;
-        if (y == 1) v -= __ldg(k.lift + x);
-        if (y == ny - 2) v -= __ldg(k.lift + k.nx + x);
-        st_field_f(k.rhsf + o, v, k.keep_l2);
+        V v = vscale(k.rhs_qf, dq);
+        if (y == 1) v = vsub(v, PerX<V>::own(k.lift, c));
+        if (y == ny - 2) v = vsub(v, PerX<V>::own(k.lift + nx, c));
+        st_rhs(k.rhsf, r0, v, k.keep_l2);
     }
     // ions: FP32 TRT, moment form (trt_f32)
-    {
-        {
-            const float vx = ux + k.mob_p * ex, vy = uy + k.mob_p * ey;
-            trt_f32<false, false>(h, dcp, Rh + dcp, vx, vy, vx * vx + vy * vy, k.wcp, k.wcm, k, 0.0f, 0.0f, 0.0f, 0.0f);
+    const V zero = bc<V>(0.0f);
+    const V usq = vfma(ux, ux, vmul(uy, uy));
+    trt_f32<false, false>(h, dcp, vadd(Rh, dcp), vaxpy(k.mob_p, ex, ux), vaxpy(k.mob_p, ey, uy), false, usq, k.wcp, k.wcm,
+                          k, zero, zero, zero, zero);
 #pragma unroll
-            for (int d = 0; d < 9; ++d) st_pop<S>(dst + ((I)(9 + d) * pl + o), h[d]);
-        }
-        {
-            const float vx = ux + k.mob_n * ex, vy = uy + k.mob_n * ey;
-            trt_f32<false, false>(t, dcn, Rt + dcn, vx, vy,
-                                  (k.flags & EK_FLAG_REST_QUIRK) ? ux * ux + uy * uy : vx * vx + vy * vy, k.wtp, k.wtm,
-                                  k, 0.0f, 0.0f, 0.0f, 0.0f);
+    for (int d = 0; d < 9; ++d) R::put(dst + (9 + d) * pl, r0, h[d]);
+    // c-: the quirk of LBM.cu:493, its rest equilibrium with the fluid's u^2
+    trt_f32<false, false>(t, dcn, vadd(Rt, dcn), vaxpy(k.mob_n, ex, ux), vaxpy(k.mob_n, ey, uy),
+                          (k.flags & EK_FLAG_REST_QUIRK) != 0, usq, k.wtp, k.wtm, k, zero, zero, zero, zero);
 #pragma unroll
-            for (int d = 0; d < 9; ++d) st_pop<S>(dst + ((I)(18 + d) * pl + o), t[d]);
-        }
-    }
+    for (int d = 0; d < 9; ++d) R::put(dst + (18 + d) * pl, r0, t[d]);
     S *df = dst;
     if (lo) {
-        st_pop<S>(df + o, f[0]);
+        R::put(df, r0, f[0]);
 #pragma unroll
-        for (int d = 1; d < 9; ++d) st_pop<S>(df + ((I)oppd(d) * pl + o), f[d]);
+        for (int d = 1; d < 9; ++d) R::put(df + oppd(d) * pl, r0, f[d]);
         return;
     }
     if (hi) {
-        st_pop<S>(df + o, f[0]);
-        st_pop<S>(df + (3 * pl + o), f[1] - k.ms);
-        st_pop<S>(df + (4 * pl + o), f[2]);
-        st_pop<S>(df + (1 * pl + o), f[3] + k.ms);
-        st_pop<S>(df + (2 * pl + o), f[4]);
-        st_pop<S>(df + (7 * pl + o), f[5] - k.md);
-        st_pop<S>(df + (8 * pl + o), f[6] + k.md);
-        st_pop<S>(df + (5 * pl + o), f[7] + k.md);
-        st_pop<S>(df + (6 * pl + o), f[8] - k.md);
+        const V ms = bc<V>(k.ms), md = bc<V>(k.md);
+        R::put(df, r0, f[0]);
+        R::put(df + 3 * pl, r0, vsub(f[1], ms));
+        R::put(df + 4 * pl, r0, f[2]);
+        R::put(df + 1 * pl, r0, vadd(f[3], ms));
+        R::put(df + 2 * pl, r0, f[4]);
+        R::put(df + 7 * pl, r0, vsub(f[5], md));
+        R::put(df + 8 * pl, r0, vadd(f[6], md));
+        R::put(df + 5 * pl, r0, vadd(f[7], md));
+        R::put(df + 6 * pl, r0, vsub(f[8], md));
         return;
     }
     // fluid: FP32 TRT with the Guo source, moment form (trt_f32); the
     // population momentum with the half force, cfl rho u
-    const float px = momx(f) + k.cfl_hdt * fx, py = momy(f) + k.cfl_hdt * fy;
-    if (k.flags & EK_FLAG_FORCE)
-        trt_f32<true, true>(f, drho, rho, ux, uy, ux * ux + uy * uy, k.wp, k.wm, k, fx, fy, px, py);
+    const V px = vaxpy(k.cfl_hdt, fx, mx), py = vaxpy(k.cfl_hdt, fy, my);
+    if (force)
+        trt_f32<true, true>(f, drho, rho, ux, uy, false, usq, k.wp, k.wm, k, fx, fy, px, py);
     else
-        trt_f32<false, true>(f, drho, rho, ux, uy, ux * ux + uy * uy, k.wp, k.wm, k, 0.0f, 0.0f, px, py);
+        trt_f32<false, true>(f, drho, rho, ux, uy, false, usq, k.wp, k.wm, k, zero, zero, px, py);
 #pragma unroll
-    for (int d = 0; d < 9; ++d) st_pop<S>(df + ((I)d * pl + o), f[d]);
+    for (int d = 0; d < 9; ++d) R::put(df + d * pl, r0, f[d]);
 }
 
-template <typename S, bool FIRST, bool EXPLICIT_E, typename I = size_t>
+// The step of the node x, or of the nodes x and x + 1 (V = float2, x even).
+template <typename S, bool FIRST, bool EXPLICIT_E, typename V>
 __device__ __forceinline__ void node_shifted(const ChanF &k, const S *__restrict__ src, S *__restrict__ dst,
-                                             double *__restrict__ fields, int x, int y, bool moments, int sbuf) {
-    float f[9], h[9], t[9];
-    gather_global<S, FIRST, I>(k, src, x, y, f, h, t);
-    collide_shifted<S, FIRST, EXPLICIT_E, I>(k, f, h, t, src, dst, fields, x, y, moments, sbuf);
+                                             double *__restrict__ fields, int x, int y, bool moments, int sbuf,
+                                             bool wait) {
+    const Cols c = make_cols<V>(x, k.nx);
+    V f[9], h[9], t[9];
+    gather_global<S, FIRST, V>(k, src, c, y, f, h, t);
+    if (wait) pdl_wait();  // the populations are in flight; psi comes from the kernel before (StepChain)
+    collide_shifted<S, FIRST, EXPLICIT_E, V>(k, f, h, t, src, dst, fields, c, y, moments, sbuf);
 }
 
 // Equilibrium deviations from the fields (pre-collision layout), written to

@@ -173,11 +173,13 @@ __device__ __forceinline__ void gather_f64(const Chan &c, const double *__restri
 // The update of node (x, y) from its raw populations (gather_f64): ion
 // anti-bounce-back at the walls, moments, E, force, right-hand side,
 // equilibria, Guo source, TRT and the stores.  src is read only for the lower
-// wall's row-1 pull.
-template <bool FIRST, bool EXPLICIT_E, bool MOMENTS, typename I>
+// wall's row-1 pull.  `moments` is a run-time flag: as a template parameter it
+// gave two bodies whose multiply-adds the compiler fused differently, so a
+// step that wrote the moments could round differently from one that did not.
+template <bool FIRST, bool EXPLICIT_E, typename I>
 __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_raw[9], double tt_raw[9],
                                          const double *__restrict__ src, double *__restrict__ dst,
-                                         double *__restrict__ fields, int x, int y) {
+                                         double *__restrict__ fields, int x, int y, bool moments) {
     const I pl = (I)c.plane;
     const int nxp = c.nxp;
     const I o = (I)y * (I)nxp + (I)x;
@@ -226,7 +228,7 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
         ux = -rhoinvm * ((fm[1] + fm[5] + fm[8] - (fm[3] + fm[6] + fm[7])) / c.cfl + forcex * c.dt * 0.5);
         uy = -rhoinvm * ((fm[2] + fm[5] + fm[6] - (fm[4] + fm[7] + fm[8])) / c.cfl + forcey * c.dt * 0.5);
     }
-    if (MOMENTS) {
+    if (moments) {
         fields[F_RHO * pl + o] = rho;
         fields[F_UX * pl + o] = ux;
         fields[F_UY * pl + o] = uy;
@@ -304,16 +306,17 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
     for (int d = 0; d < 9; ++d) df[d * pl + o] = out[d] + dt * src9[d];
 }
 
-template <bool FIRST, bool EXPLICIT_E, bool MOMENTS, typename I>
+template <bool FIRST, bool EXPLICIT_E, typename I>
 __global__ void __launch_bounds__(TPB)
 step_f64(const Chan c, const double *__restrict__ src, double *__restrict__ dst,
-         double *__restrict__ fields) {
-    const int x = blockIdx.x * TPB + threadIdx.x;
-    const int y = blockIdx.y;
-    if (x >= c.nx) return;
+         double *__restrict__ fields, bool moments, bool wait) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= c.nx || y >= c.ny) return;
     double ft[9], ht[9], tt[9];
     gather_f64<FIRST, I>(c, src, x, y, ft, ht, tt);
-    node_f64<FIRST, EXPLICIT_E, MOMENTS, I>(c, ft, ht, tt, src, dst, fields, x, y);
+    if (wait) pdl_wait();  // the populations are in flight; psi comes from the kernel before (StepChain)
+    node_f64<FIRST, EXPLICIT_E, I>(c, ft, ht, tt, src, dst, fields, x, y, moments);
 }
 
 __global__ void rates_kernel(ek_params p, Rates *out) {
@@ -413,28 +416,24 @@ cudaError_t launch_init_f64(const Chan &c, double *pops, const double *fields, b
 }
 
 cudaError_t launch_step_f64(const Chan &c, const double *src, double *dst, double *fields,
-                            bool first, bool explicit_e, bool moments, cudaStream_t s) {
-    const dim3 g = node_grid(c, c.ny);
+                            bool first, bool explicit_e, bool moments, int chain, cudaStream_t s) {
+    // blocks of narrow channels take several rows
+    int tx = 16;
+    while (tx < TPB && tx < c.nx) tx *= 2;
+    const dim3 t(tx, TPB / tx), g((c.nx + tx - 1) / tx, (c.ny + TPB / tx - 1) / (TPB / tx));
+    const bool wait = chain != CHAIN_NONE, pdl = chain == CHAIN_NEXT;
     // 32-bit offsets while the 27 population planes fit 2^32 elements
     const bool i32 = (size_t)27 * c.plane < ((size_t)1 << 32);
-#define EK_STEP(F, E, M)                                                                       \
-    do {                                                                                       \
-        if (i32) step_f64<F, E, M, uint32_t><<<g, TPB, 0, s>>>(c, src, dst, fields);           \
-        else step_f64<F, E, M, size_t><<<g, TPB, 0, s>>>(c, src, dst, fields);                 \
-    } while (0)
-    const int key = (first ? 4 : 0) | (explicit_e ? 2 : 0) | (moments ? 1 : 0);
-    switch (key) {
-        case 0: EK_STEP(false, false, false); break;
-        case 1: EK_STEP(false, false, true); break;
-        case 2: EK_STEP(false, true, false); break;
-        case 3: EK_STEP(false, true, true); break;
-        case 4: EK_STEP(true, false, false); break;
-        case 5: EK_STEP(true, false, true); break;
-        case 6: EK_STEP(true, true, false); break;
-        default: EK_STEP(true, true, true); break;
+#define EK_STEP(F, E)                                                                                               \
+    return i32 ? launch_maybe_pdl(pdl, step_f64<F, E, uint32_t>, g, t, 0, s, c, src, dst, fields, moments, wait)    \
+               : launch_maybe_pdl(pdl, step_f64<F, E, size_t>, g, t, 0, s, c, src, dst, fields, moments, wait)
+    switch ((first ? 2 : 0) | (explicit_e ? 1 : 0)) {
+        case 0: EK_STEP(false, false);
+        case 1: EK_STEP(false, true);
+        case 2: EK_STEP(true, false);
+        default: EK_STEP(true, true);
     }
 #undef EK_STEP
-    return cudaGetLastError();
 }
 
 cudaError_t launch_efield_f64(const Chan &c, double *fields, cudaStream_t s) {

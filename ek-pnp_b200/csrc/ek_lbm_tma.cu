@@ -175,7 +175,8 @@ step_tma(const __grid_constant__ CUtensorMap tsrc, const ChanF k, const S *__res
                     v[plane] = ld_pop<S>(src + plane * pl + (size_t)row * k.nxp + xs);
                 }
             }
-            collide_shifted<S, FIRST, EE>(k, v, v + 9, v + 18, src, dst, fields, x, y, mom, sbuf);
+            collide_shifted<S, FIRST, EE, float>(k, v, v + 9, v + 18, src, dst, fields, make_cols<float>(x, k.nx), y, mom,
+                                                sbuf);
         }
     }
 }

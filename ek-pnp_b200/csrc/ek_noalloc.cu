@@ -211,7 +211,6 @@ extern "C" int ek_poisson_noalloc(const ek_params *p, const double *cp, const do
     if (e != cudaSuccess || dev < 0 || dev >= NA_MAX_DEVICES) return na_fail(EK_ERR_CUDA, "cudaGetDevice");
     Scratch sc;
     if ((e = scratch_for(dev, &sc)) != cudaSuccess) return na_fail(EK_ERR_CUDA, cudaGetErrorString(e));
-    if ((e = poisson_set_smem_limits()) != cudaSuccess) return na_fail(EK_ERR_CUDA, cudaGetErrorString(e));
 
     PoissonPlan pp{};
     pp.nx = nx;
@@ -226,6 +225,7 @@ extern "C" int ek_poisson_noalloc(const ek_params *p, const double *cp, const do
     pp.tw = sc.tw;
     pp.piv = sc.piv;
     pp.spec = sc.spec;
+    if ((e = poisson_set_smem_limits(pp)) != cudaSuccess) return na_fail(EK_ERR_CUDA, cudaGetErrorString(e));
     Chan c{};
     c.nx = nx;
     c.ny = ny;

@@ -11,8 +11,8 @@
 // and this file solves it directly (Thomas recurrence with pivots computed
 // once per channel), for any ny, with no FFT in y:
 //   pass A  per pair of interior rows: real FFT in x (two rows packed as one
-//           complex row; register-blocked radix-16 passes for powers of two,
-//           direct DFT otherwise) -> spec[j][m], m = 0..nx/2
+//           complex row; register-blocked radix-16 passes for powers of two
+//           from 16 on, mixed radix otherwise) -> spec[j][m], m = 0..nx/2
 //   pass B  per x-mode m: Thomas sweeps down the column, partitioned into row
 //           segments of at most 16 rows held in registers (one thread per
 //           mode for columns taller than 8192 rows)
@@ -20,7 +20,7 @@
 // The result equals the reference's to rounding (the test suite compares).
 #include <cuda_runtime.h>
 
-#include "ek_fft32.cuh"
+#include "ek_fft16.cuh"
 #include "ek_internal.h"
 
 namespace ek {
@@ -38,66 +38,138 @@ __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y
 template <typename C> __device__ __forceinline__ C cmake(double a, double b);
 template <> __device__ __forceinline__ double2 cmake<double2>(double a, double b) { return make_double2(a, b); }
 template <> __device__ __forceinline__ float2 cmake<float2>(double a, double b) { return make_float2((float)a, (float)b); }
+__device__ __forceinline__ int brev(int i, int lg) { return (int)(__brev((unsigned)i) >> (32 - lg)); }
 
-// In-place radix-2 decimation-in-time FFT of n = 2^lg points already in
-// bit-reversed order in shared memory.  inv selects the +i exponent.
-__device__ void fft_smem(double2 *s, int n, const double2 *__restrict__ tw, bool inv) {
-    for (int len = 2; len <= n; len <<= 1) {
-        const int half = len >> 1, stride = n / len;
-        for (int t = threadIdx.x; t < (n >> 1); t += blockDim.x) {
-            const int k = t & (half - 1);
-            const int i = (t - k) * 2 + k;
-            double2 w = __ldg(tw + k * stride);
-            if (inv) w = cconj(w);
-            const double2 u = s[i], v = cmul(s[i + half], w);
-            s[i] = cadd(u, v);
-            s[i + half] = csub(u, v);
+// ---- rows of any length (FP64): mixed radix --------------------------------
+//
+// nx = r_1 r_2 ... (Stockham, self-sorting, two buffers in shared memory).  With
+// L = r_1 ... r_{i-1} the transforms of length L done so far, pass i takes the
+// elements j + q nx/r (q < r), j < nx/r, to (j/L) L r + j mod L + q' L, with
+// the twiddle exp(-2 pi i (j mod L) q / (L r)) and an r-point DFT.  Radices 4,
+// 2, 3 and 5 are butterflies held by a thread; any other prime r is summed
+// term by term, one output a thread: nx r products instead of the nx^2 of
+// the direct transform, which took 211 us (inverse 263) at 1000 x 257 on B200
+// against 10 (9) us here.  All roots are powers of the nx-th root from the table.
+struct Radices {
+    int n;
+    int r[11];  // nx <= 2048 = 4^5 2
+};
+
+template <bool INV> __device__ __forceinline__ double2 root(const double2 *__restrict__ tw, int k) {
+    const double2 w = __ldg(tw + k);
+    return INV ? cconj(w) : w;
+}
+// z times -i (forward) or +i (inverse)
+template <bool INV> __device__ __forceinline__ double2 rot90(double2 z) {
+    return INV ? make_double2(-z.y, z.x) : make_double2(z.y, -z.x);
+}
+
+template <bool INV, int R>
+__device__ __forceinline__ void radix_pass(const double2 *__restrict__ in, double2 *__restrict__ out, int nx, int L,
+                                           const double2 *__restrict__ tw) {
+    const int m = nx / R, ts = nx / (L * R);
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const int hi = j / L, k = j - hi * L;
+        double2 x[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            x[q] = in[j + q * m];
+            if (q > 0 && k > 0) x[q] = cmul(x[q], root<INV>(tw, k * q * ts));
         }
-        __syncthreads();
+        double2 *o = out + hi * L * R + k;
+        if constexpr (R == 2) {
+            o[0] = cadd(x[0], x[1]);
+            o[L] = csub(x[0], x[1]);
+        } else if constexpr (R == 4) {
+            const double2 s0 = cadd(x[0], x[2]), d0 = csub(x[0], x[2]), s1 = cadd(x[1], x[3]);
+            const double2 d1 = rot90<INV>(csub(x[1], x[3]));
+            o[0] = cadd(s0, s1);
+            o[L] = cadd(d0, d1);
+            o[2 * L] = csub(s0, s1);
+            o[3 * L] = csub(d0, d1);
+        } else if constexpr (R == 3) {
+            constexpr double h = 0.86602540378443865;  // sin(pi/3)
+            const double2 s = cadd(x[1], x[2]), d = rot90<INV>(csub(x[1], x[2]));
+            const double2 c = make_double2(x[0].x - 0.5 * s.x, x[0].y - 0.5 * s.y);
+            o[0] = cadd(x[0], s);
+            o[L] = make_double2(c.x + h * d.x, c.y + h * d.y);
+            o[2 * L] = make_double2(c.x - h * d.x, c.y - h * d.y);
+        } else {
+            static_assert(R == 5, "radices 2 to 5");
+            constexpr double c1 = 0.30901699437494742, c2 = -0.80901699437494742;  // cos(2 pi/5), cos(4 pi/5)
+            constexpr double s1 = 0.95105651629515357, s2 = 0.58778525229247313;   // sin(2 pi/5), sin(4 pi/5)
+            const double2 a1 = cadd(x[1], x[4]), a2 = cadd(x[2], x[3]);
+            const double2 b1 = rot90<INV>(csub(x[1], x[4])), b2 = rot90<INV>(csub(x[2], x[3]));
+            const double2 e1 = make_double2(x[0].x + c1 * a1.x + c2 * a2.x, x[0].y + c1 * a1.y + c2 * a2.y);
+            const double2 e2 = make_double2(x[0].x + c2 * a1.x + c1 * a2.x, x[0].y + c2 * a1.y + c1 * a2.y);
+            const double2 f1 = make_double2(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y);
+            const double2 f2 = make_double2(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y);
+            o[0] = cadd(x[0], cadd(a1, a2));
+            o[L] = cadd(e1, f1);
+            o[2 * L] = cadd(e2, f2);
+            o[3 * L] = csub(e2, f2);
+            o[4 * L] = csub(e1, f1);
+        }
     }
 }
 
-// Direct DFT of z (n points, any n) into out, both in shared memory.
-__device__ void dft_smem(const double2 *z, double2 *out, int n, const double2 *__restrict__ tw, bool inv) {
-    for (int m = threadIdx.x; m < n; m += blockDim.x) {
-        double2 acc = make_double2(0.0, 0.0);
+// A pass of prime radix r > 5: one output a thread, its r terms summed in order.
+template <bool INV>
+__device__ __forceinline__ void prime_pass(const double2 *__restrict__ in, double2 *__restrict__ out, int nx, int L,
+                                           int r, const double2 *__restrict__ tw) {
+    const int m = nx / r, ts = nx / (L * r);
+    for (int e = threadIdx.x; e < nx; e += blockDim.x) {
+        const int qo = e / m, j = e - qo * m, hi = j / L, k = j - hi * L;
+        // exponent of term q: q (k ts + qo m) mod nx
+        int step = k * ts + qo * m;
+        if (step >= nx) step -= nx;
+        double2 acc = in[j];
         int idx = 0;
-        for (int x = 0; x < n; ++x) {
-            double2 w = __ldg(tw + idx);
-            if (inv) w = cconj(w);
-            acc = cadd(acc, cmul(z[x], w));
-            idx += m;
-            if (idx >= n) idx -= n;
+        for (int q = 1; q < r; ++q) {
+            idx += step;
+            if (idx >= nx) idx -= nx;
+            acc = cadd(acc, cmul(in[j + q * m], root<INV>(tw, idx)));
         }
-        out[m] = acc;
+        out[hi * L * r + k + qo * L] = acc;
+    }
+}
+
+// Transform of nx points in a (b: the other buffer), natural order in and out;
+// returns the buffer that holds the result.  Every thread of the block calls it.
+template <bool INV>
+__device__ double2 *mixed_fft(double2 *a, double2 *b, int nx, const Radices &f, const double2 *__restrict__ tw) {
+    int L = 1;
+    for (int i = 0; i < f.n; ++i) {
+        const int r = f.r[i];
+        __syncthreads();
+        switch (r) {
+            case 2: radix_pass<INV, 2>(a, b, nx, L, tw); break;
+            case 3: radix_pass<INV, 3>(a, b, nx, L, tw); break;
+            case 4: radix_pass<INV, 4>(a, b, nx, L, tw); break;
+            case 5: radix_pass<INV, 5>(a, b, nx, L, tw); break;
+            default: prime_pass<INV>(a, b, nx, L, r, tw); break;
+        }
+        double2 *t = a;
+        a = b;
+        b = t;
+        L *= r;
     }
     __syncthreads();
+    return a;
 }
 
 // Pass A: rows y0 = 2*b+1 and y1 = y0+1 of the right-hand side -> spectra.
 __global__ void __launch_bounds__(PTPB)
-fwd_rows(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
+fwd_rows(const PoissonPlan pp, const Radices f, const double *__restrict__ rhs, int nxp) {
     extern __shared__ double2 sm[];
+    pdl_wait();
     const int nx = pp.nx;
     const int j0 = 2 * blockIdx.x, j1 = j0 + 1;
     const bool two = j1 < pp.n;
     const double *r0 = rhs + (size_t)(j0 + 1) * nxp;
     const double *r1 = rhs + (size_t)(j1 + 1) * nxp;
-    double2 *z = sm;
-    if (pp.pow2) {
-        const int sh = 32 - pp.log2nx;
-        for (int x = threadIdx.x; x < nx; x += blockDim.x) {
-            const int rx = pp.log2nx ? (int)(__brev((unsigned)x) >> sh) : 0;
-            z[rx] = make_double2(r0[x], two ? r1[x] : 0.0);
-        }
-        __syncthreads();
-        fft_smem(z, nx, pp.tw, false);
-    } else {
-        double2 *in = sm + nx;
-        for (int x = threadIdx.x; x < nx; x += blockDim.x) in[x] = make_double2(r0[x], two ? r1[x] : 0.0);
-        __syncthreads();
-        dft_smem(in, z, nx, pp.tw, false);
-    }
+    for (int x = threadIdx.x; x < nx; x += blockDim.x) sm[x] = make_double2(r0[x], two ? r1[x] : 0.0);
+    const double2 *z = mixed_fft<false>(sm, sm + nx, nx, f, pp.tw);
     // unpack the two real-input spectra: A = (Z[m] + conj Z[-m])/2, B = (Z[m] - conj Z[-m])/(2i)
     double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
     for (int m = threadIdx.x; m <= nx / 2; m += blockDim.x) {
@@ -111,6 +183,7 @@ fwd_rows(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
 // piv[j][m] = 1/(b_m - piv[j-1][m]) with b_m = -(2 + kx_m^2 dy^2).
 __global__ void __launch_bounds__(PTPB) tridiag(const PoissonPlan pp) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (m > pp.nx / 2) return;
     const size_t mp = pp.mp;
     double2 *col = pp.spec + m;
@@ -149,33 +222,22 @@ __device__ __forceinline__ void write_walls(double *__restrict__ psi, const doub
 
 // Pass C: spectra of rows (y0, y1) -> psi rows; the walls spread over the blocks.
 __global__ void __launch_bounds__(PTPB)
-inv_rows(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
+inv_rows(const PoissonPlan pp, const Radices f, const Chan c, double *__restrict__ psi) {
     extern __shared__ double2 sm[];
+    pdl_wait();
     const int nx = pp.nx, nxp = c.nxp;
     write_walls(psi, c.zlo, c.zhi, nx, c.ny, nxp, blockIdx.x, gridDim.x, blockDim.x);
     const int j0 = 2 * blockIdx.x, j1 = j0 + 1;
     const bool two = j1 < pp.n;
     const double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
-    double2 *z = sm;
-    double2 *dst = pp.pow2 ? sm : sm + nx;
-    const int sh = 32 - pp.log2nx;
     for (int m = threadIdx.x; m <= nx / 2; m += blockDim.x) {
         const double2 a = s0[m];
         const double2 b = two ? s1[m] : make_double2(0.0, 0.0);
         // Z[m] = A + iB, Z[-m] = conj(A) + i conj(B)
-        const double2 zp = make_double2(a.x - b.y, a.y + b.x);
-        const double2 zn = make_double2(a.x + b.y, -a.y + b.x);
-        if (pp.pow2) {
-            z[pp.log2nx ? (int)(__brev((unsigned)m) >> sh) : 0] = zp;
-            if (m != 0 && 2 * m != nx) z[(int)(__brev((unsigned)(nx - m)) >> sh)] = zn;
-        } else {
-            dst[m] = zp;
-            if (m != 0 && 2 * m != nx) dst[nx - m] = zn;
-        }
+        sm[m] = make_double2(a.x - b.y, a.y + b.x);
+        if (m != 0 && 2 * m != nx) sm[nx - m] = make_double2(a.x + b.y, -a.y + b.x);
     }
-    __syncthreads();
-    if (pp.pow2) fft_smem(z, nx, pp.tw, true);
-    else dft_smem(dst, z, nx, pp.tw, true);
+    const double2 *z = mixed_fft<true>(sm, sm + nx, nx, f, pp.tw);
     const double inv = 1.0 / (double)nx;
     double *p0 = psi + (size_t)(j0 + 1) * nxp, *p1 = psi + (size_t)(j1 + 1) * nxp;
     for (int x = threadIdx.x; x < nx; x += blockDim.x) {
@@ -184,199 +246,86 @@ inv_rows(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
     }
 }
 
-// ---- register-blocked radix-16 row FFTs (power-of-two nx >= 16) ----------
+// ---- radix-16 row transforms (power-of-two nx >= 16) -----------------------
 //
-// Each thread holds up to 16 complex values and runs up to four radix-2
-// stages on them in registers per pass; passes exchange through shared
-// memory.  The forward transform is decimation in frequency on natural-order
-// input (bit-reversed output); the inverse is decimation in time on
-// bit-reversed input (natural-order output).  A pass over index bits
-// [b, b+RB) owns the 2^RB elements that share every other index bit; thread t
-// of the T = nx/16 threads of one transform owns 16/2^RB such groups.
-// Twiddle of stage st for element index i: exp(-2 pi i (i mod 2^st)/2^(st+1))
-// = A * C with A = exp(-2 pi i (base mod 2^b)/2^(st+1)) from the table (one
-// load per group and stage) and C = exp(-2 pi i v_low/2^(st-b+1)) a constant
-// root of unity of order <= 16 for the in-register index bits v_low.
-// Shared memory is addressed through swz(): the low three index bits are
-// XOR-ed with bits 4..6 and with the reversed top three bits, which keeps
-// both the passes and the bit-reversed unpacking free of bank conflicts.
+// Compiled per size K = log2 nx (ek_fft16.cuh), T = nx/16 threads a row pair.
+// Blocks are small -- 64 threads up to nx = 1024, else one row pair -- so that
+// a channel of a hundred rows spreads over the GPU: with 256 threads a block,
+// 256 x 128 ran on 4 SMs (FP64: 14 us forward, 11 us inverse) and 512 x 203 on
+// 13 (FP32: 8.5 and 7.6 us).
+template <int K> struct RowCfg {
+    static constexpr int N = 1 << K, T = N >> 4;
+    static constexpr int block = T <= 64 ? 64 : T;  // threads
+    static constexpr int per = block / T;           // row pairs a block
+};
+#define EK_ROW_CASES(F) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13)
 
-__device__ __forceinline__ int brev(int i, int lg) { return (int)(__brev((unsigned)i) >> (32 - lg)); }
-__device__ __forceinline__ int swz(int i, int k) {
-    if (k < 6) return i;
-    const int top = (i >> (k - 3)) & 7;
-    const int rtop = ((top & 1) << 2) | (top & 2) | ((top >> 2) & 1);
-    return i ^ (((i >> 4) ^ rtop) & 7);
-}
-
-// Shared-memory index of element i of a transform (the FP64 form; the FP32
-// row transforms of ek_fft32.cuh have their own map).
-template <typename C> __device__ __forceinline__ int sidx(int i, int k, int p);
-template <> __device__ __forceinline__ int sidx<double2>(int i, int k, int) { return swz(i, k); }
-
-// exp(-2 pi i v/2^(sl+1)) for 0 <= v < 2^sl <= 8 (compile-time arguments)
-template <typename C>
-__device__ __forceinline__ C root16(int sl, int v) {
-    const int q = v << (3 - sl);  // angle = q * pi/8
-    switch (q) {
-        case 0: return cmake<C>(1.0, 0.0);
-        case 1: return cmake<C>(0.92387953251128674, -0.38268343236508977);
-        case 2: return cmake<C>(0.70710678118654752, -0.70710678118654752);
-        case 3: return cmake<C>(0.38268343236508977, -0.92387953251128674);
-        case 4: return cmake<C>(0.0, -1.0);
-        case 5: return cmake<C>(-0.38268343236508977, -0.92387953251128674);
-        case 6: return cmake<C>(-0.70710678118654752, -0.70710678118654752);
-        default: return cmake<C>(-0.92387953251128674, -0.38268343236508977);
-    }
-}
-
-template <bool INV, int RB, typename C>
-__device__ __forceinline__ void reg_pass(C *s, int k, int T, int t, int b, const C *__restrict__ tw, int p) {
-    constexpr int G = 16 >> RB, E = 1 << RB;
-    const int ngroups = (1 << k) >> RB;
-#pragma unroll
-    for (int q = 0; q < G; ++q) {
-        const int g = t + q * T;
-        if (g >= ngroups) continue;
-        const int kb = g & ((1 << b) - 1);
-        const int base = kb | ((g >> b) << (b + RB));
-        C r[E];
-#pragma unroll
-        for (int v = 0; v < E; ++v) r[v] = s[sidx<C>(base | (v << b), k, p)];
-        if (!INV) {
-#pragma unroll
-            for (int sl = RB - 1; sl >= 0; --sl) {
-                const int st = b + sl;
-                const C A = __ldg(tw + (kb << (k - st - 1)));
-#pragma unroll
-                for (int v = 0; v < E; ++v) {
-                    if (v & (1 << sl)) continue;
-                    const C w = cmul(A, root16<C>(sl, v & ((1 << sl) - 1)));
-                    const C u = r[v], x = r[v + (1 << sl)];
-                    r[v] = cadd(u, x);
-                    r[v + (1 << sl)] = cmul(csub(u, x), w);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int sl = 0; sl < RB; ++sl) {
-                const int st = b + sl;
-                const C A = cconj(__ldg(tw + (kb << (k - st - 1))));
-#pragma unroll
-                for (int v = 0; v < E; ++v) {
-                    if (v & (1 << sl)) continue;
-                    const C w = cmul(A, cconj(root16<C>(sl, v & ((1 << sl) - 1))));
-                    const C u = r[v], x = cmul(r[v + (1 << sl)], w);
-                    r[v] = cadd(u, x);
-                    r[v + (1 << sl)] = csub(u, x);
-                }
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < E; ++v) s[sidx<C>(base | (v << b), k, p)] = r[v];
-    }
-}
-
-template <bool INV, typename C>
-__device__ __forceinline__ void reg_pass_any(C *s, int k, int T, int t, int b, int rb, const C *tw, int p) {
-    switch (rb) {
-        case 4: reg_pass<INV, 4, C>(s, k, T, t, b, tw, p); break;
-        case 3: reg_pass<INV, 3, C>(s, k, T, t, b, tw, p); break;
-        case 2: reg_pass<INV, 2, C>(s, k, T, t, b, tw, p); break;
-        default: reg_pass<INV, 1, C>(s, k, T, t, b, tw, p); break;
-    }
-}
-
-// Whole transform of 2^k points in s; every thread of the block calls it.
-template <bool INV, typename C>
-__device__ void reg_fft(C *s, int k, int T, int t, const C *__restrict__ tw, int p) {
-    if (!INV) {
-        for (int top = k; top > 0;) {
-            const int rb = top < 4 ? top : 4;
-            reg_pass_any<false, C>(s, k, T, t, top - rb, rb, tw, p);
-            __syncthreads();
-            top -= rb;
-        }
-    } else {
-        for (int b = 0; b < k;) {
-            const int rb = k - b < 4 ? k - b : 4;
-            reg_pass_any<true, C>(s, k, T, t, b, rb, tw, p);
-            __syncthreads();
-            b += rb;
-        }
-    }
-}
-
-// Pass A, radix-16 form: row pairs (2p+1, 2p+2) of the right-hand side ->
-// spectra.  One block holds BLOCK/T row pairs.
-template <int BLOCK>
-__device__ __forceinline__ void fwd_rows_r16_dev(const PoissonPlan &pp, const double *__restrict__ rhs, int nxp,
-                                                 int pair_base, double2 *sm) {
-    const int N = pp.nx, k = pp.log2nx, T = N >> 4;
+// Pass A, FP64: row pairs (2p+1, 2p+2) of the right-hand side -> spectra.  The
+// first radix-16 pass runs on the values as loaded.
+template <int K>
+__global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
+fwd_rows_f64(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
+    extern __shared__ double2 sm[];
+    using S = fft16::Shape<K>;
+    constexpr int N = S::N, T = S::T;
+    pdl_wait();
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
-    const int pair = pair_base + p;
     double2 *s = sm + p * N;
-    const int j0 = 2 * pair, j1 = j0 + 1;
+    const int j0 = 2 * (blockIdx.x * RowCfg<K>::per + p), j1 = j0 + 1;
     const bool live = j0 < pp.n, two = j1 < pp.n;
-    const double *r0 = rhs + (size_t)(j0 + 1) * nxp, *r1 = rhs + (size_t)(j1 + 1) * nxp;
-    for (int x = t; x < N; x += T)
-        s[swz(x, k)] = live ? make_double2(__ldg(r0 + x), two ? __ldg(r1 + x) : 0.0) : make_double2(0.0, 0.0);
+    const double *r0 = rhs + (size_t)(j0 + 1) * nxp + t, *r1 = r0 + nxp;
+    double2 x[16];
+#pragma unroll
+    for (int v = 0; v < 16; ++v) x[v] = make_double2(live ? __ldg(r0 + v * T) : 0.0, two ? __ldg(r1 + v * T) : 0.0);
+    fft16::fwd_pass_store<K, 1>(x, s, t, p, pp.tw);
     __syncthreads();
-    reg_fft<false, double2>(s, k, T, t, pp.tw, p);
+    fft16::fwd_rest<K, 2>(s, t, p, pp.tw);
     if (!live) return;
     double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
     for (int m = t; m <= N / 2; m += T) {
-        const double2 a = s[swz(brev(m, k), k)], b = cconj(s[swz(brev((N - m) & (N - 1), k), k)]);
+        const double2 a = s[fft16::swz_base(brev(m, K), p)];
+        const double2 b = cconj(s[fft16::swz_base(brev((N - m) & (N - 1), K), p)]);
         s0[m] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
         if (two) s1[m] = make_double2(0.5 * (a.y - b.y), -0.5 * (a.x - b.x));
     }
 }
 
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
-fwd_rows_r16(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
+// Pass C, FP64: spectra -> psi rows (stored from registers by the last
+// radix-16 pass) and the walls.
+template <int K>
+__global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
+inv_rows_f64(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
     extern __shared__ double2 sm[];
-    fwd_rows_r16_dev<BLOCK>(pp, rhs, nxp, blockIdx.x * (BLOCK / (pp.nx >> 4)), sm);
-}
-
-// Pass C, radix-16 form: spectra -> psi rows and the walls.
-template <int BLOCK>
-__device__ __forceinline__ void inv_rows_r16_dev(const PoissonPlan &pp, int nxp, int ny, const double *zlo,
-                                                 const double *zhi, double *__restrict__ psi, int pair_base,
-                                                 double2 *sm) {
-    const int N = pp.nx, k = pp.log2nx, T = N >> 4;
+    using S = fft16::Shape<K>;
+    constexpr int N = S::N, T = S::T;
+    pdl_wait();
+    write_walls(psi, c.zlo, c.zhi, N, c.ny, c.nxp, blockIdx.x, gridDim.x, blockDim.x);
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
-    const int pair = pair_base + p;
     double2 *s = sm + p * N;
-    const int j0 = 2 * pair, j1 = j0 + 1;
+    const int j0 = 2 * (blockIdx.x * RowCfg<K>::per + p), j1 = j0 + 1;
     const bool live = j0 < pp.n, two = j1 < pp.n;
-    const int per = BLOCK / T;
-    write_walls(psi, zlo, zhi, N, ny, nxp, pair_base / per, ((pp.n + 1) / 2 + per - 1) / per, BLOCK);
     const double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
-    for (int m = t; m <= N / 2; m += T) {
-        const double2 a = live ? s0[m] : make_double2(0.0, 0.0);
-        const double2 b = two ? s1[m] : make_double2(0.0, 0.0);
-        s[swz(brev(m, k), k)] = make_double2(a.x - b.y, a.y + b.x);  // A + iB
-        if (m != 0 && 2 * m != N) s[swz(brev(N - m, k), k)] = make_double2(a.x + b.y, -a.y + b.x);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        const int m = t + i * T;
+        if (i == 8 && t != 0) break;
+        const double2 a = live ? s0[m] : make_double2(0.0, 0.0), b = two ? s1[m] : make_double2(0.0, 0.0);
+        s[fft16::swz_base(brev(m, K), p)] = make_double2(a.x - b.y, a.y + b.x);  // A + iB
+        if (m != 0 && 2 * m != N) s[fft16::swz_base(brev(N - m, K), p)] = make_double2(a.x + b.y, -a.y + b.x);
     }
     __syncthreads();
-    reg_fft<true, double2>(s, k, T, t, pp.tw, p);
-    const double inv = 1.0 / (double)N;
-    if (live) {
-        double *p0 = psi + (size_t)(j0 + 1) * nxp, *p1 = psi + (size_t)(j1 + 1) * nxp;
-        for (int x = t; x < N; x += T) {
-            const double2 z = s[swz(x, k)];
-            p0[x] = z.x * inv;
-            if (two) p1[x] = z.y * inv;
-        }
+    fft16::inv_partial<K>(s, t, p);
+    fft16::inv_full<K, S::NF>(s, t, p, pp.tw);
+    double2 x[16];
+    fft16::inv_pass_load<K, 1>(x, s, t, p, pp.tw);
+    if (!live) return;
+    constexpr double inv = 1.0 / (double)N;
+    double *p0 = psi + (size_t)(j0 + 1) * c.nxp + t, *p1 = p0 + c.nxp;
+#pragma unroll
+    for (int v = 0; v < 16; ++v) {
+        p0[v * T] = x[v].x * inv;
+        if (two) p1[v * T] = x[v].y * inv;
     }
-}
-
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
-inv_rows_r16(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
-    extern __shared__ double2 sm[];
-    inv_rows_r16_dev<BLOCK>(pp, c.nxp, c.ny, c.zlo, c.zhi, psi, blockIdx.x * (BLOCK / (pp.nx >> 4)), sm);
 }
 
 // ---- FP32 form of passes A and C ------------------------------------------
@@ -413,11 +362,13 @@ __device__ __forceinline__ double group_sum(double v, int T, double *red) {
 // x-fluctuation is in rhsf).
 // From the second solve on the offset is the previous solve's row mean and
 // one pass over the row does both; the first solve takes two passes and the
-// exact mean.  The first radix-16 pass runs on the values as loaded.
+// exact mean.  The offset is rounded to FP32 first, so that the value minus
+// the offset rounds once, as one FP32 subtraction.  The first radix-16 pass
+// runs on the values as loaded.
 template <int BLOCK, int K>
 __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan &c, int pair_base, float2 *sm,
                                                double *red) {
-    using S = fft32::Shape<K>;
+    using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
     const int pair = pair_base + p;
@@ -431,27 +382,39 @@ __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan
     const double k0 = live ? rhs_row_constant(pp, c, j0 + 1) : 0.0, k1 = two ? rhs_row_constant(pp, c, j1 + 1) : 0.0;
     const bool exact = *pp.rowmean_ok == 0;  // the same for every block of the launch
     // value - offset = rhsf + (row constant - offset)
-    double d0 = (live && !exact) ? k0 - pp.rowmean[j0] : 0.0, d1 = (two && !exact) ? k1 - pp.rowmean[j1] : 0.0;
+    float d0 = (live && !exact) ? (float)(k0 - pp.rowmean[j0]) : 0.0f, d1 = (two && !exact) ? (float)(k1 - pp.rowmean[j1]) : 0.0f;
     double a0 = 0.0, a1 = 0.0;
     float2 x[16];
+    if constexpr (T == 1) {  // a row a thread: 16 consecutive values
+        const float4 *q0 = reinterpret_cast<const float4 *>(pp.rhsf + r0), *q1 = reinterpret_cast<const float4 *>(pp.rhsf + r1);
+        const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const float4 u = live ? __ldg(q0 + v) : none, w = two ? __ldg(q1 + v) : none;
+            x[4 * v] = make_float2(u.x, w.x);
+            x[4 * v + 1] = make_float2(u.y, w.y);
+            x[4 * v + 2] = make_float2(u.z, w.z);
+            x[4 * v + 3] = make_float2(u.w, w.w);
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < 16; ++v)
+            x[v] = make_float2(live ? __ldg(pp.rhsf + (r0 + (unsigned)(v * T))) : 0.0f,
+                               two ? __ldg(pp.rhsf + (r1 + (unsigned)(v * T))) : 0.0f);
+    }
 #pragma unroll
     for (int v = 0; v < 16; ++v) {
-        const float f0 = live ? __ldg(pp.rhsf + (r0 + (unsigned)(v * T))) : 0.0f,
-                    f1 = two ? __ldg(pp.rhsf + (r1 + (unsigned)(v * T))) : 0.0f;
-        a0 += (double)f0;
-        a1 += (double)f1;
-        x[v] = make_float2((float)((double)f0 + d0), (float)((double)f1 + d1));
+        a0 += (double)x[v].x;
+        a1 += (double)x[v].y;
     }
     a0 = group_sum<BLOCK>(a0, T, red) + (double)N * k0;
     a1 = group_sum<BLOCK>(a1, T, red) + (double)N * k1;
     if (exact) {
-        d0 = k0 - a0 / (double)N;
-        d1 = k1 - a1 / (double)N;
-#pragma unroll
-        for (int v = 0; v < 16; ++v)
-            x[v] = make_float2(live ? (float)((double)__ldg(pp.rhsf + (r0 + (unsigned)(v * T))) + d0) : 0.0f,
-                               two ? (float)((double)__ldg(pp.rhsf + (r1 + (unsigned)(v * T))) + d1) : 0.0f);
+        d0 = live ? (float)(k0 - a0 / (double)N) : 0.0f;
+        d1 = two ? (float)(k1 - a1 / (double)N) : 0.0f;
     }
+#pragma unroll
+    for (int v = 0; v < 16; ++v) x[v] = __fadd2_rn(x[v], make_float2(d0, d1));
     if (t == 0 && live) {
         pp.spec[(size_t)j0 * pp.mp] = make_double2(a0, 0.0);
         pp.rowmean[j0] = a0 / (double)N;
@@ -460,16 +423,36 @@ __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan
             pp.rowmean[j1] = a1 / (double)N;
         }
     }
-    fft32::fwd_pass_store<K, 1>(x, s, t, p, pp.twf);
+    fft16::fwd_pass_store<K, 1>(x, s, t, p, pp.twf);
     __syncthreads();
-    fft32::fwd_rest<K, 2>(s, t, p, pp.twf);
+    fft16::fwd_rest<K, 2>(s, t, p, pp.twf);
     if (!live) return;
     const unsigned q0 = (unsigned)j0 * (unsigned)pp.mp, q1 = q0 + (unsigned)pp.mp;
-    for (int m = t; m <= N / 2; m += T) {
-        if (m == 0) continue;
-        const float2 a = s[fft32::swz_base(brev(m, K), p)], b = cconj(s[fft32::swz_base(brev(N - m, K), p)]);
-        pp.specf[q0 + (unsigned)m] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
-        if (two) pp.specf[q1 + (unsigned)m] = make_float2(0.5f * (a.y - b.y), -0.5f * (a.x - b.x));
+    auto mode = [&](int m, float2 *A, float2 *B) {
+        const float2 a = s[fft16::swz_base(brev(m, K), p)], b = cconj(s[fft16::swz_base(brev(N - m, K), p)]);
+        *A = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
+        *B = make_float2(0.5f * (a.y - b.y), -0.5f * (a.x - b.x));
+    };
+    if constexpr (T == 1) {  // modes 0 (not used: zero) to 8 of a row, in 16-byte stores
+        float2 A[9], B[9];
+        A[0] = B[0] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int m = 1; m <= 8; ++m) mode(m, &A[m], &B[m]);
+#pragma unroll
+        for (int m = 0; m < 8; m += 2) {
+            *reinterpret_cast<float4 *>(pp.specf + (q0 + m)) = make_float4(A[m].x, A[m].y, A[m + 1].x, A[m + 1].y);
+            if (two) *reinterpret_cast<float4 *>(pp.specf + (q1 + m)) = make_float4(B[m].x, B[m].y, B[m + 1].x, B[m + 1].y);
+        }
+        pp.specf[q0 + 8] = A[8];
+        if (two) pp.specf[q1 + 8] = B[8];
+    } else {
+        for (int m = t; m <= N / 2; m += T) {
+            if (m == 0) continue;
+            float2 A, B;
+            mode(m, &A, &B);
+            pp.specf[q0 + (unsigned)m] = A;
+            if (two) pp.specf[q1 + (unsigned)m] = B;
+        }
     }
 }
 
@@ -501,7 +484,7 @@ __device__ __forceinline__ void write_walls_f32(const PoissonPlan &pp, const Cha
 template <int BLOCK, int K>
 __device__ __forceinline__ void inv_rows_f32_k(const PoissonPlan &pp, const Chan &c, double *__restrict__ psi,
                                                bool write_f64, int pair_base, float2 *sm) {
-    using S = fft32::Shape<K>;
+    using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
     const int pair = pair_base + p;
@@ -516,26 +499,41 @@ __device__ __forceinline__ void inv_rows_f32_k(const PoissonPlan &pp, const Chan
     // modes m = t + i T (i < 8) and, for t = 0, m = N/2: all loads first
     const float2 zero = make_float2(0.0f, 0.0f);
     float2 a[9], b[9];
+    if constexpr (T == 1) {  // a row a thread: modes 0 (its slot holds zero) to 8
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        const int m = t + i * T;
-        const bool in = i < 8 || t == 0;
-        a[i] = (live && in && m) ? pp.specf[q0 + (unsigned)m] : zero;
-        b[i] = (two && in && m) ? pp.specf[q1 + (unsigned)m] : zero;
+        for (int i = 0; i < 8; i += 2) {
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 u = live ? *reinterpret_cast<const float4 *>(pp.specf + (q0 + i)) : none;
+            const float4 w = two ? *reinterpret_cast<const float4 *>(pp.specf + (q1 + i)) : none;
+            a[i] = i ? make_float2(u.x, u.y) : zero;
+            a[i + 1] = make_float2(u.z, u.w);
+            b[i] = i ? make_float2(w.x, w.y) : zero;
+            b[i + 1] = make_float2(w.z, w.w);
+        }
+        a[8] = live ? pp.specf[q0 + 8] : zero;
+        b[8] = two ? pp.specf[q1 + 8] : zero;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            const int m = t + i * T;
+            const bool in = i < 8 || t == 0;
+            a[i] = (live && in && m) ? pp.specf[q0 + (unsigned)m] : zero;
+            b[i] = (two && in && m) ? pp.specf[q1 + (unsigned)m] : zero;
+        }
     }
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
         const int m = t + i * T;
         if (i == 8 && t != 0) break;
-        s[fft32::swz_base(brev(m, K), p)] = make_float2(a[i].x - b[i].y, a[i].y + b[i].x);  // A + iB
+        s[fft16::swz_base(brev(m, K), p)] = make_float2(a[i].x - b[i].y, a[i].y + b[i].x);  // A + iB
         if (m != 0 && 2 * m != N)
-            s[fft32::swz_base(brev(N - m, K), p)] = make_float2(a[i].x + b[i].y, -a[i].y + b[i].x);
+            s[fft16::swz_base(brev(N - m, K), p)] = make_float2(a[i].x + b[i].y, -a[i].y + b[i].x);
     }
     __syncthreads();
-    fft32::inv_partial<K>(s, t, p);
-    fft32::inv_full<K, S::NF>(s, t, p, pp.twf);
+    fft16::inv_partial<K>(s, t, p);
+    fft16::inv_full<K, S::NF>(s, t, p, pp.twf);
     float2 x[16];
-    fft32::inv_pass_load<K, 1>(x, s, t, p, pp.twf);
+    fft16::inv_pass_load<K, 1>(x, s, t, p, pp.twf);
     const double inv = 1.0 / (double)N;
     const float invf = 1.0f / (float)N;  // a power of two: exact
     if (pair_base == 0 && threadIdx.x == 0) *pp.rowmean_ok = 1;
@@ -547,12 +545,24 @@ __device__ __forceinline__ void inv_rows_f32_k(const PoissonPlan &pp, const Chan
             if (two) pp.psim[j1 + 1] = mean1;
         }
         const unsigned o0 = (unsigned)(j0 + 1) * (unsigned)nxp + (unsigned)t, o1 = o0 + (unsigned)nxp;
+        if constexpr (T == 1) {
+#pragma unroll
+            for (int v = 0; v < 16; v += 4) {
+                st_field_f4(pp.psif + (o0 + v), make_float4(x[v].x * invf, x[v + 1].x * invf, x[v + 2].x * invf, x[v + 3].x * invf),
+                            pp.keep_l2);
+                if (two)
+                    st_field_f4(pp.psif + (o1 + v),
+                                make_float4(x[v].y * invf, x[v + 1].y * invf, x[v + 2].y * invf, x[v + 3].y * invf), pp.keep_l2);
+            }
+        }
 #pragma unroll
         for (int v = 0; v < 16; ++v) {
             const float y0 = x[v].x * invf, y1 = x[v].y * invf;
             const unsigned dv = (unsigned)(v * T);
-            st_field_f(pp.psif + (o0 + dv), y0, pp.keep_l2);
-            if (two) st_field_f(pp.psif + (o1 + dv), y1, pp.keep_l2);
+            if constexpr (T > 1) {
+                st_field_f(pp.psif + (o0 + dv), y0, pp.keep_l2);
+                if (two) st_field_f(pp.psif + (o1 + dv), y1, pp.keep_l2);
+            }
             if (write_f64) {
                 psi[o0 + dv] = mean0 + (double)y0;
                 if (two) psi[o1 + dv] = mean1 + (double)y1;
@@ -561,59 +571,53 @@ __device__ __forceinline__ void inv_rows_f32_k(const PoissonPlan &pp, const Chan
     }
 }
 
-// Transform sizes a block of BLOCK threads runs: 256 threads take every
-// 16 <= nx <= 4096 (several row pairs a block below 4096), 512 threads one
-// row pair of nx = 8192.
-template <int BLOCK, int K> __host__ __device__ constexpr bool r16f_fits() {
-    return BLOCK == 256 ? (K >= 4 && K <= 12) : ((1 << K) >> 4) == BLOCK;
-}
-
-#define EK_R16F_CASES(F) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13)
-
-template <int BLOCK>
-__device__ __forceinline__ void fwd_rows_r16f_dev(const PoissonPlan &pp, const Chan &c, int pair_base, float2 *sm,
-                                                  double *red) {
-    switch (pp.log2nx) {
-#define EK_CASE(K)                                                                        \
-    case K:                                                                               \
-        if constexpr (r16f_fits<BLOCK, K>()) fwd_rows_f32_k<BLOCK, K>(pp, c, pair_base, sm, red); \
-        break;
-        EK_R16F_CASES(EK_CASE)
-#undef EK_CASE
-        default: break;
-    }
-}
-
-template <int BLOCK>
-__device__ __forceinline__ void inv_rows_r16f_dev(const PoissonPlan &pp, const Chan &c, double *__restrict__ psi,
-                                                  bool write_f64, int pair_base, float2 *sm) {
-    switch (pp.log2nx) {
-#define EK_CASE(K)                                                                                    \
-    case K:                                                                                           \
-        if constexpr (r16f_fits<BLOCK, K>()) inv_rows_f32_k<BLOCK, K>(pp, c, psi, write_f64, pair_base, sm); \
-        break;
-        EK_R16F_CASES(EK_CASE)
-#undef EK_CASE
-        default: break;
-    }
-}
-
-// 4 blocks of 256 threads per SM: the 511 row pairs of a 4096 x 1024 channel
-// then run in one wave (3 blocks per SM leave a second, nearly empty wave).
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
-fwd_rows_r16f(const PoissonPlan pp, const Chan c) {
+// Pass A and C of a single channel, compiled per size; 1024 threads an SM (64
+// registers a thread hold the 16 points of a transform).
+template <int K>
+__global__ void __launch_bounds__(RowCfg<K>::block, 1024 / RowCfg<K>::block)
+fwd_rows_f32(const PoissonPlan pp, const Chan c) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ double red[(RowCfg<K>::block + 31) / 32];
     pdl_wait();
+    fwd_rows_f32_k<RowCfg<K>::block, K>(pp, c, blockIdx.x * RowCfg<K>::per, (float2 *)smraw, red);
+}
+
+template <int K>
+__global__ void __launch_bounds__(RowCfg<K>::block, 1024 / RowCfg<K>::block)
+inv_rows_f32(const PoissonPlan pp, const Chan c, double *__restrict__ psi, bool write_f64) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ double red[BLOCK / 32];
-    fwd_rows_r16f_dev<BLOCK>(pp, c, blockIdx.x * (BLOCK / (pp.nx >> 4)), (float2 *)smraw, red);
+    pdl_wait();
+    inv_rows_f32_k<RowCfg<K>::block, K>(pp, c, psi, write_f64, blockIdx.x * RowCfg<K>::per, (float2 *)smraw);
+}
+
+// Sizes that a batch block of BLOCK threads runs, whole transforms only.
+template <int BLOCK, int K> __host__ __device__ constexpr bool batch_fits() { return ((1 << K) >> 4) <= BLOCK && K <= 12; }
+
+template <int BLOCK>
+__device__ __forceinline__ void fwd_rows_any(const PoissonPlan &pp, const Chan &c, int pair_base, float2 *sm, double *red) {
+    switch (pp.log2nx) {
+#define EK_CASE(K)                                                                                     \
+    case K:                                                                                            \
+        if constexpr (batch_fits<BLOCK, K>()) fwd_rows_f32_k<BLOCK, K>(pp, c, pair_base, sm, red);     \
+        break;
+        EK_ROW_CASES(EK_CASE)
+#undef EK_CASE
+        default: break;
+    }
 }
 
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
-inv_rows_r16f(const PoissonPlan pp, const Chan c, double *__restrict__ psi, bool write_f64) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    inv_rows_r16f_dev<BLOCK>(pp, c, psi, write_f64, blockIdx.x * (BLOCK / (pp.nx >> 4)), (float2 *)smraw);
+__device__ __forceinline__ void inv_rows_any(const PoissonPlan &pp, const Chan &c, double *__restrict__ psi, bool write_f64,
+                                             int pair_base, float2 *sm) {
+    switch (pp.log2nx) {
+#define EK_CASE(K)                                                                                                 \
+    case K:                                                                                                        \
+        if constexpr (batch_fits<BLOCK, K>()) inv_rows_f32_k<BLOCK, K>(pp, c, psi, write_f64, pair_base, sm);      \
+        break;
+        EK_ROW_CASES(EK_CASE)
+#undef EK_CASE
+        default: break;
+    }
 }
 
 // ---- pass B, partitioned Thomas solve ------------------------------------
@@ -676,13 +680,15 @@ __device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *_
     const int m = m_base + mode;
     const bool mvalid = m <= mlast;
     const int L = (n + S - 1) / S, ja = seg * L, cnt = max(0, min(n, ja + L) - ja);
+    const unsigned o = (unsigned)ja * (unsigned)mp + (unsigned)m;  // n mp < 2^32 (n <= 8192)
     R c[TB_L];
     C v[TB_L];
+    pdl_wait();
 #pragma unroll
     for (int q = 0; q < TB_L; ++q) {
         const bool on = mvalid && q < cnt;
-        c[q] = on ? __ldg(piv + (size_t)(ja + q) * mp + m) : R(0);
-        const C sv = on ? spec[(size_t)(ja + q) * mp + m] : cmake<C>(0.0, 0.0);
+        c[q] = on ? __ldg(piv + (o + q * (unsigned)mp)) : R(0);
+        const C sv = on ? spec[o + q * (unsigned)mp] : cmake<C>(0.0, 0.0);
         v[q] = cmake<C>(dy2 * sv.x, dy2 * sv.y);
     }
     C d = cmake<C>(0.0, 0.0);
@@ -724,7 +730,7 @@ __device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *_
     for (int q = TB_L - 1; q >= 0; --q) {
         if (q < cnt) {
             nu = -c[q] * nu;
-            spec[(size_t)(ja + q) * mp + m] = cmake<C>(v[q].x + nu * X.x, v[q].y + nu * X.y);
+            spec[o + q * (unsigned)mp] = cmake<C>(v[q].x + nu * X.x, v[q].y + nu * X.y);
         }
     }
 }
@@ -789,6 +795,7 @@ __device__ __forceinline__ void zero_mode_f64(const PoissonPlan &pp, ColumnShare
     const size_t stride = 2 * (size_t)pp.mp;  // element j of the column at col[j * stride]
     double *col = &pp.spec[0].x;
     const double dy2 = pp.dy2;
+    pdl_wait();
     // segment sum of h, then H at the segment's start
     double s1 = 0.0;
     for (int q = 0; q < cnt; ++q) s1 += dy2 * __ldg(col + (size_t)(ja + q) * stride);
@@ -831,24 +838,44 @@ __global__ void __launch_bounds__(TB_THREADS, 2) tridiag_modes_f32(const Poisson
 // A block's work item names its channel and its first row pair (passes A,
 // C) or first x-mode (pass B); the channel's plan comes from a device table.
 // Batches run the FP32 form.
-__global__ void __launch_bounds__(256, 4)
+// The channel's plan and constants are staged in shared memory (as a copy in
+// registers they spilled 3.9 KB a thread of the forward pass).  BLOCK: 64
+// threads where every channel's transform fits them (nx <= 1024), else 256.
+struct RowItem {
+    PoissonPlan pp;
+    Chan c;
+};
+static_assert(sizeof(PoissonPlan) % 8 == 0 && sizeof(Chan) % 8 == 0, "copied by 8-byte words");
+template <int BLOCK>
+__device__ __forceinline__ void stage_item(RowItem &it, const PoissonPlan *__restrict__ plan, const Chan *__restrict__ chan) {
+    for (int i = threadIdx.x; i < (int)(sizeof(PoissonPlan) / 8); i += BLOCK)
+        ((unsigned long long *)&it.pp)[i] = __ldg((const unsigned long long *)plan + i);
+    for (int i = threadIdx.x; i < (int)(sizeof(Chan) / 8); i += BLOCK)
+        ((unsigned long long *)&it.c)[i] = __ldg((const unsigned long long *)chan + i);
+    __syncthreads();
+}
+
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 batch_fwd_rows_f32(const PoissonPlan *__restrict__ plans, const Chan *__restrict__ chans,
                    const int2 *__restrict__ items) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ double red[256 / 32];
+    __shared__ double red[BLOCK / 32];
+    __shared__ __align__(16) RowItem ri;
     const int2 it = items[blockIdx.x];
-    const PoissonPlan pp = plans[it.x];
-    fwd_rows_r16f_dev<256>(pp, chans[it.x], it.y, (float2 *)smraw, red);
+    stage_item<BLOCK>(ri, plans + it.x, chans + it.x);
+    fwd_rows_any<BLOCK>(ri.pp, ri.c, it.y, (float2 *)smraw, red);
 }
 
-__global__ void __launch_bounds__(256, 4)
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 batch_inv_rows_f32(const PoissonPlan *__restrict__ plans, const Chan *__restrict__ chans,
                    double *const *__restrict__ fields, const int2 *__restrict__ items, bool write_f64) {
     extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ __align__(16) RowItem ri;
     const int2 it = items[blockIdx.x];
-    const PoissonPlan pp = plans[it.x];
-    const Chan &c = chans[it.x];
-    inv_rows_r16f_dev<256>(pp, c, fields[it.x] + F_PSI * c.plane, write_f64, it.y, (float2 *)smraw);
+    stage_item<BLOCK>(ri, plans + it.x, chans + it.x);
+    inv_rows_any<BLOCK>(ri.pp, ri.c, fields[it.x] + F_PSI * ri.c.plane, write_f64, it.y, (float2 *)smraw);
 }
 
 // items {channel, first mode, modes per block}: FP32 mode blocks, and for
@@ -876,21 +903,81 @@ int tridiag_modes(int n) {
 
 bool use_r16(const PoissonPlan &pp) { return pp.pow2 && pp.nx >= 16; }
 
-// Threads per block and row pairs per block of the radix-16 row kernels.
-void r16_shape(int nx, int *threads, int *per) {
-    const int T = nx >> 4;
-    *threads = T >= 256 ? T : 256;
-    *per = *threads / T;
+// nx as radices of the mixed form: fours, a two, threes, fives, other primes.
+Radices radices(int nx) {
+    Radices f{};
+    const int small[4] = {4, 2, 3, 5};
+    for (int r : small)
+        while (nx % r == 0) {
+            f.r[f.n++] = r;
+            nx /= r;
+        }
+    for (int r = 7; nx > 1; r += 2)
+        while (nx % r == 0) {
+            f.r[f.n++] = r;
+            nx /= r;
+        }
+    return f;
+}
+// Threads of a mixed-form block: a butterfly of radix 4 a thread and pass.
+int mixed_threads(int nx) {
+    const int t = (nx / 4 + 31) / 32 * 32;
+    return t < 32 ? 32 : (t > PTPB ? PTPB : t);
 }
 
-size_t r16_smem(int nx, int per) { return (size_t)per * nx * sizeof(double2); }
+// Launches of one size of the row kernels.
+template <int K> struct RowLaunch {
+    static constexpr int block = RowCfg<K>::block;
+    static int grid(const PoissonPlan &pp) { return ((pp.n + 1) / 2 + RowCfg<K>::per - 1) / RowCfg<K>::per; }
+    template <typename C> static constexpr size_t smem() { return (size_t)RowCfg<K>::per * RowCfg<K>::N * sizeof(C); }
+    static cudaError_t fwd64(const PoissonPlan &pp, const double *rhs, int nxp, cudaStream_t s) {
+        return launch_pdl(fwd_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, rhs, nxp);
+    }
+    static cudaError_t inv64(const PoissonPlan &pp, const Chan &c, double *psi, bool pdl, cudaStream_t s) {
+        return launch_maybe_pdl(pdl, inv_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, c, psi);
+    }
+    static cudaError_t fwd32(const PoissonPlan &pp, const Chan &c, cudaStream_t s) {
+        return launch_pdl(fwd_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c);
+    }
+    static cudaError_t inv32(const PoissonPlan &pp, const Chan &c, double *psi, bool write_f64, bool pdl, cudaStream_t s) {
+        return launch_maybe_pdl(pdl, inv_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c, psi, write_f64);
+    }
+    static cudaError_t limits(bool f32) {
+        const void *fns[] = {(const void *)fwd_rows_f64<K>, (const void *)inv_rows_f64<K>, (const void *)fwd_rows_f32<K>,
+                             (const void *)inv_rows_f32<K>};
+        for (int i = 0; i < (f32 ? 4 : 2); ++i) {
+            const size_t bytes = i < 2 ? smem<double2>() : smem<float2>();
+            cudaError_t e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(fns[i], cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+};
+#define EK_ROW_DISPATCH(lg, call)                       \
+    switch (lg) {                                       \
+        case 4: return RowLaunch<4>::call;              \
+        case 5: return RowLaunch<5>::call;              \
+        case 6: return RowLaunch<6>::call;              \
+        case 7: return RowLaunch<7>::call;              \
+        case 8: return RowLaunch<8>::call;              \
+        case 9: return RowLaunch<9>::call;              \
+        case 10: return RowLaunch<10>::call;            \
+        case 11: return RowLaunch<11>::call;            \
+        case 12: return RowLaunch<12>::call;            \
+        case 13: return RowLaunch<13>::call;            \
+        default: return cudaErrorInvalidValue;          \
+    }
+
+// Programmatic launch of passes B and C: where the passes are one wave of
+// blocks it hides their launch latency; on channels of many nodes it made the
+// step longer (4096 x 1024: 4.5 us a step), the waiting blocks taking the place
+// of running ones.
+bool small_channel(const PoissonPlan &pp) { return (size_t)pp.nx * pp.ny <= PDL_NODES; }
 
 }  // namespace
 
-size_t poisson_smem_bytes_f64(int nx) {
-    const bool pow2 = nx > 0 && (nx & (nx - 1)) == 0;
-    return (size_t)nx * sizeof(double2) * (pow2 ? 1 : 2);
-}
+size_t poisson_smem_bytes_f64(int nx) { return 2 * (size_t)nx * sizeof(double2); }
 
 cudaError_t poisson_pass_f64(int pass, const PoissonPlan &pp, const Chan &c, double *fields, cudaStream_t s) {
     return poisson_pass_f64_at(pass, pp, c, fields + F_RHS * c.plane, fields + F_PSI * c.plane, s);
@@ -898,31 +985,21 @@ cudaError_t poisson_pass_f64(int pass, const PoissonPlan &pp, const Chan &c, dou
 
 cudaError_t poisson_pass_f64_at(int pass, const PoissonPlan &pp, const Chan &c, const double *rhs, double *psi,
                                 cudaStream_t s) {
-    const int rows2 = (pp.n + 1) / 2;
+    const bool pdl = small_channel(pp);
     if (pass == 1) {
         const int M = tridiag_modes(pp.n);
-        if (M > 0) tridiag_part<<<(pp.nx / 2 + M) / M, TB_THREADS, 0, s>>>(pp, M);
-        else tridiag<<<(pp.nx / 2 + 1 + PTPB - 1) / PTPB, PTPB, 0, s>>>(pp);
-        return cudaGetLastError();
+        if (M > 0) return launch_maybe_pdl(pdl, tridiag_part, dim3((pp.nx / 2 + M) / M), dim3(TB_THREADS), 0, s, pp, M);
+        return launch_maybe_pdl(pdl, tridiag, dim3((pp.nx / 2 + 1 + PTPB - 1) / PTPB), dim3(PTPB), 0, s, pp);
     }
     if (use_r16(pp)) {
-        int threads, per;
-        r16_shape(pp.nx, &threads, &per);
-        const size_t smem = r16_smem(pp.nx, per);
-        const int blocks = (rows2 + per - 1) / per;
-        if (threads == 256) {
-            if (pass == 0) fwd_rows_r16<256><<<blocks, 256, smem, s>>>(pp, rhs, c.nxp);
-            else inv_rows_r16<256><<<blocks, 256, smem, s>>>(pp, c, psi);
-        } else {
-            if (pass == 0) fwd_rows_r16<512><<<blocks, 512, smem, s>>>(pp, rhs, c.nxp);
-            else inv_rows_r16<512><<<blocks, 512, smem, s>>>(pp, c, psi);
-        }
-        return cudaGetLastError();
+        if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd64(pp, rhs, c.nxp, s))
+        EK_ROW_DISPATCH(pp.log2nx, inv64(pp, c, psi, pdl, s))
     }
+    const Radices f = radices(pp.nx);
+    const dim3 grid((pp.n + 1) / 2), block(mixed_threads(pp.nx));
     const size_t smem = poisson_smem_bytes_f64(pp.nx);
-    if (pass == 0) fwd_rows<<<rows2, PTPB, smem, s>>>(pp, rhs, c.nxp);
-    else inv_rows<<<rows2, PTPB, smem, s>>>(pp, c, psi);
-    return cudaGetLastError();
+    if (pass == 0) return launch_pdl(fwd_rows, grid, block, smem, s, pp, f, rhs, c.nxp);
+    return launch_maybe_pdl(pdl, inv_rows, grid, block, smem, s, pp, f, c, psi);
 }
 
 int poisson_tridiag_modes(int n) { return tridiag_modes(n); }
@@ -934,36 +1011,33 @@ bool poisson_f32_supported(const PoissonPlan &pp) {
 cudaError_t poisson_tridiag_f32(const PoissonPlan &pp, cudaStream_t s) {
     if (!poisson_f32_supported(pp)) return cudaErrorInvalidValue;
     const int M = tridiag_modes(pp.n);
-    tridiag_modes_f32<<<1 + (pp.nx / 2 + M - 1) / M, TB_THREADS, 0, s>>>(pp, M);
-    return cudaGetLastError();
+    return launch_maybe_pdl(small_channel(pp), tridiag_modes_f32, dim3(1 + (pp.nx / 2 + M - 1) / M), dim3(TB_THREADS), 0, s, pp,
+                            M);
 }
 
 cudaError_t poisson_pass_f32(int pass, const PoissonPlan &pp, const Chan &c, double *psi, bool write_f64,
                              cudaStream_t s) {
     // pass B of this form runs through poisson_tridiag_f32
     if (!poisson_f32_supported(pp) || pass == 1) return cudaErrorInvalidValue;
-    int threads, per;
-    r16_shape(pp.nx, &threads, &per);
-    const size_t smem = (size_t)per * pp.nx * sizeof(float2);
-    const int blocks = ((pp.n + 1) / 2 + per - 1) / per;
-    if (threads == 256) {
-        if (pass == 0) return launch_pdl(fwd_rows_r16f<256>, dim3(blocks), dim3(256), smem, s, pp, c);
-        inv_rows_r16f<256><<<blocks, 256, smem, s>>>(pp, c, psi, write_f64);
-    } else {
-        if (pass == 0) return launch_pdl(fwd_rows_r16f<512>, dim3(blocks), dim3(512), smem, s, pp, c);
-        inv_rows_r16f<512><<<blocks, 512, smem, s>>>(pp, c, psi, write_f64);
-    }
-    return cudaGetLastError();
+    if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd32(pp, c, s))
+    EK_ROW_DISPATCH(pp.log2nx, inv32(pp, c, psi, write_f64, small_channel(pp), s))
 }
 
+int batch_row_block(int nx_max) { return nx_max <= 1024 ? 64 : 256; }
+
 cudaError_t batch_poisson(int pass, const PoissonPlan *plans, const Chan *chans, double *const *fields,
-                          const void *items, int nitems, bool write_f64, cudaStream_t s) {
+                          const void *items, int nitems, int block, bool write_f64, cudaStream_t s) {
     if (nitems <= 0) return cudaSuccess;
     if (pass == 1) return cudaErrorInvalidValue;  // runs through batch_tridiag_f32
-    if (pass == 0)
-        batch_fwd_rows_f32<<<nitems, 256, 32768, s>>>(plans, chans, (const int2 *)items);
-    else
-        batch_inv_rows_f32<<<nitems, 256, 32768, s>>>(plans, chans, fields, (const int2 *)items, write_f64);
+    const size_t smem = (size_t)block * 16 * sizeof(float2);
+    const int2 *it = (const int2 *)items;
+    if (block == 64) {
+        if (pass == 0) batch_fwd_rows_f32<64><<<nitems, 64, smem, s>>>(plans, chans, it);
+        else batch_inv_rows_f32<64><<<nitems, 64, smem, s>>>(plans, chans, fields, it, write_f64);
+    } else {
+        if (pass == 0) batch_fwd_rows_f32<256><<<nitems, 256, smem, s>>>(plans, chans, it);
+        else batch_inv_rows_f32<256><<<nitems, 256, smem, s>>>(plans, chans, fields, it, write_f64);
+    }
     return cudaGetLastError();
 }
 
@@ -972,20 +1046,31 @@ cudaError_t batch_tridiag_f32(const PoissonPlan *plans, const void *items, int n
     return cudaGetLastError();
 }
 
-cudaError_t poisson_set_smem_limits() {
-    const void *fns[] = {(const void *)fwd_rows, (const void *)inv_rows, (const void *)fwd_rows_r16<256>,
-                         (const void *)inv_rows_r16<256>, (const void *)fwd_rows_r16<512>,
-                         (const void *)inv_rows_r16<512>, (const void *)fwd_rows_r16f<256>,
-                         (const void *)inv_rows_r16f<256>, (const void *)fwd_rows_r16f<512>,
-                         (const void *)inv_rows_r16f<512>, (const void *)batch_fwd_rows_f32,
-                         (const void *)batch_inv_rows_f32};
-    for (const void *f : fns) {
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e != cudaSuccess) return e;
+namespace {
+template <typename F>
+cudaError_t row_limits(F *f, size_t smem) {
+    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return e;
+}
+}  // namespace
+
+// Only the kernels of this length: an attribute call loads its kernel.
+cudaError_t poisson_set_smem_limits(const PoissonPlan &pp) {
+    if (use_r16(pp)) EK_ROW_DISPATCH(pp.log2nx, limits(pp.specf != nullptr))
+    const cudaError_t e = row_limits(fwd_rows, poisson_smem_bytes_f64(pp.nx));
+    return e == cudaSuccess ? row_limits(inv_rows, poisson_smem_bytes_f64(pp.nx)) : e;
+}
+
+cudaError_t batch_set_smem_limits(int block) {
+    const size_t smem = (size_t)block * 16 * sizeof(float2);
+    cudaError_t e;
+    if (block == 64) {
+        e = row_limits(batch_fwd_rows_f32<64>, smem);
+        return e == cudaSuccess ? row_limits(batch_inv_rows_f32<64>, smem) : e;
     }
-    return cudaSuccess;
+    e = row_limits(batch_fwd_rows_f32<256>, smem);
+    return e == cudaSuccess ? row_limits(batch_inv_rows_f32<256>, smem) : e;
 }
 
 }  // namespace ek
