@@ -155,6 +155,8 @@ void refresh_chan(ek_ctx *c) {
     h.ext_x = p.ext_x;
     h.exf = p.exf;
     h.r = c->rates;
+    const double ci = 1.0 / p.cfl;
+    h.inv = {1.0 / p.cs2, ci, 1.0 / p.dx, 1.0 / p.dy, 1.0 / p.eps, W0 / p.cs2, WS / p.cs2, WD / p.cs2, ci * ci / p.cs2};
     h.zlo = c->wall;
     h.zhi = c->wall + p.nx;
     h.cplo = c->wall + 2 * p.nx;

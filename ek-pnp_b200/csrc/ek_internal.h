@@ -153,6 +153,13 @@ struct Rates {
     double ms, md;    // moving top wall terms
 };
 
+// Reciprocals of a channel's constants and the weights over cs2 (LBM.cu:556-572),
+// rounded once: the FP64 step divides by the constants through them.
+struct Recips {
+    double cs2, cfl, dx, dy, eps;
+    double w0_cs2, ws_cs2, wd_cs2, ci2_cs2;  // W / cs2, (1/cfl)^2 / cs2
+};
+
 // Per-channel constants, passed by value to every kernel.
 struct Chan {
     int nx, ny, nxp, flags;
@@ -160,6 +167,7 @@ struct Chan {
     double dx, dy, dt, cfl, cs2, rho0, c0;
     double mob_p, mob_n, f_charge, eps, ext_x, exf;
     Rates r;
+    Recips inv;
     const double *zlo, *zhi, *cplo, *cphi, *cnlo, *cnhi;  // per-x wall values (nx each)
     // Shifted storage only: per-row reference densities divided by 36, three
     // rows of ny floats (fluid, c+, c-).  A population of species s stored at

@@ -32,6 +32,21 @@ namespace ek {
 namespace {
 
 constexpr int TPB = 128;
+// Blocks an SM of the step: 4 (127 registers).  A pass of 10 steps of 4096 x 1024
+// on B200: 4.42 ms; 3 blocks (145 registers) 4.49, 5 (96, spilling) 4.45, 6 4.65.
+constexpr int STEP_BLOCKS = 4;
+
+// a / b for a constant b with its correctly rounded reciprocal ib: one
+// correction of the product by the exact remainder (Markstein 1990), which
+// rounds as the division does -- in three multiply-adds instead of a division's
+// twenty-odd instructions.  A node divides by the constants some thirty times,
+// and the chain of them was most of a small channel's launch: without
+// them 10 x 101 takes 15.3 us a step, not 17.6, and 4096 x 1024 442 us, not 489
+// (B200).  A non-finite a gives a NaN.
+__device__ __forceinline__ double div_by(double a, double b, double ib) {
+    const double q = __dmul_rn(a, ib);
+    return __fma_rn(__fma_rn(-b, q, a), ib, q);
+}
 
 __device__ __forceinline__ double sum9(const double t[9]) {
     return t[0] + t[1] + t[2] + t[3] + t[4] + t[5] + t[6] + t[7] + t[8];
@@ -98,16 +113,16 @@ __device__ __forceinline__ void equilibria(double dens, double tux, double tuy, 
 }
 
 // Guo forcing populations (LBM.cu:556-572); e_i = c_i/CFL.
-__device__ __forceinline__ void guo_pops(double ux, double uy, double fx, double fy, double cs2,
-                                         double cfl, double s[9]) {
-    const double coe0 = W0 / cs2, coes = WS / cs2, coed = WD / cs2;
-    const double ci = 1.0 / cfl;
+__device__ __forceinline__ void guo_pops(double ux, double uy, double fx, double fy, const Chan &c, double s[9]) {
+    const double coe0 = c.inv.w0_cs2, coes = c.inv.ws_cs2, coed = c.inv.wd_cs2;
+    const double ci = c.inv.cfl;
+    const double qx = div_by((ci * ux) * ci, c.cs2, c.inv.cs2), qy = div_by((ci * uy) * ci, c.cs2, c.inv.cs2);
     s[0] = coe0 * (-ux * fx - uy * fy);
-    s[1] = coes * (((ci - ux) + (ci * ux) * ci / cs2) * fx - uy * fy);
-    s[2] = coes * (-ux * fx + ((ci - uy) + (ci * uy) * ci / cs2) * fy);
-    s[3] = coes * (((-ci - ux) + (ci * ux) * ci / cs2) * fx - uy * fy);
-    s[4] = coes * (-ux * fx + ((-ci - uy) + (ci * uy) * ci / cs2) * fy);
-    const double ci2 = ci * ci / cs2;
+    s[1] = coes * (((ci - ux) + qx) * fx - uy * fy);
+    s[2] = coes * (-ux * fx + ((ci - uy) + qy) * fy);
+    s[3] = coes * (((-ci - ux) + qx) * fx - uy * fy);
+    s[4] = coes * (-ux * fx + ((-ci - uy) + qy) * fy);
+    const double ci2 = c.inv.ci2_cs2;
     s[5] = coed * (((ci - ux) + (ux + uy) * ci2) * fx + ((ci - uy) + (ux + uy) * ci2) * fy);
     s[6] = coed * (((-ci - ux) + (ux - uy) * ci2) * fx + ((ci - uy) + (-ux + uy) * ci2) * fy);
     s[7] = coed * (((-ci - ux) + (ux + uy) * ci2) * fx + ((-ci - uy) + (ux + uy) * ci2) * fy);
@@ -132,14 +147,20 @@ __device__ __forceinline__ void relax(const double t[9], const double e[9], doub
     trt_pair(t[6], t[8], e[6], e[8], wp, wm, &o[6], &o[8]);
 }
 
+// v / cs2 / cfl
+__device__ __forceinline__ double by_cs2_cfl(double v, const Chan &c) {
+    return div_by(div_by(v, c.cs2, c.inv.cs2), c.cfl, c.inv.cfl);
+}
+
 // Field E at a node from psi: central differences with periodic x, and the
 // wall rows take the adjacent row's Ey (gpu_efield + gpu_bc, poisson.cu:145-174).
 __device__ __forceinline__ void efield_at(const double *__restrict__ psi, const Chan &c, int x,
                                           int y, int xm, int xp, double *ex, double *ey) {
     const size_t r = (size_t)y * c.nxp;
-    *ex = 0.5 * (__ldg(psi + r + xm) - __ldg(psi + r + xp)) / c.dx;
+    *ex = div_by(0.5 * (__ldg(psi + r + xm) - __ldg(psi + r + xp)), c.dx, c.inv.dx);
     const int yc = y == 0 ? 1 : (y == c.ny - 1 ? c.ny - 2 : y);
-    *ey = 0.5 * (__ldg(psi + (size_t)(yc - 1) * c.nxp + x) - __ldg(psi + (size_t)(yc + 1) * c.nxp + x)) / c.dy;
+    *ey = div_by(0.5 * (__ldg(psi + (size_t)(yc - 1) * c.nxp + x) - __ldg(psi + (size_t)(yc + 1) * c.nxp + x)), c.dy,
+                 c.inv.dy);
 }
 
 // The raw populations of node (x, y) as stored: FIRST -> its own values;
@@ -216,8 +237,8 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
         forcex = c.f_charge * (charge - temp) * (Ex + c.ext_x) + c.exf;
         forcey = c.f_charge * (charge - temp) * Ey;
     }
-    double ux = rhoinv * ((ft[1] + ft[5] + ft[8] - (ft[3] + ft[6] + ft[7])) / c.cfl + forcex * c.dt * 0.5);
-    double uy = rhoinv * ((ft[2] + ft[5] + ft[6] - (ft[4] + ft[7] + ft[8])) / c.cfl + forcey * c.dt * 0.5);
+    double ux = rhoinv * (div_by(ft[1] + ft[5] + ft[8] - (ft[3] + ft[6] + ft[7]), c.cfl, c.inv.cfl) + forcex * c.dt * 0.5);
+    double uy = rhoinv * (div_by(ft[2] + ft[5] + ft[6] - (ft[4] + ft[7] + ft[8]), c.cfl, c.inv.cfl) + forcey * c.dt * 0.5);
     if (lo) {
         // lower wall: minus the velocity of row 1 (LBM.cu:402-443)
         double fm[9];
@@ -225,8 +246,8 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
         if (FIRST) own9(sf, pl, o1, fm);
         else pull9(sf, pl, nxp, x, 1, xm, xp, 0, 2, fm);
         const double rhoinvm = 1.0 / sum9(fm);
-        ux = -rhoinvm * ((fm[1] + fm[5] + fm[8] - (fm[3] + fm[6] + fm[7])) / c.cfl + forcex * c.dt * 0.5);
-        uy = -rhoinvm * ((fm[2] + fm[5] + fm[6] - (fm[4] + fm[7] + fm[8])) / c.cfl + forcey * c.dt * 0.5);
+        ux = -rhoinvm * (div_by(fm[1] + fm[5] + fm[8] - (fm[3] + fm[6] + fm[7]), c.cfl, c.inv.cfl) + forcex * c.dt * 0.5);
+        uy = -rhoinvm * (div_by(fm[2] + fm[5] + fm[6] - (fm[4] + fm[7] + fm[8]), c.cfl, c.inv.cfl) + forcey * c.dt * 0.5);
     }
     if (moments) {
         fields[F_RHO * pl + o] = rho;
@@ -237,25 +258,27 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
     }
     if (!lo && !hi) {
         // Poisson right-hand side with the Dirichlet lifting (poisson.cu:228-241)
-        double v = -c.f_charge * (charge - temp) / c.eps;
+        double v = div_by(-c.f_charge * (charge - temp), c.eps, c.inv.eps);
         if (y == 1) v = v - c.zlo[x] / c.dy / c.dy;
         if (y == c.ny - 2) v = v - c.zhi[x] / c.dy / c.dy;
         fields[F_RHS * pl + o] = v;
     }
 
     // ion equilibria in the drift velocities u + K E (LBM.cu:479-552)
-    const double omusq = 1.0 - 0.5 * (ux * ux + uy * uy) / c.cs2;
-    const double omusq_c = 1.0 - 0.5 * ((ux + c.mob_p * Ex) * (ux + c.mob_p * Ex) + (uy + c.mob_p * Ey) * (uy + c.mob_p * Ey)) / c.cs2;
-    const double omusq_cn = 1.0 - 0.5 * ((ux + c.mob_n * Ex) * (ux + c.mob_n * Ex) + (uy + c.mob_n * Ey) * (uy + c.mob_n * Ey)) / c.cs2;
+    const double omusq = 1.0 - div_by(0.5 * (ux * ux + uy * uy), c.cs2, c.inv.cs2);
+    const double omusq_c = 1.0 - div_by(0.5 * ((ux + c.mob_p * Ex) * (ux + c.mob_p * Ex) + (uy + c.mob_p * Ey) * (uy + c.mob_p * Ey)),
+                                         c.cs2, c.inv.cs2);
+    const double omusq_cn = 1.0 - div_by(0.5 * ((ux + c.mob_n * Ex) * (ux + c.mob_n * Ex) + (uy + c.mob_n * Ey) * (uy + c.mob_n * Ey)),
+                                         c.cs2, c.inv.cs2);
     {
         double e[9], out[9];
-        equilibria(charge, (ux + c.mob_p * Ex) / c.cs2 / c.cfl, (uy + c.mob_p * Ey) / c.cs2 / c.cfl,
+        equilibria(charge, by_cs2_cfl(ux + c.mob_p * Ex, c), by_cs2_cfl(uy + c.mob_p * Ey, c),
                    omusq_c, omusq_c, e);
         relax(ht, e, c.r.wcp, c.r.wcm, out);
         double *dh = dst + 9 * pl;
 #pragma unroll
         for (int d = 0; d < 9; ++d) dh[d * pl + o] = out[d];
-        equilibria(temp, (ux + c.mob_n * Ex) / c.cs2 / c.cfl, (uy + c.mob_n * Ey) / c.cs2 / c.cfl,
+        equilibria(temp, by_cs2_cfl(ux + c.mob_n * Ex, c), by_cs2_cfl(uy + c.mob_n * Ey, c),
                    omusq_cn, (c.flags & EK_FLAG_REST_QUIRK) ? omusq : omusq_cn, e);
         relax(tt, e, c.r.wtp, c.r.wtm, out);
         double *dt_ = dst + 18 * pl;
@@ -285,8 +308,8 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
     }
     // fluid: equilibrium, Guo source, TRT (LBM.cu:468-803)
     double e[9], fpop[9];
-    equilibria(rho, ux / c.cs2 / c.cfl, uy / c.cs2 / c.cfl, omusq, omusq, e);
-    guo_pops(ux, uy, forcex, forcey, c.cs2, c.cfl, fpop);
+    equilibria(rho, by_cs2_cfl(ux, c), by_cs2_cfl(uy, c), omusq, omusq, e);
+    guo_pops(ux, uy, forcex, forcey, c, fpop);
     const double sp = c.r.sp, sm = c.r.sm, dt = c.dt;
     double src9[9];
     src9[0] = sp * fpop[0];
@@ -307,7 +330,7 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
 }
 
 template <bool FIRST, bool EXPLICIT_E, typename I>
-__global__ void __launch_bounds__(TPB)
+__global__ void __launch_bounds__(TPB, STEP_BLOCKS)
 step_f64(const Chan c, const double *__restrict__ src, double *__restrict__ dst,
          double *__restrict__ fields, bool moments, bool wait) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
