@@ -546,7 +546,7 @@ int ek_create(const ek_params *p, ek_ctx **out) {
     while ((1 << lg) < p->nx) ++lg;
     c->pp.log2nx = c->pp.pow2 ? lg : 0;
     c->pp.dy2 = p->dy * p->dy;
-    if (p->storage != EK_STORE_F64 && c->pp.pow2 && p->nx >= 16 && poisson_tridiag_modes(c->n) > 0) {
+    if (p->storage != EK_STORE_F64 && c->pp.pow2 && p->nx >= 16 && poisson_tridiag_modes(c->n, p->nx) > 0) {
         // FP32 form of the Poisson solve: FP32 pivots and spectrum; the row
         // transforms' twiddles per radix-16 pass on bits [b, b+4), b = lg-4,
         // lg-8, ... >= 1: exp(-2 pi i kb f / 2^(b+4)) at (f-1) 2^b + kb

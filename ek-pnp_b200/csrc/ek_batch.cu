@@ -16,8 +16,8 @@
 // Steps run in cycles of an even number R of steps.  The last step of a cycle
 // writes the moments and, with re-basing on, the cycle ends with the re-basing
 // of every channel's shifted populations to its new row means (three more
-// launches, done in place so that device pointers never change).  A whole
-// cycle is captured once in a CUDA graph and replayed.  The block shape of the
+// launches, done in place so that device pointers never change).  Cycles are
+// captured in two CUDA graphs (ten steps; the end of a cycle) and replayed.  The block shape of the
 // LBM kernel (threads, tile width, blocks per SM) is picked by timing the
 // candidates (ek_batch_autotune).
 //
@@ -238,8 +238,10 @@ struct ek_batch {
     bool rebase = true;
     bool use_graph = true;
     bool poisson_f32 = false;        // every channel runs the FP32 Poisson form
-    cudaGraphExec_t graph = nullptr;
-    int graph_cur = -1;              // parity the graph was captured for
+    // a cycle is graph_bodies replays of graph_body (GRAPH_STEPS steps) and one of graph (the rest of it)
+    cudaGraphExec_t graph = nullptr, graph_body = nullptr;
+    int graph_bodies = 0;
+    int graph_cur = -1;              // parity the graphs were captured for
     int64_t launches = 0;
     // device tables
     ChanF *d_chanf = nullptr;
@@ -296,7 +298,8 @@ int launches_per_step(const ek_batch *) { return 4; }
 
 void release_graph(ek_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
+    if (b->graph_body) cudaGraphExecDestroy(b->graph_body);
+    b->graph = b->graph_body = nullptr;
     b->graph_cur = -1;
 }
 
@@ -377,7 +380,7 @@ int build_tables(ek_batch *b) {
         if (b->active[i]) {
             const int per = b->row_block / (nx >> 4);
             for (int q = 0; q < (n + 1) / 2; q += per) pairs.push_back(make_int2((int)i, q));
-            const int M = poisson_tridiag_modes(n);
+            const int M = poisson_tridiag_modes(n, nx);
             // the zero mode in FP64 (an item with 0 modes per block); modes 1.. in FP32
             zeros.push_back(make_int3((int)i, 0, 0));
             for (int m0 = 1; m0 <= nx / 2; m0 += M) modes.push_back(make_int3((int)i, m0, M));
@@ -454,17 +457,16 @@ int launch_rebase(ek_batch *b) {
     return EK_OK;
 }
 
-// Graph of one full cycle starting at parity b->cur: R steps, moments on the
-// last, then the re-basing.
-int capture_graph(ek_batch *b) {
-    release_graph(b);
+// Graph of `steps` steps from parity b->cur, `end` closing a cycle: moments on
+// the last step, then the re-basing.
+int capture_steps(ek_batch *b, int steps, bool end, cudaGraphExec_t *out) {
     const int saved_cur = b->cur;
     const int64_t saved_launches = b->launches;
     cudaGraph_t g = nullptr;
     EK_BCUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
     int rc = EK_OK;
-    for (int i = 0; i < b->cycle && rc == EK_OK; ++i) rc = launch_step(b, false, false, i == b->cycle - 1);
-    if (rc == EK_OK && b->rebase) rc = launch_rebase(b);
+    for (int i = 0; i < steps && rc == EK_OK; ++i) rc = launch_step(b, false, false, end && i == steps - 1);
+    if (rc == EK_OK && end && b->rebase) rc = launch_rebase(b);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     b->cur = saved_cur;
     b->launches = saved_launches;
@@ -473,9 +475,27 @@ int capture_graph(ek_batch *b) {
         return rc;
     }
     EK_BCUDA(e, "graph capture");
-    e = cudaGraphInstantiate(&b->graph, g, 0);
+    e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     EK_BCUDA(e, "graph instantiate");
+    return EK_OK;
+}
+
+// Graphs of one full cycle of R steps starting at parity b->cur: a body of
+// GRAPH_STEPS steps (even, so that it can follow itself) and the end of the
+// cycle.  One graph of the whole cycle held 4 R + 3 kernels, and a run to
+// steady state captures and instantiates again whenever channels freeze.
+constexpr int GRAPH_STEPS = 10;
+int capture_graph(ek_batch *b) {
+    release_graph(b);
+    b->graph_bodies = (b->cycle - 2) / GRAPH_STEPS;
+    int rc = EK_OK;
+    if (b->graph_bodies > 0) rc = capture_steps(b, GRAPH_STEPS, false, &b->graph_body);
+    if (rc == EK_OK) rc = capture_steps(b, b->cycle - b->graph_bodies * GRAPH_STEPS, true, &b->graph);
+    if (rc != EK_OK) {
+        release_graph(b);
+        return rc;
+    }
     b->graph_cur = b->cur;
     return EK_OK;
 }
@@ -526,7 +546,7 @@ int ek_batch_create(const ek_params *params, int32_t count, ek_batch **out) {
         if (!pow2(p.nx) || p.nx < 16 || p.nx > 4096)
             return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batched channels need nx a power of two in [16, 4096]");
         if (p.flags & EK_FLAG_EXPLICIT_E) return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batches derive E from psi");
-        if (p.ny < 3 || poisson_tridiag_modes(p.ny - 2) == 0)
+        if (p.ny < 3 || poisson_tridiag_modes(p.ny - 2, p.nx) == 0)
             return ek::ctx_fail(EK_ERR_UNSUPPORTED, "batched channels need 3 <= ny <= 8194");
     }
     ek_batch *b = new ek_batch();
@@ -643,6 +663,8 @@ int ek_batch_step(ek_batch *b, int32_t nsteps) {
                 rc = capture_graph(b);
                 if (rc != EK_OK) return rc;
             }
+            for (int i = 0; i < b->graph_bodies; ++i)
+                EK_BCUDA(cudaGraphLaunch(b->graph_body, b->stream), "graph launch");
             EK_BCUDA(cudaGraphLaunch(b->graph, b->stream), "graph launch");
             b->launches += launches_per_cycle(b);
             done += b->cycle;

@@ -99,26 +99,46 @@ __device__ __forceinline__ void st_field_f2(float *p, float2 v, bool keep) {
 }
 
 template <typename... Exp, typename... Act>
-cudaError_t launch_pdl(void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
+cudaError_t launch_attrs(const cudaLaunchAttribute *at, int nat, void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t s, Act &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.attrs = const_cast<cudaLaunchAttribute *>(at);
+    cfg.numAttrs = nat;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Act>(args)...);
 }
 
-// launch_pdl, or an ordinary launch where pdl is false.
 template <typename... Exp, typename... Act>
-cudaError_t launch_maybe_pdl(bool pdl, void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
-    if (pdl) return launch_pdl(kern, grid, block, smem, s, std::forward<Act>(args)...);
-    kern<<<grid, block, smem, s>>>(std::forward<Act>(args)...);
-    return cudaGetLastError();
+cudaError_t launch_pdl(void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    return launch_attrs(at, 1, kern, grid, block, smem, s, std::forward<Act>(args)...);
+}
+
+// A kernel of a small channel's step (PDL_NODES): launch_pdl where chain is
+// set, an ordinary launch otherwise.  Chained kernels overlap on the SMs and so share one split
+// of L1 and shared memory: all ask for the same small share of shared memory,
+// since the LBM step lives on L1 (its pulls read every line twice or more).
+// A kernel scheduled while another holds the largest share gets the L1 that is
+// left: on B200 that cost a batch of 64 channels 27 % of its step.
+// 1000 x 257 FP64 on B200: 46 us a step at 7 to 25 %, 53 at 100 %.
+constexpr unsigned CHAIN_SMEM_PERCENT = 25;
+template <typename... Exp, typename... Act>
+cudaError_t launch_chain(bool chain, void (*kern)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
+    if (!chain) {
+        kern<<<grid, block, smem, s>>>(std::forward<Act>(args)...);
+        return cudaGetLastError();
+    }
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[1].val.sharedMemCarveout = CHAIN_SMEM_PERCENT;
+    return launch_attrs(at, 2, kern, grid, block, smem, s, std::forward<Act>(args)...);
 }
 // Channels of at most this many nodes: every kernel of a step is about one
 // wave of blocks, and the step a chain of launch latencies.
@@ -317,7 +337,7 @@ cudaError_t batch_tridiag_f32(const PoissonPlan *plans, const void *items, int n
 cudaError_t batch_poisson(int pass, const PoissonPlan *plans, const Chan *chans, double *const *fields,
                           const void *items, int nitems, int block, bool write_f64, cudaStream_t s);
 int batch_row_block(int nx_max);
-int poisson_tridiag_modes(int n);
+int poisson_tridiag_modes(int n, int nx);
 // Steady-state residual sums (ek_residual.cu): per channel 8 FP64 sums,
 // (q - q_snap)^2 then q^2 for q in (ux, c+, c-, psi); the snapshot is updated.
 cudaError_t launch_residual_f64(const Chan &c, const double *fields, double *snap, double *part,

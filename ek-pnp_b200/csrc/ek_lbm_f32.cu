@@ -118,11 +118,11 @@ cudaError_t step_typed(const ChanF &k, const void *src, void *dst, double *field
     S *b = (S *)dst;
     const bool wait = chain != CHAIN_NONE, pdl = chain == CHAIN_NEXT;
     if (first) {
-        if (ee) return launch_maybe_pdl(pdl, step_shifted<S, true, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
-        return launch_maybe_pdl(pdl, step_shifted<S, true, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+        if (ee) return launch_chain(pdl, step_shifted<S, true, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+        return launch_chain(pdl, step_shifted<S, true, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
     }
-    if (ee) return launch_maybe_pdl(pdl, step_shifted<S, false, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
-    return launch_maybe_pdl(pdl, step_shifted<S, false, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+    if (ee) return launch_chain(pdl, step_shifted<S, false, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+    return launch_chain(pdl, step_shifted<S, false, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
 }
 
 __global__ void __launch_bounds__(256) row_refs(const Chan c, const double *__restrict__ fields, int qf, int qp,

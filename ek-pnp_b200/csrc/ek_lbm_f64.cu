@@ -448,8 +448,8 @@ cudaError_t launch_step_f64(const Chan &c, const double *src, double *dst, doubl
     // 32-bit offsets while the 27 population planes fit 2^32 elements
     const bool i32 = (size_t)27 * c.plane < ((size_t)1 << 32);
 #define EK_STEP(F, E)                                                                                               \
-    return i32 ? launch_maybe_pdl(pdl, step_f64<F, E, uint32_t>, g, t, 0, s, c, src, dst, fields, moments, wait)    \
-               : launch_maybe_pdl(pdl, step_f64<F, E, size_t>, g, t, 0, s, c, src, dst, fields, moments, wait)
+    return i32 ? launch_chain(pdl, step_f64<F, E, uint32_t>, g, t, 0, s, c, src, dst, fields, moments, wait)    \
+               : launch_chain(pdl, step_f64<F, E, size_t>, g, t, 0, s, c, src, dst, fields, moments, wait)
     switch ((first ? 2 : 0) | (explicit_e ? 1 : 0)) {
         case 0: EK_STEP(false, false);
         case 1: EK_STEP(false, true);

@@ -253,6 +253,13 @@ inv_rows(const PoissonPlan pp, const Radices f, const Chan c, double *__restrict
 // a channel of a hundred rows spreads over the GPU: with 256 threads a block,
 // 256 x 128 ran on 4 SMs (FP64: 14 us forward, 11 us inverse) and 512 x 203 on
 // 13 (FP32: 8.5 and 7.6 us).
+// Shared memory asked for, in percent of the largest share: room for the blocks
+// that the registers allow (128 KB at 4096 and 8192), the rest of the SM's memory
+// left to L1 for the twiddles.  With all of it a pass of 10 steps took 2.5 % longer on
+// B200 at 4096 x 1024 FP64 (4.45 ms against 4.33) and at 8192 x 2048 FP32 (9.13
+// against 8.90).
+constexpr int ROW_SMEM_PERCENT = 60;
+
 template <int K> struct RowCfg {
     static constexpr int N = 1 << K, T = N >> 4;
     static constexpr int block = T <= 64 ? 64 : T;  // threads
@@ -893,10 +900,16 @@ batch_tridiag_modes_f32(const PoissonPlan *__restrict__ plans, const int3 *__res
                                     sh.f);
 }
 
-// Modes per block of tridiag_part for n rows, so that every segment has at
-// most TB_L rows (0: too tall, use the one-thread-per-mode `tridiag`).
-int tridiag_modes(int n) {
-    for (int M = 8; M >= 1; M >>= 1)
+// Modes per block of the partitioned solve for n rows, so that every segment
+// has at most TB_L rows (0: too tall, use the one-thread-per-mode `tridiag`),
+// and no more than a channel of nx columns has (rounded up to a power of two):
+// a wide block reads longer runs of a row and scans fewer segments (64 uneven
+// channels: 72.5 ms a cycle with up to 16 modes, 75.6 with up to 8; from 32 on
+// short channels lose more to the fewer blocks than the scan gives back).
+int tridiag_modes(int n, int nx) {
+    int most = 16;
+    while (most > 1 && most / 2 > nx / 2) most /= 2;
+    for (int M = most; M >= 1; M >>= 1)
         if ((n + TB_THREADS / M - 1) / (TB_THREADS / M) <= TB_L) return M;
     return 0;
 }
@@ -930,17 +943,19 @@ template <int K> struct RowLaunch {
     static constexpr int block = RowCfg<K>::block;
     static int grid(const PoissonPlan &pp) { return ((pp.n + 1) / 2 + RowCfg<K>::per - 1) / RowCfg<K>::per; }
     template <typename C> static constexpr size_t smem() { return (size_t)RowCfg<K>::per * RowCfg<K>::N * sizeof(C); }
-    static cudaError_t fwd64(const PoissonPlan &pp, const double *rhs, int nxp, cudaStream_t s) {
-        return launch_pdl(fwd_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, rhs, nxp);
+    static cudaError_t fwd64(const PoissonPlan &pp, const double *rhs, int nxp, bool chain, cudaStream_t s) {
+        if (!chain) return launch_pdl(fwd_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, rhs, nxp);
+        return launch_chain(true, fwd_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, rhs, nxp);
     }
     static cudaError_t inv64(const PoissonPlan &pp, const Chan &c, double *psi, bool pdl, cudaStream_t s) {
-        return launch_maybe_pdl(pdl, inv_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, c, psi);
+        return launch_chain(pdl, inv_rows_f64<K>, dim3(grid(pp)), dim3(block), smem<double2>(), s, pp, c, psi);
     }
-    static cudaError_t fwd32(const PoissonPlan &pp, const Chan &c, cudaStream_t s) {
-        return launch_pdl(fwd_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c);
+    static cudaError_t fwd32(const PoissonPlan &pp, const Chan &c, bool chain, cudaStream_t s) {
+        if (!chain) return launch_pdl(fwd_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c);
+        return launch_chain(true, fwd_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c);
     }
     static cudaError_t inv32(const PoissonPlan &pp, const Chan &c, double *psi, bool write_f64, bool pdl, cudaStream_t s) {
-        return launch_maybe_pdl(pdl, inv_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c, psi, write_f64);
+        return launch_chain(pdl, inv_rows_f32<K>, dim3(grid(pp)), dim3(block), smem<float2>(), s, pp, c, psi, write_f64);
     }
     static cudaError_t limits(bool f32) {
         const void *fns[] = {(const void *)fwd_rows_f64<K>, (const void *)inv_rows_f64<K>, (const void *)fwd_rows_f32<K>,
@@ -948,7 +963,7 @@ template <int K> struct RowLaunch {
         for (int i = 0; i < (f32 ? 4 : 2); ++i) {
             const size_t bytes = i < 2 ? smem<double2>() : smem<float2>();
             cudaError_t e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(fns[i], cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(fns[i], cudaFuncAttributePreferredSharedMemoryCarveout, ROW_SMEM_PERCENT);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -987,31 +1002,33 @@ cudaError_t poisson_pass_f64_at(int pass, const PoissonPlan &pp, const Chan &c, 
                                 cudaStream_t s) {
     const bool pdl = small_channel(pp);
     if (pass == 1) {
-        const int M = tridiag_modes(pp.n);
-        if (M > 0) return launch_maybe_pdl(pdl, tridiag_part, dim3((pp.nx / 2 + M) / M), dim3(TB_THREADS), 0, s, pp, M);
-        return launch_maybe_pdl(pdl, tridiag, dim3((pp.nx / 2 + 1 + PTPB - 1) / PTPB), dim3(PTPB), 0, s, pp);
+        const int M = tridiag_modes(pp.n, pp.nx);
+        if (M > 0) return launch_chain(pdl, tridiag_part, dim3((pp.nx / 2 + M) / M), dim3(TB_THREADS), 0, s, pp, M);
+        return launch_chain(pdl, tridiag, dim3((pp.nx / 2 + 1 + PTPB - 1) / PTPB), dim3(PTPB), 0, s, pp);
     }
     if (use_r16(pp)) {
-        if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd64(pp, rhs, c.nxp, s))
+        if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd64(pp, rhs, c.nxp, pdl, s))
         EK_ROW_DISPATCH(pp.log2nx, inv64(pp, c, psi, pdl, s))
     }
     const Radices f = radices(pp.nx);
     const dim3 grid((pp.n + 1) / 2), block(mixed_threads(pp.nx));
     const size_t smem = poisson_smem_bytes_f64(pp.nx);
-    if (pass == 0) return launch_pdl(fwd_rows, grid, block, smem, s, pp, f, rhs, c.nxp);
-    return launch_maybe_pdl(pdl, inv_rows, grid, block, smem, s, pp, f, c, psi);
+    if (pass == 0)
+        return pdl ? launch_chain(true, fwd_rows, grid, block, smem, s, pp, f, rhs, c.nxp)
+                   : launch_pdl(fwd_rows, grid, block, smem, s, pp, f, rhs, c.nxp);
+    return launch_chain(pdl, inv_rows, grid, block, smem, s, pp, f, c, psi);
 }
 
-int poisson_tridiag_modes(int n) { return tridiag_modes(n); }
+int poisson_tridiag_modes(int n, int nx) { return tridiag_modes(n, nx); }
 
 bool poisson_f32_supported(const PoissonPlan &pp) {
-    return use_r16(pp) && tridiag_modes(pp.n) > 0 && pp.twf && pp.pivf && pp.specf && pp.rowmean && pp.rowmean_ok;
+    return use_r16(pp) && tridiag_modes(pp.n, pp.nx) > 0 && pp.twf && pp.pivf && pp.specf && pp.rowmean && pp.rowmean_ok;
 }
 
 cudaError_t poisson_tridiag_f32(const PoissonPlan &pp, cudaStream_t s) {
     if (!poisson_f32_supported(pp)) return cudaErrorInvalidValue;
-    const int M = tridiag_modes(pp.n);
-    return launch_maybe_pdl(small_channel(pp), tridiag_modes_f32, dim3(1 + (pp.nx / 2 + M - 1) / M), dim3(TB_THREADS), 0, s, pp,
+    const int M = tridiag_modes(pp.n, pp.nx);
+    return launch_chain(small_channel(pp), tridiag_modes_f32, dim3(1 + (pp.nx / 2 + M - 1) / M), dim3(TB_THREADS), 0, s, pp,
                             M);
 }
 
@@ -1019,7 +1036,7 @@ cudaError_t poisson_pass_f32(int pass, const PoissonPlan &pp, const Chan &c, dou
                              cudaStream_t s) {
     // pass B of this form runs through poisson_tridiag_f32
     if (!poisson_f32_supported(pp) || pass == 1) return cudaErrorInvalidValue;
-    if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd32(pp, c, s))
+    if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd32(pp, c, small_channel(pp), s))
     EK_ROW_DISPATCH(pp.log2nx, inv32(pp, c, psi, write_f64, small_channel(pp), s))
 }
 
@@ -1050,7 +1067,7 @@ namespace {
 template <typename F>
 cudaError_t row_limits(F *f, size_t smem) {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, ROW_SMEM_PERCENT);
     return e;
 }
 }  // namespace
