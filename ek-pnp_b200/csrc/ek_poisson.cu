@@ -635,47 +635,76 @@ __device__ __forceinline__ void inv_rows_any(const PoissonPlan &pp, const Chan &
 // d_j = (dy^2 S_j - d_{j-1}) piv_j is linear in the value entering a segment,
 // so each segment first runs with a zero entry value while accumulating the
 // product of (-piv); the true entry values follow from composing the
-// segments' affine maps D -> e + f D in order, a log2(S)-round scan over the
-// segments of each mode in shared memory, and each segment adds its
-// correction.  The backward recurrence x_j = d_j - piv_j x_{j+1} is split the
+// segments' affine maps D -> e + f D in order (seg_carry), and each segment
+// adds its correction.  The backward recurrence x_j = d_j - piv_j x_{j+1} is split the
 // same way.  The result is the Thomas solution, reassociated.
 constexpr int TB_THREADS = 512;
 constexpr int TB_L = 16;
 
+constexpr int TB_WARPS = TB_THREADS / 32;
+constexpr int TB_MODES = 16;  // most modes a block
+
+// Composite maps of each warp's segments, per mode; one set for each sweep.
 template <typename R, typename C> struct TridiagSharedT {
-    C ends[TB_THREADS];
-    R mults[TB_THREADS];
+    C ends[2][TB_WARPS][TB_MODES];
+    R mults[2][TB_WARPS][TB_MODES];
 };
 using TridiagShared = TridiagSharedT<double, double2>;
 
+__device__ __forceinline__ float2 shfl_c(float2 v, int lane) {
+    return make_float2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+__device__ __forceinline__ double2 shfl_c(double2 v, int lane) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
 // Value entering this thread's segment: the affine maps D -> e + f D of the
 // segments of its mode (the block's threads are seg * M + mode) composed in
-// order -- forward from segment 0 (FWD) or backward from segment S-1 -- by a
-// Kogge-Stone scan over the S segments in shared memory (log2 S rounds); the
-// first segment in that order enters with 0.  Every thread of the block
-// calls it.
+// order -- forward from segment 0 (FWD) or backward from segment S-1; the
+// first segment in that order enters with 0.  A warp composes its 32/M
+// segments by shuffles and leaves its total in shared memory; after one barrier
+// each thread runs through the totals of the warps before its own (15 at most).
+// (A Kogge-Stone scan of all segments in shared memory, two barriers a round:
+// 6.7 us a launch at 256 x 128 FP64 on B200 against 5.6, 22.3 against 17.7 at
+// 4096 x 1024.)  Every thread of the block calls it.
 template <bool FWD, typename R, typename C>
-__device__ __forceinline__ C seg_carry(C e, R f, int seg, int S, int M, TridiagSharedT<R, C> &sh) {
-    const int tid = threadIdx.x, mode = tid - seg * M;
-    for (int off = 1; off < S; off <<= 1) {
-        sh.ends[tid] = e;
-        sh.mults[tid] = f;
-        __syncthreads();
-        const int src = FWD ? seg - off : seg + off;
-        if (FWD ? src >= 0 : src < S) {
-            const C e2 = sh.ends[src * M + mode];
-            const R f2 = sh.mults[src * M + mode];
+__device__ __forceinline__ C seg_carry(C e, R f, int M, TridiagSharedT<R, C> &sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mode = lane & (M - 1);
+    for (int off = M; off < 32; off <<= 1) {
+        const int src = FWD ? lane - off : lane + off;
+        const C e2 = shfl_c(e, src & 31);
+        const R f2 = __shfl_sync(0xffffffffu, f, src & 31);
+        if (FWD ? src >= 0 : src < 32) {
             e = cmake<C>(e.x + f * e2.x, e.y + f * e2.y);  // this segment after the earlier ones
             f = f * f2;
         }
-        __syncthreads();
     }
-    sh.ends[tid] = e;
+    constexpr int set = FWD ? 0 : 1;
+    if (FWD ? lane >= 32 - M : lane < M) {
+        sh.ends[set][warp][mode] = e;
+        sh.mults[set][warp][mode] = f;
+    }
     __syncthreads();
-    const int prev = FWD ? seg - 1 : seg + 1;
-    const C out = (FWD ? prev >= 0 : prev < S) ? sh.ends[prev * M + mode] : cmake<C>(0.0, 0.0);
-    __syncthreads();  // sh is written again by the next call
-    return out;
+    C D = cmake<C>(0.0, 0.0);
+    if (FWD) {
+        for (int w = 0; w < warp; ++w) {
+            const C ew = sh.ends[set][w][mode];
+            const R fw = sh.mults[set][w][mode];
+            D = cmake<C>(ew.x + fw * D.x, ew.y + fw * D.y);
+        }
+    } else {
+        for (int w = TB_WARPS - 1; w > warp; --w) {
+            const C ew = sh.ends[set][w][mode];
+            const R fw = sh.mults[set][w][mode];
+            D = cmake<C>(ew.x + fw * D.x, ew.y + fw * D.y);
+        }
+    }
+    // through the segments of this warp before this thread's
+    const int src = FWD ? lane - M : lane + M;
+    const C ep = shfl_c(e, src & 31);
+    const R fp = __shfl_sync(0xffffffffu, f, src & 31);
+    if (FWD ? src >= 0 : src < 32) D = cmake<C>(ep.x + fp * D.x, ep.y + fp * D.y);
+    return D;
 }
 
 // One block of the partitioned solve on a spectrum of type C (pivots R).
@@ -709,7 +738,7 @@ __device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *_
         }
     }
     {
-        const C D = seg_carry<true>(d, mu, seg, S, M, sh);  // true entry value of the segment
+        const C D = seg_carry<true>(d, mu, M, sh);  // true entry value of the segment
         mu = R(1);
 #pragma unroll
         for (int q = 0; q < TB_L; ++q) {
@@ -730,7 +759,7 @@ __device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *_
             v[q] = x;
         }
     }
-    const C X = seg_carry<false>(x, nu, seg, S, M, sh);  // true exit value of the segment (x_n = 0)
+    const C X = seg_carry<false>(x, nu, M, sh);  // true exit value of the segment (x_n = 0)
     if (!mvalid) return;
     nu = R(1);
 #pragma unroll
@@ -903,11 +932,11 @@ batch_tridiag_modes_f32(const PoissonPlan *__restrict__ plans, const int3 *__res
 // Modes per block of the partitioned solve for n rows, so that every segment
 // has at most TB_L rows (0: too tall, use the one-thread-per-mode `tridiag`),
 // and no more than a channel of nx columns has (rounded up to a power of two):
-// a wide block reads longer runs of a row and scans fewer segments (64 uneven
-// channels: 72.5 ms a cycle with up to 16 modes, 75.6 with up to 8; from 32 on
-// short channels lose more to the fewer blocks than the scan gives back).
+// a wide block reads longer runs of a row (64 uneven channels on B200: 71.9 ms a
+// cycle with up to 16 modes, 74.4 with up to 8, 71.5 with up to 32; 256 x 128
+// FP64: 14.6, 14.7 and 15.1 us a step: few blocks).
 int tridiag_modes(int n, int nx) {
-    int most = 16;
+    int most = TB_MODES;
     while (most > 1 && most / 2 > nx / 2) most /= 2;
     for (int M = most; M >= 1; M >>= 1)
         if ((n + TB_THREADS / M - 1) / (TB_THREADS / M) <= TB_L) return M;
