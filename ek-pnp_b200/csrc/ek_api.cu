@@ -318,7 +318,13 @@ int poisson_now(ek_ctx *c, bool write_f64, bool from_moments = false) {
         EK_CUDA(launch_compose_rhs(c->pp, c->chan, rhs, c->stream), "rhs kernel");
         ++c->launches;
     }
-    for (int pass = 0; pass < 3; ++pass) {
+    // one launch for a small channel; with profiling on, the passes by themselves
+    const int blocks = c->prof ? 0 : c->cluster[f32 ? 1 : 0];
+    if (blocks > 0) {
+        EK_CUDA(poisson_cluster(c->pp, c->chan, f32, rhs, psi, write_f64, blocks, c->stream), "poisson kernel");
+        ++c->launches;
+    }
+    for (int pass = 0; pass < 3 && blocks == 0; ++pass) {
         int rc = timed(c, 1 + pass, "poisson kernel", [&] {
             // FP32 form, pass B: the FP64 zero mode rides in the FP32 modes' kernel
             if (f32 && pass == 1) return poisson_tridiag_f32(c->pp, c->stream);
@@ -577,6 +583,8 @@ int ek_create(const ek_params *p, ek_ctx **out) {
     }
     e = poisson_set_smem_limits(c->pp);
     if (e != cudaSuccess) { free_ctx(c); return cuda_fail(e, "context set-up"); }
+    c->cluster[0] = poisson_cluster_blocks(c->pp, false);
+    if (c->pp.specf) c->cluster[1] = poisson_cluster_blocks(c->pp, true);
     refresh_chan(c);
     int rcl = upload_lift(c);
     if (rcl != EK_OK) { free_ctx(c); return rcl; }

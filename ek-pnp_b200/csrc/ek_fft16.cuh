@@ -64,14 +64,8 @@ __device__ __forceinline__ C w16(C z) {
         constexpr bool minus_i = (m == 4) != INV;
         return minus_i ? mk(z.y, -z.x) : mk(-z.y, z.x);
     } else if constexpr ((m & 1) == 0) {
-        // (c + i s) with |c| = |s| = cos(pi/4)
-        constexpr R c = (R)((m == 2 || m == 14) ? R2 : -R2);
-        constexpr R s0 = (R)((m == 2 || m == 6) ? -R2 : R2);  // forward imaginary part
-        constexpr R s = INV ? -s0 : s0;
-        constexpr bool same = (c > 0) == (s > 0);
-        // z (c + i s) = (c z.x - s z.y, s z.x + c z.y)
-        if constexpr (same) return mk(c * (z.x - z.y), c * (z.x + z.y));
-        else return mk(c * (z.x + z.y), c * (z.y - z.x));
+        static_assert(m & 1, "the odd multiples of pi/4 are rot45's");
+        return z;
     } else {
         constexpr double cs[8] = {1.0, C1, R2, S1, 0.0, -S1, -R2, -C1};   // cos(pi j/8), j < 8
         constexpr double sn[8] = {0.0, S1, R2, C1, 1.0, C1, R2, S1};      // sin(pi j/8), j < 8
@@ -82,15 +76,36 @@ __device__ __forceinline__ C w16(C z) {
     }
 }
 
-// 4-point DFT in place: (a, b, c, d) -> (X0, X1, X2, X3)
+// z * exp(-/+ 2 pi i m/16) for m = 2, 6 (odd multiples of pi/4) is R45<m> times
+// rot45<INV, m>(z): the factor is left to the sums that follow (one multiply-add
+// each).
+template <int M> __host__ __device__ constexpr double R45() { return M == 2 ? R2 : -R2; }
+template <bool INV, int M, typename C>
+__device__ __forceinline__ C rot45(C z) {
+    static_assert(M == 2 || M == 6, "m = 2 or 6");
+    // (c + i s) z with s = -c (forward m = 2, inverse m = 6) or s = c
+    return ((M == 2) != INV) ? mk(z.x + z.y, z.y - z.x) : mk(z.x - z.y, z.x + z.y);
+}
+// a + c t for a constant c, rounded once
+__device__ __forceinline__ float2 axpy(double c, float2 t, float2 a) { return __ffma2_rn(make_float2((float)c, (float)c), t, a); }
+__device__ __forceinline__ double2 axpy(double c, double2 t, double2 a) { return make_double2(a.x + c * t.x, a.y + c * t.y); }
+__device__ __forceinline__ float2 times(double c, float2 t) { return __fmul2_rn(make_float2((float)c, (float)c), t); }
+__device__ __forceinline__ double2 times(double c, double2 t) { return make_double2(c * t.x, c * t.y); }
+
+// Second half of a 4-point DFT: s0 = a + c, d0 = a - c, s1 = b + d, d1 = b - d
+// -> X0, X1, X2, X3 in a, b, c, d.
 template <bool INV, typename C>
-__device__ __forceinline__ void dft4(C &a, C &b, C &c, C &d) {
-    const C s0 = a + c, d0 = a - c, s1 = b + d, d1 = b - d;
+__device__ __forceinline__ void dft4_end(C s0, C d0, C s1, C d1, C &a, C &b, C &c, C &d) {
     a = s0 + s1;
     c = s0 - s1;
     const C plus = mk(d0.x - d1.y, d0.y + d1.x), minus = mk(d0.x + d1.y, d0.y - d1.x);  // d0 +- i d1
     b = INV ? plus : minus;
     d = INV ? minus : plus;
+}
+// 4-point DFT in place: (a, b, c, d) -> (X0, X1, X2, X3)
+template <bool INV, typename C>
+__device__ __forceinline__ void dft4(C &a, C &b, C &c, C &d) {
+    dft4_end<INV>(a + c, a - c, b + d, b - d, a, b, c, d);
 }
 
 // 16-point DFT in place; output f sits at x[out16(f)]
@@ -101,17 +116,19 @@ __device__ __forceinline__ void dft16(C (&x)[16]) {
     // 4-point DFTs over n1
 #pragma unroll
     for (int n1 = 0; n1 < 4; ++n1) dft4<INV>(x[n1], x[n1 + 4], x[n1 + 8], x[n1 + 12]);
-    x[5] = w16<INV, 1>(x[5]);
-    x[6] = w16<INV, 2>(x[6]);
-    x[7] = w16<INV, 3>(x[7]);
-    x[9] = w16<INV, 2>(x[9]);
-    x[10] = w16<INV, 4>(x[10]);
-    x[11] = w16<INV, 6>(x[11]);
-    x[13] = w16<INV, 3>(x[13]);
-    x[14] = w16<INV, 6>(x[14]);
-    x[15] = w16<INV, 9>(x[15]);
-#pragma unroll
-    for (int f2 = 0; f2 < 4; ++f2) dft4<INV>(x[4 * f2], x[4 * f2 + 1], x[4 * f2 + 2], x[4 * f2 + 3]);
+    dft4<INV>(x[0], x[1], x[2], x[3]);
+    {  // W^1, W^2, W^3
+        const C b = w16<INV, 1>(x[5]), d = w16<INV, 3>(x[7]), t = rot45<INV, 2>(x[6]);
+        dft4_end<INV>(axpy(R45<2>(), t, x[4]), axpy(-R45<2>(), t, x[4]), b + d, b - d, x[4], x[5], x[6], x[7]);
+    }
+    {  // W^2, W^4, W^6
+        const C c = w16<INV, 4>(x[10]), t = rot45<INV, 2>(x[9]), d = times(R45<6>(), rot45<INV, 6>(x[11]));
+        dft4_end<INV>(x[8] + c, x[8] - c, axpy(R45<2>(), t, d), axpy(R45<2>(), t, mk(-d.x, -d.y)), x[8], x[9], x[10], x[11]);
+    }
+    {  // W^3, W^6, W^9
+        const C b = w16<INV, 3>(x[13]), d = w16<INV, 9>(x[15]), t = rot45<INV, 6>(x[14]);
+        dft4_end<INV>(axpy(R45<6>(), t, x[12]), axpy(-R45<6>(), t, x[12]), b + d, b - d, x[12], x[13], x[14], x[15]);
+    }
 }
 
 // 2^Q-point DFT (Q = 1..3) in place on x[o .. o + 2^Q); output f at x[o + outq<Q>(f)]
@@ -129,15 +146,16 @@ __device__ __forceinline__ void dftq(C *x) {
         // 2-point DFTs over n1
         dft4<INV>(x[0], x[2], x[4], x[6]);
         dft4<INV>(x[1], x[3], x[5], x[7]);
-        x[3] = w16<INV, 2>(x[3]);
-        x[5] = w16<INV, 4>(x[5]);
-        x[7] = w16<INV, 6>(x[7]);
-#pragma unroll
-        for (int f2 = 0; f2 < 4; ++f2) {
-            const C a = x[2 * f2], b = x[2 * f2 + 1];
-            x[2 * f2] = a + b;
-            x[2 * f2 + 1] = a - b;
-        }
+        const C a0 = x[0], b0 = x[1], a2 = x[4], b2 = w16<INV, 4>(x[5]);
+        const C t1 = rot45<INV, 2>(x[3]), t3 = rot45<INV, 6>(x[7]), a1 = x[2], a3 = x[6];
+        x[0] = a0 + b0;
+        x[1] = a0 - b0;
+        x[2] = axpy(R45<2>(), t1, a1);
+        x[3] = axpy(-R45<2>(), t1, a1);
+        x[4] = a2 + b2;
+        x[5] = a2 - b2;
+        x[6] = axpy(R45<6>(), t3, a3);
+        x[7] = axpy(-R45<6>(), t3, a3);
     }
 }
 
@@ -189,6 +207,13 @@ template <int K, int I> __device__ __forceinline__ double2 pass_tw(const double2
     return __ldg(t + ((kb * f) << (K - 4 - Shape<K>::bit(I))));
 }
 
+// Barrier of the threads that run transforms: the whole block (n = 0), or its
+// first n threads (whole warps) where the others have none.
+__device__ __forceinline__ void rows_sync(int n) {
+    if (n == 0) __syncthreads();
+    else asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
+}
+
 // Thread t's group of full pass I: first element and in-group offset kb.
 template <int K, int I>
 __device__ __forceinline__ void group(int t, int &base, int &kb) {
@@ -226,13 +251,13 @@ __device__ __forceinline__ void fwd_pass_load(C (&x)[16], const C *s, int t, int
 
 // Forward passes 2..NF and the partial pass, after pass 1 stored into s.
 template <int K, int I, typename C>
-__device__ __forceinline__ void fwd_rest(C *s, int t, int p, const C *__restrict__ twp) {
+__device__ __forceinline__ void fwd_rest(C *s, int t, int p, const C *__restrict__ twp, int ns = 0) {
     if constexpr (I <= Shape<K>::NF) {
         C x[16];
         fwd_pass_load<K, I>(x, s, t, p);  // a pass writes back onto its group's own slots
         fwd_pass_store<K, I>(x, s, t, p, twp);
-        __syncthreads();
-        fwd_rest<K, I + 1>(s, t, p, twp);
+        rows_sync(ns);
+        fwd_rest<K, I + 1>(s, t, p, twp, ns);
     } else if constexpr (Shape<K>::Q > 0) {
         constexpr int Q = Shape<K>::Q, R = 1 << Q;
         const int sb = swz_base(t << 4, p);
@@ -245,7 +270,7 @@ __device__ __forceinline__ void fwd_rest(C *s, int t, int p, const C *__restrict
         for (int j = 0; j < 16; j += R)
 #pragma unroll
             for (int f = 0; f < R; ++f) s[sb ^ (j + brevq(f, Q))] = x[j + outq<Q>(f)];
-        __syncthreads();
+        rows_sync(ns);
     }
 }
 
@@ -283,18 +308,18 @@ __device__ __forceinline__ void inv_pass_store(const C (&x)[16], C *s, int t, in
 // Inverse passes NF..2 (after the partial pass); pass 1 is left to the caller,
 // which takes its output from registers.
 template <int K, int I, typename C>
-__device__ __forceinline__ void inv_full(C *s, int t, int p, const C *__restrict__ twp) {
+__device__ __forceinline__ void inv_full(C *s, int t, int p, const C *__restrict__ twp, int ns = 0) {
     if constexpr (I >= 2) {
         C x[16];
         inv_pass_load<K, I>(x, s, t, p, twp);
         inv_pass_store<K, I>(x, s, t, p);
-        __syncthreads();
-        inv_full<K, I - 1>(s, t, p, twp);
+        rows_sync(ns);
+        inv_full<K, I - 1>(s, t, p, twp, ns);
     }
 }
 
 template <int K, typename C>
-__device__ __forceinline__ void inv_partial(C *s, int t, int p) {
+__device__ __forceinline__ void inv_partial(C *s, int t, int p, int ns = 0) {
     if constexpr (Shape<K>::Q > 0) {
         constexpr int Q = Shape<K>::Q, R = 1 << Q;
         const int sb = swz_base(t << 4, p);
@@ -312,7 +337,7 @@ __device__ __forceinline__ void inv_partial(C *s, int t, int p) {
 #pragma unroll
             for (int v = 0; v < R; ++v) s[sb ^ (j + v)] = y[v];
         }
-        __syncthreads();
+        rows_sync(ns);
     }
 }
 

@@ -337,6 +337,12 @@ cudaError_t batch_tridiag_f32(const PoissonPlan *plans, const void *items, int n
 cudaError_t batch_poisson(int pass, const PoissonPlan *plans, const Chan *chans, double *const *fields,
                           const void *items, int nitems, int block, bool write_f64, cudaStream_t s);
 int batch_row_block(int nx_max);
+// The whole solve of a small channel in one launch, by one cluster of `blocks`
+// blocks: poisson_cluster_blocks of the plan (0: the separate passes), looked up
+// outside a capture.
+int poisson_cluster_blocks(const PoissonPlan &pp, bool f32);
+cudaError_t poisson_cluster(const PoissonPlan &pp, const Chan &c, bool f32, const double *rhs, double *psi, bool write_f64,
+                            int blocks, cudaStream_t s);
 int poisson_tridiag_modes(int n, int nx);
 // Steady-state residual sums (ek_residual.cu): per channel 8 FP64 sums,
 // (q - q_snap)^2 then q^2 for q in (ux, c+, c-, psi); the snapshot is updated.

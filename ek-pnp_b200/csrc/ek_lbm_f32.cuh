@@ -275,17 +275,19 @@ template <typename V> __device__ __forceinline__ void reframe_up_wall(V p[9], co
 }
 
 // Ion anti-bounce-back in deviations: d_ibar = -q_i + 2 w_i (c_wall - R).
+template <typename V> __device__ __forceinline__ V wall_reflect(float w2, V dcw, V q) {
+    return vaxpy(w2, dcw, vscale(-1.0f, q));
+}
 template <typename V> __device__ __forceinline__ void ion_wall_dev(const V q[9], V dcw, V p[9]) {
-    const V m0 = vscale(2.0f * W0F, dcw), ms = vscale(2.0f * WSF, dcw), md = vscale(2.0f * WDF, dcw);
-    p[0] = vsub(m0, q[0]);
-    p[3] = vsub(ms, q[1]);
-    p[4] = vsub(ms, q[2]);
-    p[1] = vsub(ms, q[3]);
-    p[2] = vsub(ms, q[4]);
-    p[7] = vsub(md, q[5]);
-    p[8] = vsub(md, q[6]);
-    p[5] = vsub(md, q[7]);
-    p[6] = vsub(md, q[8]);
+    p[0] = wall_reflect(2.0f * W0F, dcw, q[0]);
+    p[3] = wall_reflect(2.0f * WSF, dcw, q[1]);
+    p[4] = wall_reflect(2.0f * WSF, dcw, q[2]);
+    p[1] = wall_reflect(2.0f * WSF, dcw, q[3]);
+    p[2] = wall_reflect(2.0f * WSF, dcw, q[4]);
+    p[7] = wall_reflect(2.0f * WDF, dcw, q[5]);
+    p[8] = wall_reflect(2.0f * WDF, dcw, q[6]);
+    p[5] = wall_reflect(2.0f * WDF, dcw, q[7]);
+    p[6] = wall_reflect(2.0f * WDF, dcw, q[8]);
 }
 
 // Moments with opposite directions paired first.  In the double layer the
@@ -334,23 +336,23 @@ __device__ __forceinline__ float div36(float v) { return v * (1.0f / 36.0f); }
 //    force source sm cfl dt F is split the same way.
 // Ions (not FLUID) relax their flux to 4 dens c/36 per pair unit: the ion
 // flux is not conserved, so no factor accumulates.
-// Pairs are carried doubled (d1 + d3, d1 - d3), which is exact.
+// Pairs are carried doubled (d1 + d3, d1 - d3), which is exact.  Which sums take
+// a product unrounded (vfma) is part of the form: runs repeat earlier ones bit
+// for bit, FP16 storage too, whose rounding any other choice would scatter.
 template <bool FORCE, bool FLUID, typename V>
 __device__ __forceinline__ void trt_f32(V d[9], V ddens, V dens, V ux, V uy, bool rest_fluid, V usq_fluid, float wp,
                                         float wm, const ChanF &k, V fx, V fy, V px, V py) {
     const V vsq = vfma(ux, ux, vmul(uy, uy));
     const V base = vfma(vscale(-k.hinvcs2, vsq), dens, ddens);
     const V cx = vscale(k.kcu, ux), cy = vscale(k.kcu, uy);
-    const V qx = vmul(dens, cx), qy = vmul(dens, cy);
-    // symmetric equilibria: straight pairs (doubled), diagonal mass and xy
+    // symmetric equilibria: straight pairs, diagonal mass (z / 9) and xy (q9 / 9)
     // moments, rest remainder
-    const V b9 = vscale(WSF, base), ax = vscale(1.0f / 9.0f, qx), ay = vscale(1.0f / 9.0f, qy);
-    const V xx = vmul(ax, cx), yy = vmul(ay, cy);
-    const V seq13 = vaxpy(2.0f, b9, xx), seq24 = vaxpy(2.0f, b9, yy);
-    const V seq_s = vaxpy(0.5f, xx, vaxpy(0.5f, yy, b9));
-    const V seq_q = vmul(ax, cy);
-    V e0 = vsub(ddens, vadd(vadd(seq13, seq24), seq_s));
-    if (rest_fluid) e0 = vfma(vscale(W0F * k.hinvcs2, dens), vsub(vsq, usq_fluid), e0);
+    const V seq13 = vscale(WSF, vfma(dens, vmul(vscale(0.5f, cx), cx), base));
+    const V seq24 = vscale(WSF, vfma(dens, vmul(vscale(0.5f, cy), cy), base));
+    const V z = vfma(dens, vscale(0.5f, vfma(cx, cx, vmul(cy, cy))), base);
+    const V q9 = vmul(dens, vmul(cx, cy));
+    V e0 = vsub(ddens, vaxpy(1.0f / 9.0f, z, vaxpy(2.0f, seq13, vscale(2.0f, seq24))));
+    if (rest_fluid) e0 = vfma(vscale(W0F, dens), vscale(k.hinvcs2, vsub(vsq, usq_fluid)), e0);
     // antisymmetric equilibria (half-pair units: a13 = (d1 - d3)/2, X = d5 - d6 - d7 + d8)
     V aq13, aqx, aq24, aqy;
     if (FLUID) {
@@ -359,35 +361,38 @@ __device__ __forceinline__ void trt_f32(V d[9], V ddens, V dens, V ux, V uy, boo
         aq24 = vscale(1.0f / 3.0f, py);
         aqy = vaxpy(-2.0f, aq24, py);
     } else {
-        aq13 = aqx = ax;
-        aq24 = aqy = ay;
+        aq13 = aqx = vscale(1.0f / 9.0f, vmul(dens, cx));
+        aq24 = aqy = vscale(1.0f / 9.0f, vmul(dens, cy));
     }
     const V nwp = bc<V>(-wp), nwm = bc<V>(-wm);
     V d0 = vfma(nwp, vsub(d[0], e0), d[0]);
     V s13 = vadd(d[1], d[3]), a13 = vsub(d[1], d[3]);
     V s24 = vadd(d[2], d[4]), a24 = vsub(d[2], d[4]);
-    s13 = vfma(nwp, vsub(s13, seq13), s13);
+    s13 = vfma(nwp, vaxpy(-2.0f, seq13, s13), s13);
     a13 = vfma(nwm, vaxpy(-2.0f, aq13, a13), a13);
-    s24 = vfma(nwp, vsub(s24, seq24), s24);
+    s24 = vfma(nwp, vaxpy(-2.0f, seq24, s24), s24);
     a24 = vfma(nwm, vaxpy(-2.0f, aq24, a24), a24);
     const V A = vsub(d[5], d[6]), B = vsub(d[8], d[7]);  // x-differences of values from one row
     const V C = vadd(d[5], d[6]), D = vadd(d[7], d[8]);
     V X = vadd(A, B), Q = vsub(A, B), Y = vsub(C, D), S = vadd(C, D);
-    S = vfma(nwp, vsub(S, seq_s), S);
-    Q = vfma(nwp, vsub(Q, seq_q), Q);
+    S = vfma(nwp, vaxpy(-1.0f / 9.0f, z, S), S);
+    Q = vfma(nwp, vaxpy(-1.0f / 9.0f, q9, Q), Q);
     X = vfma(nwm, vsub(X, aqx), X);
     Y = vfma(nwm, vsub(Y, aqy), Y);
     if (FORCE) {
-        const V nuF = vscale(-k.inv_cs2, vfma(ux, fx, vmul(uy, fy)));
+        const V uF = vscale(k.inv_cs2, vfma(ux, fx, vmul(uy, fy)));
         const V cfx = vscale(k.gF, fx), cfy = vscale(k.gF, fy);
-        const float sp9 = k.sp * k.dt * WSF;
+        const float sp = k.sp * k.dt;
         // symmetric (mass-free) part: the rest takes the remainder
-        const V t13 = vfma(cx, cfx, nuF), t24 = vfma(cy, cfy, nuF), ts = vfma(cx, cfx, t24);
-        d0 = vaxpy(-sp9, vaxpy(2.0f, vadd(t13, t24), ts), d0);
-        s13 = vaxpy(2.0f * sp9, t13, s13);
-        s24 = vaxpy(2.0f * sp9, t24, s24);
-        S = vaxpy(sp9, ts, S);
-        Q = vaxpy(sp9, vfma(cx, cfy, vmul(cy, cfx)), Q);
+        const V g13 = vscale(sp, vscale(WSF, vfma(cx, cfx, vscale(-1.0f, uF))));
+        const V g24 = vscale(sp, vscale(WSF, vfma(cy, cfy, vscale(-1.0f, uF))));
+        const V ws = vscale(1.0f / 9.0f, vsub(vfma(cx, cfx, vmul(cy, cfy)), uF));
+        const V wq = vscale(1.0f / 9.0f, vfma(cx, cfy, vmul(cy, cfx)));
+        d0 = vsub(d0, vaxpy(sp, ws, vaxpy(2.0f, g13, vscale(2.0f, g24))));
+        s13 = vaxpy(2.0f, g13, s13);
+        s24 = vaxpy(2.0f, g24, s24);
+        S = vaxpy(sp, ws, S);
+        Q = vaxpy(sp, wq, Q);
         // momentum: sm cfl dt F, a third to each straight half-pair unit
         const V fsx = vscale(k.srcF, fx), fsy = vscale(k.srcF, fy);
         const V q13 = vscale(1.0f / 3.0f, fsx), q24 = vscale(1.0f / 3.0f, fsy);

@@ -66,9 +66,9 @@ template <bool INV> __device__ __forceinline__ double2 rot90(double2 z) {
 
 template <bool INV, int R>
 __device__ __forceinline__ void radix_pass(const double2 *__restrict__ in, double2 *__restrict__ out, int nx, int L,
-                                           const double2 *__restrict__ tw) {
+                                           const double2 *__restrict__ tw, int t, int T) {
     const int m = nx / R, ts = nx / (L * R);
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+    for (int j = t; j < m; j += T) {
         const int hi = j / L, k = j - hi * L;
         double2 x[R];
 #pragma unroll
@@ -116,9 +116,9 @@ __device__ __forceinline__ void radix_pass(const double2 *__restrict__ in, doubl
 // A pass of prime radix r > 5: one output a thread, its r terms summed in order.
 template <bool INV>
 __device__ __forceinline__ void prime_pass(const double2 *__restrict__ in, double2 *__restrict__ out, int nx, int L,
-                                           int r, const double2 *__restrict__ tw) {
+                                           int r, const double2 *__restrict__ tw, int t, int T) {
     const int m = nx / r, ts = nx / (L * r);
-    for (int e = threadIdx.x; e < nx; e += blockDim.x) {
+    for (int e = t; e < nx; e += T) {
         const int qo = e / m, j = e - qo * m, hi = j / L, k = j - hi * L;
         // exponent of term q: q (k ts + qo m) mod nx
         int step = k * ts + qo * m;
@@ -134,49 +134,57 @@ __device__ __forceinline__ void prime_pass(const double2 *__restrict__ in, doubl
     }
 }
 
-// Transform of nx points in a (b: the other buffer), natural order in and out;
-// returns the buffer that holds the result.  Every thread of the block calls it.
+// Transform of nx points in a (b: the other buffer) by threads t < T of a group,
+// natural order in and out; returns the buffer that holds the result.  Every
+// thread of the block calls it, with the same nx.
 template <bool INV>
-__device__ double2 *mixed_fft(double2 *a, double2 *b, int nx, const Radices &f, const double2 *__restrict__ tw) {
+__device__ double2 *mixed_fft(double2 *a, double2 *b, int nx, const Radices &f, const double2 *__restrict__ tw, int t,
+                              int T, int ns) {
     int L = 1;
     for (int i = 0; i < f.n; ++i) {
         const int r = f.r[i];
-        __syncthreads();
+        fft16::rows_sync(ns);
         switch (r) {
-            case 2: radix_pass<INV, 2>(a, b, nx, L, tw); break;
-            case 3: radix_pass<INV, 3>(a, b, nx, L, tw); break;
-            case 4: radix_pass<INV, 4>(a, b, nx, L, tw); break;
-            case 5: radix_pass<INV, 5>(a, b, nx, L, tw); break;
-            default: prime_pass<INV>(a, b, nx, L, r, tw); break;
+            case 2: radix_pass<INV, 2>(a, b, nx, L, tw, t, T); break;
+            case 3: radix_pass<INV, 3>(a, b, nx, L, tw, t, T); break;
+            case 4: radix_pass<INV, 4>(a, b, nx, L, tw, t, T); break;
+            case 5: radix_pass<INV, 5>(a, b, nx, L, tw, t, T); break;
+            default: prime_pass<INV>(a, b, nx, L, r, tw, t, T); break;
         }
-        double2 *t = a;
+        double2 *swap = a;
         a = b;
-        b = t;
+        b = swap;
         L *= r;
     }
-    __syncthreads();
+    fft16::rows_sync(ns);
     return a;
 }
 
-// Pass A: rows y0 = 2*b+1 and y1 = y0+1 of the right-hand side -> spectra.
-__global__ void __launch_bounds__(PTPB)
-fwd_rows(const PoissonPlan pp, const Radices f, const double *__restrict__ rhs, int nxp) {
-    extern __shared__ double2 sm[];
-    pdl_wait();
-    const int nx = pp.nx;
-    const int j0 = 2 * blockIdx.x, j1 = j0 + 1;
-    const bool two = j1 < pp.n;
+// Pass A of any length: row pair (2 pair + 1, 2 pair + 2) of the right-hand side
+// -> spectra, by threads t < T of a group (z: 2 nx points of shared memory).
+__device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Radices &f, const double *__restrict__ rhs,
+                                                 int nxp, int pair, bool live, double2 *z0, int t, int T, int ns = 0) {
+    const int nx = pp.nx, j0 = 2 * pair, j1 = j0 + 1;
+    const bool two = live && j1 < pp.n;
     const double *r0 = rhs + (size_t)(j0 + 1) * nxp;
     const double *r1 = rhs + (size_t)(j1 + 1) * nxp;
-    for (int x = threadIdx.x; x < nx; x += blockDim.x) sm[x] = make_double2(r0[x], two ? r1[x] : 0.0);
-    const double2 *z = mixed_fft<false>(sm, sm + nx, nx, f, pp.tw);
+    for (int x = t; x < nx; x += T) z0[x] = make_double2(live ? r0[x] : 0.0, two ? r1[x] : 0.0);
+    const double2 *z = mixed_fft<false>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
+    if (!live) return;
     // unpack the two real-input spectra: A = (Z[m] + conj Z[-m])/2, B = (Z[m] - conj Z[-m])/(2i)
     double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
-    for (int m = threadIdx.x; m <= nx / 2; m += blockDim.x) {
+    for (int m = t; m <= nx / 2; m += T) {
         const double2 a = z[m], b = cconj(z[m == 0 ? 0 : nx - m]);
         s0[m] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
         if (two) s1[m] = make_double2(0.5 * (a.y - b.y), -0.5 * (a.x - b.x));
     }
+}
+
+__global__ void __launch_bounds__(PTPB)
+fwd_rows(const PoissonPlan pp, const Radices f, const double *__restrict__ rhs, int nxp) {
+    extern __shared__ double2 sm[];
+    pdl_wait();
+    fwd_rows_any_len(pp, f, rhs, nxp, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
 }
 
 // Pass B: one thread per x-mode, Thomas sweep over the n interior rows.
@@ -220,30 +228,35 @@ __device__ __forceinline__ void write_walls(double *__restrict__ psi, const doub
     }
 }
 
-// Pass C: spectra of rows (y0, y1) -> psi rows; the walls spread over the blocks.
+// Pass C of any length: spectra of a row pair -> psi rows.
+__device__ __forceinline__ void inv_rows_any_len(const PoissonPlan &pp, const Radices &f, int nxp, double *__restrict__ psi,
+                                                 int pair, bool live, double2 *z0, int t, int T, int ns = 0) {
+    const int nx = pp.nx, j0 = 2 * pair, j1 = j0 + 1;
+    const bool two = live && j1 < pp.n;
+    const double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
+    for (int m = t; m <= nx / 2; m += T) {
+        const double2 a = live ? s0[m] : make_double2(0.0, 0.0);
+        const double2 b = two ? s1[m] : make_double2(0.0, 0.0);
+        // Z[m] = A + iB, Z[-m] = conj(A) + i conj(B)
+        z0[m] = make_double2(a.x - b.y, a.y + b.x);
+        if (m != 0 && 2 * m != nx) z0[nx - m] = make_double2(a.x + b.y, -a.y + b.x);
+    }
+    const double2 *z = mixed_fft<true>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
+    if (!live) return;
+    const double inv = 1.0 / (double)nx;
+    double *p0 = psi + (size_t)(j0 + 1) * nxp, *p1 = psi + (size_t)(j1 + 1) * nxp;
+    for (int x = t; x < nx; x += T) {
+        p0[x] = z[x].x * inv;
+        if (two) p1[x] = z[x].y * inv;
+    }
+}
+
 __global__ void __launch_bounds__(PTPB)
 inv_rows(const PoissonPlan pp, const Radices f, const Chan c, double *__restrict__ psi) {
     extern __shared__ double2 sm[];
     pdl_wait();
-    const int nx = pp.nx, nxp = c.nxp;
-    write_walls(psi, c.zlo, c.zhi, nx, c.ny, nxp, blockIdx.x, gridDim.x, blockDim.x);
-    const int j0 = 2 * blockIdx.x, j1 = j0 + 1;
-    const bool two = j1 < pp.n;
-    const double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
-    for (int m = threadIdx.x; m <= nx / 2; m += blockDim.x) {
-        const double2 a = s0[m];
-        const double2 b = two ? s1[m] : make_double2(0.0, 0.0);
-        // Z[m] = A + iB, Z[-m] = conj(A) + i conj(B)
-        sm[m] = make_double2(a.x - b.y, a.y + b.x);
-        if (m != 0 && 2 * m != nx) sm[nx - m] = make_double2(a.x + b.y, -a.y + b.x);
-    }
-    const double2 *z = mixed_fft<true>(sm, sm + nx, nx, f, pp.tw);
-    const double inv = 1.0 / (double)nx;
-    double *p0 = psi + (size_t)(j0 + 1) * nxp, *p1 = psi + (size_t)(j1 + 1) * nxp;
-    for (int x = threadIdx.x; x < nx; x += blockDim.x) {
-        p0[x] = z[x].x * inv;
-        if (two) p1[x] = z[x].y * inv;
-    }
+    write_walls(psi, c.zlo, c.zhi, pp.nx, c.ny, c.nxp, blockIdx.x, gridDim.x, blockDim.x);
+    inv_rows_any_len(pp, f, c.nxp, psi, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
 }
 
 // ---- radix-16 row transforms (power-of-two nx >= 16) -----------------------
@@ -267,26 +280,25 @@ template <int K> struct RowCfg {
 };
 #define EK_ROW_CASES(F) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13)
 
-// Pass A, FP64: row pairs (2p+1, 2p+2) of the right-hand side -> spectra.  The
-// first radix-16 pass runs on the values as loaded.
+// Pass A, FP64, of the row pairs pair_base + p (p: the transform's index in the
+// block) below pair_end: right-hand side -> spectra.  The first radix-16 pass
+// runs on the values as loaded.
 template <int K>
-__global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
-fwd_rows_f64(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
-    extern __shared__ double2 sm[];
+__device__ __forceinline__ void fwd_rows_f64_k(const PoissonPlan &pp, const double *__restrict__ rhs, int nxp, int pair_base,
+                                               int pair_end, double2 *sm, int ns = 0) {
     using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
-    pdl_wait();
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
     double2 *s = sm + p * N;
-    const int j0 = 2 * (blockIdx.x * RowCfg<K>::per + p), j1 = j0 + 1;
-    const bool live = j0 < pp.n, two = j1 < pp.n;
+    const int pair = pair_base + p, j0 = 2 * pair, j1 = j0 + 1;
+    const bool live = pair < pair_end, two = live && j1 < pp.n;
     const double *r0 = rhs + (size_t)(j0 + 1) * nxp + t, *r1 = r0 + nxp;
     double2 x[16];
 #pragma unroll
     for (int v = 0; v < 16; ++v) x[v] = make_double2(live ? __ldg(r0 + v * T) : 0.0, two ? __ldg(r1 + v * T) : 0.0);
     fft16::fwd_pass_store<K, 1>(x, s, t, p, pp.tw);
-    __syncthreads();
-    fft16::fwd_rest<K, 2>(s, t, p, pp.tw);
+    fft16::rows_sync(ns);
+    fft16::fwd_rest<K, 2>(s, t, p, pp.tw, ns);
     if (!live) return;
     double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
     for (int m = t; m <= N / 2; m += T) {
@@ -298,19 +310,16 @@ fwd_rows_f64(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
 }
 
 // Pass C, FP64: spectra -> psi rows (stored from registers by the last
-// radix-16 pass) and the walls.
+// radix-16 pass).
 template <int K>
-__global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
-inv_rows_f64(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
-    extern __shared__ double2 sm[];
+__device__ __forceinline__ void inv_rows_f64_k(const PoissonPlan &pp, int nxp, double *__restrict__ psi, int pair_base,
+                                               int pair_end, double2 *sm, int ns = 0) {
     using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
-    pdl_wait();
-    write_walls(psi, c.zlo, c.zhi, N, c.ny, c.nxp, blockIdx.x, gridDim.x, blockDim.x);
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
     double2 *s = sm + p * N;
-    const int j0 = 2 * (blockIdx.x * RowCfg<K>::per + p), j1 = j0 + 1;
-    const bool live = j0 < pp.n, two = j1 < pp.n;
+    const int pair = pair_base + p, j0 = 2 * pair, j1 = j0 + 1;
+    const bool live = pair < pair_end, two = live && j1 < pp.n;
     const double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
@@ -320,19 +329,36 @@ inv_rows_f64(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
         s[fft16::swz_base(brev(m, K), p)] = make_double2(a.x - b.y, a.y + b.x);  // A + iB
         if (m != 0 && 2 * m != N) s[fft16::swz_base(brev(N - m, K), p)] = make_double2(a.x + b.y, -a.y + b.x);
     }
-    __syncthreads();
-    fft16::inv_partial<K>(s, t, p);
-    fft16::inv_full<K, S::NF>(s, t, p, pp.tw);
+    fft16::rows_sync(ns);
+    fft16::inv_partial<K>(s, t, p, ns);
+    fft16::inv_full<K, S::NF>(s, t, p, pp.tw, ns);
     double2 x[16];
     fft16::inv_pass_load<K, 1>(x, s, t, p, pp.tw);
     if (!live) return;
     constexpr double inv = 1.0 / (double)N;
-    double *p0 = psi + (size_t)(j0 + 1) * c.nxp + t, *p1 = p0 + c.nxp;
+    double *p0 = psi + (size_t)(j0 + 1) * nxp + t, *p1 = p0 + nxp;
 #pragma unroll
     for (int v = 0; v < 16; ++v) {
         p0[v * T] = x[v].x * inv;
         if (two) p1[v * T] = x[v].y * inv;
     }
+}
+
+template <int K>
+__global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
+fwd_rows_f64(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
+    extern __shared__ double2 sm[];
+    pdl_wait();
+    fwd_rows_f64_k<K>(pp, rhs, nxp, blockIdx.x * RowCfg<K>::per, (pp.n + 1) / 2, sm);
+}
+
+template <int K>
+__global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
+inv_rows_f64(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
+    extern __shared__ double2 sm[];
+    pdl_wait();
+    write_walls(psi, c.zlo, c.zhi, pp.nx, c.ny, c.nxp, blockIdx.x, gridDim.x, blockDim.x);
+    inv_rows_f64_k<K>(pp, c.nxp, psi, blockIdx.x * RowCfg<K>::per, (pp.n + 1) / 2, sm);
 }
 
 // ---- FP32 form of passes A and C ------------------------------------------
@@ -345,18 +371,18 @@ inv_rows_f64(const PoissonPlan pp, const Chan c, double *__restrict__ psi) {
 // groups contiguous in the block); every thread of the block calls it and
 // gets the group's first lane's (or the block-level) value.
 template <int BLOCK>
-__device__ __forceinline__ double group_sum(double v, int T, double *red) {
+__device__ __forceinline__ double group_sum(double v, int T, double *red, int ns = 0) {
     const int w = T < 32 ? T : 32;
     for (int o = w >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (T < 32) return __shfl_sync(0xffffffffu, v, (threadIdx.x & 31) & ~(T - 1));
     v = __shfl_sync(0xffffffffu, v, 0);
     if (T == 32) return v;
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
+    fft16::rows_sync(ns);
     const int nw = T >> 5, g0 = (int)(threadIdx.x / T) * nw;
     double s = 0.0;
     for (int i = 0; i < nw; ++i) s += red[g0 + i];
-    __syncthreads();
+    fft16::rows_sync(ns);
     return s;
 }
 
@@ -369,27 +395,25 @@ __device__ __forceinline__ double group_sum(double v, int T, double *red) {
 // x-fluctuation is in rhsf).
 // From the second solve on the offset is the previous solve's row mean and
 // one pass over the row does both; the first solve takes two passes and the
-// exact mean.  The offset is rounded to FP32 first, so that the value minus
-// the offset rounds once, as one FP32 subtraction.  The first radix-16 pass
-// runs on the values as loaded.
+// exact mean.  The first radix-16 pass runs on the values as loaded.
 template <int BLOCK, int K>
-__device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan &c, int pair_base, float2 *sm,
-                                               double *red) {
+__device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan &c, int pair_base, int pair_end,
+                                               float2 *sm, double *red, int ns = 0) {
     using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
     const int pair = pair_base + p;
     float2 *s = sm + p * N;
     const int j0 = 2 * pair, j1 = j0 + 1;
-    const bool live = j0 < pp.n, two = j1 < pp.n;
+    const bool live = pair < pair_end, two = live && j1 < pp.n;
     const int nxp = c.nxp;
     // 32-bit offsets from the planes' base pointers (a plane is below 2^32
     // elements: one channel's planes fit device memory)
     const unsigned r0 = (unsigned)(j0 + 1) * (unsigned)nxp + (unsigned)t, r1 = r0 + (unsigned)nxp;
     const double k0 = live ? rhs_row_constant(pp, c, j0 + 1) : 0.0, k1 = two ? rhs_row_constant(pp, c, j1 + 1) : 0.0;
     const bool exact = *pp.rowmean_ok == 0;  // the same for every block of the launch
-    // value - offset = rhsf + (row constant - offset)
-    float d0 = (live && !exact) ? (float)(k0 - pp.rowmean[j0]) : 0.0f, d1 = (two && !exact) ? (float)(k1 - pp.rowmean[j1]) : 0.0f;
+    // value - offset = rhsf + (row constant - offset), rounded once
+    double d0 = (live && !exact) ? k0 - pp.rowmean[j0] : 0.0, d1 = (two && !exact) ? k1 - pp.rowmean[j1] : 0.0;
     double a0 = 0.0, a1 = 0.0;
     float2 x[16];
     if constexpr (T == 1) {  // a row a thread: 16 consecutive values
@@ -409,19 +433,33 @@ __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan
             x[v] = make_float2(live ? __ldg(pp.rhsf + (r0 + (unsigned)(v * T))) : 0.0f,
                                two ? __ldg(pp.rhsf + (r1 + (unsigned)(v * T))) : 0.0f);
     }
+    auto less_offset = [&](bool sum) {
 #pragma unroll
-    for (int v = 0; v < 16; ++v) {
-        a0 += (double)x[v].x;
-        a1 += (double)x[v].y;
-    }
-    a0 = group_sum<BLOCK>(a0, T, red) + (double)N * k0;
-    a1 = group_sum<BLOCK>(a1, T, red) + (double)N * k1;
+        for (int v = 0; v < 16; ++v) {
+            const double f0 = (double)x[v].x, f1 = (double)x[v].y;
+            if (sum) {
+                a0 += f0;
+                a1 += f1;
+            }
+            x[v] = make_float2((float)(f0 + d0), (float)(f1 + d1));
+        }
+    };
     if (exact) {
-        d0 = live ? (float)(k0 - a0 / (double)N) : 0.0f;
-        d1 = two ? (float)(k1 - a1 / (double)N) : 0.0f;
-    }
 #pragma unroll
-    for (int v = 0; v < 16; ++v) x[v] = __fadd2_rn(x[v], make_float2(d0, d1));
+        for (int v = 0; v < 16; ++v) {
+            a0 += (double)x[v].x;
+            a1 += (double)x[v].y;
+        }
+    } else {
+        less_offset(true);
+    }
+    a0 = group_sum<BLOCK>(a0, T, red, ns) + (double)N * k0;
+    a1 = group_sum<BLOCK>(a1, T, red, ns) + (double)N * k1;
+    if (exact) {
+        d0 = live ? k0 - a0 / (double)N : 0.0;
+        d1 = two ? k1 - a1 / (double)N : 0.0;
+        less_offset(false);
+    }
     if (t == 0 && live) {
         pp.spec[(size_t)j0 * pp.mp] = make_double2(a0, 0.0);
         pp.rowmean[j0] = a0 / (double)N;
@@ -431,8 +469,8 @@ __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan
         }
     }
     fft16::fwd_pass_store<K, 1>(x, s, t, p, pp.twf);
-    __syncthreads();
-    fft16::fwd_rest<K, 2>(s, t, p, pp.twf);
+    fft16::rows_sync(ns);
+    fft16::fwd_rest<K, 2>(s, t, p, pp.twf, ns);
     if (!live) return;
     const unsigned q0 = (unsigned)j0 * (unsigned)pp.mp, q1 = q0 + (unsigned)pp.mp;
     auto mode = [&](int m, float2 *A, float2 *B) {
@@ -490,17 +528,15 @@ __device__ __forceinline__ void write_walls_f32(const PoissonPlan &pp, const Cha
 // (mean + fluctuation) when write_f64.
 template <int BLOCK, int K>
 __device__ __forceinline__ void inv_rows_f32_k(const PoissonPlan &pp, const Chan &c, double *__restrict__ psi,
-                                               bool write_f64, int pair_base, float2 *sm) {
+                                               bool write_f64, int pair_base, int pair_end, float2 *sm, int ns = 0) {
     using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
     const int p = threadIdx.x / T, t = threadIdx.x - p * T;
     const int pair = pair_base + p;
     float2 *s = sm + p * N;
     const int j0 = 2 * pair, j1 = j0 + 1;
-    const bool live = j0 < pp.n, two = j1 < pp.n;
+    const bool live = pair < pair_end, two = live && j1 < pp.n;
     const int nxp = c.nxp;
-    constexpr int per = BLOCK / T;
-    write_walls_f32(pp, c, psi, write_f64, pair_base / per, ((pp.n + 1) / 2 + per - 1) / per, BLOCK);
     // 32-bit offsets from the planes' base pointers (as in fwd_rows_f32_k)
     const unsigned q0 = (unsigned)j0 * (unsigned)pp.mp, q1 = q0 + (unsigned)pp.mp;
     // modes m = t + i T (i < 8) and, for t = 0, m = N/2: all loads first
@@ -536,9 +572,9 @@ __device__ __forceinline__ void inv_rows_f32_k(const PoissonPlan &pp, const Chan
         if (m != 0 && 2 * m != N)
             s[fft16::swz_base(brev(N - m, K), p)] = make_float2(a[i].x + b[i].y, -a[i].y + b[i].x);
     }
-    __syncthreads();
-    fft16::inv_partial<K>(s, t, p);
-    fft16::inv_full<K, S::NF>(s, t, p, pp.twf);
+    fft16::rows_sync(ns);
+    fft16::inv_partial<K>(s, t, p, ns);
+    fft16::inv_full<K, S::NF>(s, t, p, pp.twf, ns);
     float2 x[16];
     fft16::inv_pass_load<K, 1>(x, s, t, p, pp.twf);
     const double inv = 1.0 / (double)N;
@@ -586,7 +622,7 @@ fwd_rows_f32(const PoissonPlan pp, const Chan c) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[(RowCfg<K>::block + 31) / 32];
     pdl_wait();
-    fwd_rows_f32_k<RowCfg<K>::block, K>(pp, c, blockIdx.x * RowCfg<K>::per, (float2 *)smraw, red);
+    fwd_rows_f32_k<RowCfg<K>::block, K>(pp, c, blockIdx.x * RowCfg<K>::per, (pp.n + 1) / 2, (float2 *)smraw, red);
 }
 
 template <int K>
@@ -594,7 +630,8 @@ __global__ void __launch_bounds__(RowCfg<K>::block, 1024 / RowCfg<K>::block)
 inv_rows_f32(const PoissonPlan pp, const Chan c, double *__restrict__ psi, bool write_f64) {
     extern __shared__ __align__(16) unsigned char smraw[];
     pdl_wait();
-    inv_rows_f32_k<RowCfg<K>::block, K>(pp, c, psi, write_f64, blockIdx.x * RowCfg<K>::per, (float2 *)smraw);
+    write_walls_f32(pp, c, psi, write_f64, blockIdx.x, gridDim.x, blockDim.x);
+    inv_rows_f32_k<RowCfg<K>::block, K>(pp, c, psi, write_f64, blockIdx.x * RowCfg<K>::per, (pp.n + 1) / 2, (float2 *)smraw);
 }
 
 // Sizes that a batch block of BLOCK threads runs, whole transforms only.
@@ -605,7 +642,7 @@ __device__ __forceinline__ void fwd_rows_any(const PoissonPlan &pp, const Chan &
     switch (pp.log2nx) {
 #define EK_CASE(K)                                                                                     \
     case K:                                                                                            \
-        if constexpr (batch_fits<BLOCK, K>()) fwd_rows_f32_k<BLOCK, K>(pp, c, pair_base, sm, red);     \
+        if constexpr (batch_fits<BLOCK, K>()) fwd_rows_f32_k<BLOCK, K>(pp, c, pair_base, (pp.n + 1) / 2, sm, red); \
         break;
         EK_ROW_CASES(EK_CASE)
 #undef EK_CASE
@@ -616,10 +653,13 @@ __device__ __forceinline__ void fwd_rows_any(const PoissonPlan &pp, const Chan &
 template <int BLOCK>
 __device__ __forceinline__ void inv_rows_any(const PoissonPlan &pp, const Chan &c, double *__restrict__ psi, bool write_f64,
                                              int pair_base, float2 *sm) {
+    const int per = BLOCK / (pp.nx >> 4);
+    write_walls_f32(pp, c, psi, write_f64, pair_base / per, ((pp.n + 1) / 2 + per - 1) / per, BLOCK);
     switch (pp.log2nx) {
 #define EK_CASE(K)                                                                                                 \
     case K:                                                                                                        \
-        if constexpr (batch_fits<BLOCK, K>()) inv_rows_f32_k<BLOCK, K>(pp, c, psi, write_f64, pair_base, sm);      \
+        if constexpr (batch_fits<BLOCK, K>())                                                                      \
+            inv_rows_f32_k<BLOCK, K>(pp, c, psi, write_f64, pair_base, (pp.n + 1) / 2, sm);                        \
         break;
         EK_ROW_CASES(EK_CASE)
 #undef EK_CASE
@@ -642,18 +682,24 @@ constexpr int TB_THREADS = 512;
 constexpr int TB_L = 16;
 
 constexpr int TB_WARPS = TB_THREADS / 32;
-constexpr int TB_MODES = 16;  // most modes a block
+constexpr int TB_MODES = 16;      // most modes a block, FP64
+constexpr int TB_MODES_F32 = 8;   // FP32
 
-// Composite maps of each warp's segments, per mode; one set for each sweep.
-template <typename R, typename C> struct TridiagSharedT {
-    C ends[2][TB_WARPS][TB_MODES];
-    R mults[2][TB_WARPS][TB_MODES];
+// Shared memory of the carries.  FP64: composite maps of each warp's segments,
+// per mode, one set for each sweep.  FP32: the segments' maps, two sets used in
+// turn by the scan's rounds.
+struct TridiagShared {
+    double2 ends[2][TB_WARPS][TB_MODES];
+    double mults[2][TB_WARPS][TB_MODES];
 };
-using TridiagShared = TridiagSharedT<double, double2>;
+struct TridiagSharedF {
+    float2 ends[2][TB_THREADS];
+    float mults[2][TB_THREADS];
+};
+template <typename R> struct SharedOf;
+template <> struct SharedOf<double> { using type = TridiagShared; };
+template <> struct SharedOf<float> { using type = TridiagSharedF; };
 
-__device__ __forceinline__ float2 shfl_c(float2 v, int lane) {
-    return make_float2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
-}
 __device__ __forceinline__ double2 shfl_c(double2 v, int lane) {
     return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
 }
@@ -667,8 +713,10 @@ __device__ __forceinline__ double2 shfl_c(double2 v, int lane) {
 // (A Kogge-Stone scan of all segments in shared memory, two barriers a round:
 // 6.7 us a launch at 256 x 128 FP64 on B200 against 5.6, 22.3 against 17.7 at
 // 4096 x 1024.)  Every thread of the block calls it.
-template <bool FWD, typename R, typename C>
-__device__ __forceinline__ C seg_carry(C e, R f, int M, TridiagSharedT<R, C> &sh) {
+template <bool FWD>
+__device__ __forceinline__ double2 seg_carry(double2 e, double f, int M, TridiagShared &sh) {
+    using C = double2;
+    using R = double;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mode = lane & (M - 1);
     for (int off = M; off < 32; off <<= 1) {
         const int src = FWD ? lane - off : lane + off;
@@ -707,21 +755,59 @@ __device__ __forceinline__ C seg_carry(C e, R f, int M, TridiagSharedT<R, C> &sh
     return D;
 }
 
-// One block of the partitioned solve on a spectrum of type C (pivots R).
-template <typename R, typename C>
-__device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *__restrict__ spec, int n, int nx,
-                                                 size_t mp, R dy2, int M, int m_base, TridiagSharedT<R, C> &sh) {
+// The same in FP32, by a Kogge-Stone scan over the S segments in shared memory,
+// one barrier a round.  (The order of the products is part of a result's
+// rounding: FP16 and FP32 runs repeat earlier ones bit for bit with this one.)
+template <bool FWD>
+__device__ __forceinline__ float2 seg_carry(float2 e, float f, int M, TridiagSharedF &sh) {
+    const int tid = threadIdx.x, S = TB_THREADS / M, seg = tid / M, mode = tid & (M - 1);
+    int set = 0;
+    for (int off = 1; off < S; off <<= 1, set ^= 1) {
+        sh.ends[set][tid] = e;
+        sh.mults[set][tid] = f;
+        __syncthreads();
+        const int src = FWD ? seg - off : seg + off;
+        if (FWD ? src >= 0 : src < S) {
+            const float2 e2 = sh.ends[set][src * M + mode];
+            const float f2 = sh.mults[set][src * M + mode];
+            e = make_float2(e.x + f * e2.x, e.y + f * e2.y);  // this segment after the earlier ones
+            f = f * f2;
+        }
+    }
+    sh.ends[set][tid] = e;
+    __syncthreads();
+    const int prev = FWD ? seg - 1 : seg + 1;
+    const float2 out = (FWD ? prev >= 0 : prev < S) ? sh.ends[set][prev * M + mode] : make_float2(0.0f, 0.0f);
+    __syncthreads();  // sh is written again by the next call
+    return out;
+}
+
+// (v - d) c with the difference and the product rounded (d, a product itself, is
+// not fused into the difference: FP32 keeps the rounding of earlier runs).
+__device__ __forceinline__ float2 rn_sub_mul(float2 v, float2 d, float c) {
+    return make_float2(__fmul_rn(__fsub_rn(v.x, d.x), c), __fmul_rn(__fsub_rn(v.y, d.y), c));
+}
+__device__ __forceinline__ double2 rn_sub_mul(double2 v, double2 d, double c) {
+    return make_double2((v.x - d.x) * c, (v.y - d.y) * c);
+}
+
+// One block of the partitioned solve on a spectrum of type C (pivots R), with
+// segments of at most LMAX rows.  Rows past the end carry zero pivots and values,
+// which pass zero on in either direction, so the sweeps need no row test.
+template <int LMAX, typename R, typename C>
+__device__ __forceinline__ void tridiag_part_len(const R *__restrict__ piv, C *__restrict__ spec, int n, int nx,
+                                                 size_t mp, R dy2, int M, int m_base, typename SharedOf<R>::type &sh) {
     const int mlast = nx / 2;
-    const int tid = threadIdx.x, mode = tid % M, seg = tid / M, S = TB_THREADS / M;
+    const int tid = threadIdx.x, mode = tid & (M - 1), S = TB_THREADS / M, seg = tid / M;
     const int m = m_base + mode;
     const bool mvalid = m <= mlast;
     const int L = (n + S - 1) / S, ja = seg * L, cnt = max(0, min(n, ja + L) - ja);
     const unsigned o = (unsigned)ja * (unsigned)mp + (unsigned)m;  // n mp < 2^32 (n <= 8192)
-    R c[TB_L];
-    C v[TB_L];
+    R c[LMAX];
+    C v[LMAX];
     pdl_wait();
 #pragma unroll
-    for (int q = 0; q < TB_L; ++q) {
+    for (int q = 0; q < LMAX; ++q) {
         const bool on = mvalid && q < cnt;
         c[q] = on ? __ldg(piv + (o + q * (unsigned)mp)) : R(0);
         const C sv = on ? spec[o + q * (unsigned)mp] : cmake<C>(0.0, 0.0);
@@ -730,45 +816,53 @@ __device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *_
     C d = cmake<C>(0.0, 0.0);
     R mu = R(1);
 #pragma unroll
-    for (int q = 0; q < TB_L; ++q) {
-        if (q < cnt) {
-            d = cmake<C>((v[q].x - d.x) * c[q], (v[q].y - d.y) * c[q]);
-            mu = -c[q] * mu;
-            v[q] = d;
-        }
+    for (int q = 0; q < LMAX; ++q) {
+        d = rn_sub_mul(v[q], d, c[q]);
+        mu = -c[q] * mu;
+        v[q] = d;
+        // the segment's own end, where L < LMAX (the same for every thread)
+        if (LMAX > 1 && q + 1 == L) break;
     }
     {
         const C D = seg_carry<true>(d, mu, M, sh);  // true entry value of the segment
         mu = R(1);
 #pragma unroll
-        for (int q = 0; q < TB_L; ++q) {
-            if (q < cnt) {
-                mu = -c[q] * mu;
-                v[q].x += mu * D.x;
-                v[q].y += mu * D.y;
-            }
+        for (int q = 0; q < LMAX; ++q) {
+            mu = -c[q] * mu;
+            v[q].x += mu * D.x;
+            v[q].y += mu * D.y;
         }
     }
     C x = cmake<C>(0.0, 0.0);
     R nu = R(1);
 #pragma unroll
-    for (int q = TB_L - 1; q >= 0; --q) {
-        if (q < cnt) {
-            x = cmake<C>(v[q].x - c[q] * x.x, v[q].y - c[q] * x.y);
-            nu = -c[q] * nu;
-            v[q] = x;
-        }
+    for (int q = LMAX - 1; q >= 0; --q) {
+        if (q >= L) continue;
+        x = cmake<C>(v[q].x - c[q] * x.x, v[q].y - c[q] * x.y);
+        nu = -c[q] * nu;
+        v[q] = x;
     }
     const C X = seg_carry<false>(x, nu, M, sh);  // true exit value of the segment (x_n = 0)
     if (!mvalid) return;
     nu = R(1);
 #pragma unroll
-    for (int q = TB_L - 1; q >= 0; --q) {
+    for (int q = LMAX - 1; q >= 0; --q) {
         if (q < cnt) {
             nu = -c[q] * nu;
             spec[o + q * (unsigned)mp] = cmake<C>(v[q].x + nu * X.x, v[q].y + nu * X.y);
         }
     }
+}
+
+// The form for the segments' length: a sweep unrolled to 16 rows costs a channel
+// of 7 rows a segment more than twice its arithmetic (FP64 most of all).
+template <typename R, typename C>
+__device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *__restrict__ spec, int n, int nx,
+                                                 size_t mp, R dy2, int M, int m_base, typename SharedOf<R>::type &sh) {
+    const int S = TB_THREADS / M, L = (n + S - 1) / S;
+    if (L <= 4) tridiag_part_len<4, R, C>(piv, spec, n, nx, mp, dy2, M, m_base, sh);
+    else if (L <= 8) tridiag_part_len<8, R, C>(piv, spec, n, nx, mp, dy2, M, m_base, sh);
+    else tridiag_part_len<TB_L, R, C>(piv, spec, n, nx, mp, dy2, M, m_base, sh);
 }
 
 __device__ __forceinline__ void tridiag_part_dev(const PoissonPlan &pp, int M, int m_base, TridiagShared &sh) {
@@ -783,7 +877,7 @@ __global__ void __launch_bounds__(TB_THREADS) tridiag_part(const PoissonPlan pp,
 // Shared memory of the FP32 form's column kernel: the FP32 modes' segment
 // ends, or the zero mode's per-warp scan totals.
 union ColumnShared {
-    TridiagSharedT<float, float2> f;
+    TridiagSharedF f;
     double wtot[TB_THREADS / 32];
 };
 
@@ -834,13 +928,13 @@ __device__ __forceinline__ void zero_mode_f64(const PoissonPlan &pp, ColumnShare
     pdl_wait();
     // segment sum of h, then H at the segment's start
     double s1 = 0.0;
-    for (int q = 0; q < cnt; ++q) s1 += dy2 * __ldg(col + (size_t)(ja + q) * stride);
+    for (int q = 0; q < cnt; ++q) s1 += dy2 * col[(size_t)(ja + q) * stride];
     double tot;
     const double h0 = block_scan(s1, sh, &tot) - s1;  // H_{ja - 1}
     // segment sum of H, then the sum of H before the segment and over all rows
     double H = h0, s2 = 0.0;
     for (int q = 0; q < cnt; ++q) {
-        H += dy2 * __ldg(col + (size_t)(ja + q) * stride);
+        H += dy2 * col[(size_t)(ja + q) * stride];
         s2 += H;
     }
     double S;
@@ -850,7 +944,7 @@ __device__ __forceinline__ void zero_mode_f64(const PoissonPlan &pp, ColumnShare
     double G = G0;
     for (int q = 0; q < cnt; ++q) {
         const int j = ja + q;
-        const double hj = dy2 * __ldg(col + (size_t)j * stride);
+        const double hj = dy2 * col[(size_t)j * stride];
         col[(size_t)j * stride] = (double)(j + 1) * g0 + G;
         H += hj;
         G += H;
@@ -868,6 +962,106 @@ __global__ void __launch_bounds__(TB_THREADS, 2) tridiag_modes_f32(const Poisson
     }
     tridiag_part_gen<float, float2>(pp.pivf, pp.specf, pp.n, pp.nx, (size_t)pp.mp, (float)pp.dy2, M,
                                     1 + (blockIdx.x - 1) * M, sh.f);
+}
+
+// ---- a small channel's whole solve in one launch ------------------------------
+//
+// One cluster of up to 16 blocks runs passes A, B and C with the cluster's
+// barrier between them: three launches' boundaries cost a channel of a few
+// thousand nodes more than the passes' work.  Each block takes an equal share of
+// the row pairs, then every gridDim.x-th group of modes; the spectrum goes
+// through L2.  The arithmetic is that of the separate passes, group for group, so
+// the bits are theirs.  On larger channels 16 SMs are too few
+// (poisson_cluster_blocks has the line and both sides).
+constexpr int CL_THREADS = TB_THREADS;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+union ClusterShared {
+    ColumnShared col;
+    TridiagShared col64;
+    double red[CL_THREADS / 32];
+};
+
+// Row pairs a block takes per round: as many as its threads hold, fewer where
+// the channel's pairs then spread over all blocks.
+__device__ __forceinline__ int cluster_share(int pairs, int per) {
+    const int k = (pairs + (int)gridDim.x - 1) / (int)gridDim.x;
+    return k < per ? k : per;
+}
+
+// Threads of the whole warps that `live` threads fill.
+__device__ __forceinline__ int rows_threads(int live) { return (live + 31) & ~31; }
+
+template <int K>
+__global__ void __launch_bounds__(CL_THREADS, 1)
+solve_cluster_f32(const PoissonPlan pp, const Chan c, double *__restrict__ psi, bool write_f64, int M) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ ClusterShared sh;
+    float2 *sm = (float2 *)smraw;
+    pdl_wait();
+    const int b = blockIdx.x, nb = gridDim.x, pairs = (pp.n + 1) / 2;
+    const int k = cluster_share(pairs, CL_THREADS / fft16::Shape<K>::T);
+    const int ns = rows_threads(k * fft16::Shape<K>::T);  // warps without a row pair take no part
+    if ((int)threadIdx.x < ns)
+        for (int p0 = b * k; p0 < pairs; p0 += nb * k) {
+            fwd_rows_f32_k<CL_THREADS, K>(pp, c, p0, min(pairs, p0 + k), sm, sh.red, ns);
+            fft16::rows_sync(ns);
+        }
+    cluster_barrier();
+    const int groups = 1 + (pp.nx / 2 + M - 1) / M;
+    for (int g = b; g < groups; g += nb) {
+        if (g == 0) zero_mode_f64(pp, sh.col);
+        else
+            tridiag_part_gen<float, float2>(pp.pivf, pp.specf, pp.n, pp.nx, (size_t)pp.mp, (float)pp.dy2, M, 1 + (g - 1) * M,
+                                            sh.col.f);
+        __syncthreads();
+    }
+    cluster_barrier();
+    write_walls_f32(pp, c, psi, write_f64, b, nb, CL_THREADS);
+    if ((int)threadIdx.x < ns)
+        for (int p0 = b * k; p0 < pairs; p0 += nb * k) {
+            inv_rows_f32_k<CL_THREADS, K>(pp, c, psi, write_f64, p0, min(pairs, p0 + k), sm, ns);
+            fft16::rows_sync(ns);
+        }
+}
+
+// FP64: K = log2 nx of the radix-16 transforms, 0 for any other length (T
+// threads a row pair).
+template <int K>
+__global__ void __launch_bounds__(CL_THREADS, 1)
+solve_cluster_f64(const PoissonPlan pp, const Radices f, int T, const Chan c, const double *__restrict__ rhs,
+                  double *__restrict__ psi, int M) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ ClusterShared sh;
+    double2 *sm = (double2 *)smraw;
+    pdl_wait();
+    const int b = blockIdx.x, nb = gridDim.x, pairs = (pp.n + 1) / 2;
+    const int k = cluster_share(pairs, CL_THREADS / T), t = threadIdx.x % T, q = threadIdx.x / T;
+    const int ns = rows_threads(k * T);  // warps without a row pair take no part
+    if ((int)threadIdx.x < ns)
+        for (int p0 = b * k; p0 < pairs; p0 += nb * k) {
+            if constexpr (K > 0) fwd_rows_f64_k<K>(pp, rhs, c.nxp, p0, min(pairs, p0 + k), sm, ns);
+            else fwd_rows_any_len(pp, f, rhs, c.nxp, p0 + q, q < k && p0 + q < pairs, sm + (size_t)q * 2 * pp.nx, t, T, ns);
+            fft16::rows_sync(ns);
+        }
+    cluster_barrier();
+    const int groups = (pp.nx / 2 + M) / M;
+    for (int g = b; g < groups; g += nb) {
+        tridiag_part_dev(pp, M, g * M, sh.col64);
+        __syncthreads();
+    }
+    cluster_barrier();
+    write_walls(psi, c.zlo, c.zhi, pp.nx, c.ny, c.nxp, b, nb, CL_THREADS);
+    if ((int)threadIdx.x < ns)
+        for (int p0 = b * k; p0 < pairs; p0 += nb * k) {
+            if constexpr (K > 0) inv_rows_f64_k<K>(pp, c.nxp, psi, p0, min(pairs, p0 + k), sm, ns);
+            else inv_rows_any_len(pp, f, c.nxp, psi, p0 + q, q < k && p0 + q < pairs, sm + (size_t)q * 2 * pp.nx, t, T, ns);
+            fft16::rows_sync(ns);
+        }
 }
 
 // ---- batched passes: one launch for many channels -------------------------
@@ -932,11 +1126,11 @@ batch_tridiag_modes_f32(const PoissonPlan *__restrict__ plans, const int3 *__res
 // Modes per block of the partitioned solve for n rows, so that every segment
 // has at most TB_L rows (0: too tall, use the one-thread-per-mode `tridiag`),
 // and no more than a channel of nx columns has (rounded up to a power of two):
-// a wide block reads longer runs of a row (64 uneven channels on B200: 71.9 ms a
-// cycle with up to 16 modes, 74.4 with up to 8, 71.5 with up to 32; 256 x 128
-// FP64: 14.6, 14.7 and 15.1 us a step: few blocks).
-int tridiag_modes(int n, int nx) {
-    int most = TB_MODES;
+// a wide block reads longer runs of a row (256 x 128 FP64 on B200: 14.6 us a step
+// with up to 16 modes, 14.7 with up to 8, 15.1 with up to 32: few blocks).  FP32
+// keeps 8, and with it the segments and the rounding of earlier runs.
+int tridiag_modes(int n, int nx, bool f32) {
+    int most = f32 ? TB_MODES_F32 : TB_MODES;
     while (most > 1 && most / 2 > nx / 2) most /= 2;
     for (int M = most; M >= 1; M >>= 1)
         if ((n + TB_THREADS / M - 1) / (TB_THREADS / M) <= TB_L) return M;
@@ -1031,7 +1225,7 @@ cudaError_t poisson_pass_f64_at(int pass, const PoissonPlan &pp, const Chan &c, 
                                 cudaStream_t s) {
     const bool pdl = small_channel(pp);
     if (pass == 1) {
-        const int M = tridiag_modes(pp.n, pp.nx);
+        const int M = tridiag_modes(pp.n, pp.nx, false);
         if (M > 0) return launch_chain(pdl, tridiag_part, dim3((pp.nx / 2 + M) / M), dim3(TB_THREADS), 0, s, pp, M);
         return launch_chain(pdl, tridiag, dim3((pp.nx / 2 + 1 + PTPB - 1) / PTPB), dim3(PTPB), 0, s, pp);
     }
@@ -1048,15 +1242,15 @@ cudaError_t poisson_pass_f64_at(int pass, const PoissonPlan &pp, const Chan &c, 
     return launch_chain(pdl, inv_rows, grid, block, smem, s, pp, f, c, psi);
 }
 
-int poisson_tridiag_modes(int n, int nx) { return tridiag_modes(n, nx); }
+int poisson_tridiag_modes(int n, int nx) { return tridiag_modes(n, nx, true); }
 
 bool poisson_f32_supported(const PoissonPlan &pp) {
-    return use_r16(pp) && tridiag_modes(pp.n, pp.nx) > 0 && pp.twf && pp.pivf && pp.specf && pp.rowmean && pp.rowmean_ok;
+    return use_r16(pp) && tridiag_modes(pp.n, pp.nx, true) > 0 && pp.twf && pp.pivf && pp.specf && pp.rowmean && pp.rowmean_ok;
 }
 
 cudaError_t poisson_tridiag_f32(const PoissonPlan &pp, cudaStream_t s) {
     if (!poisson_f32_supported(pp)) return cudaErrorInvalidValue;
-    const int M = tridiag_modes(pp.n, pp.nx);
+    const int M = tridiag_modes(pp.n, pp.nx, true);
     return launch_chain(small_channel(pp), tridiag_modes_f32, dim3(1 + (pp.nx / 2 + M - 1) / M), dim3(TB_THREADS), 0, s, pp,
                             M);
 }
@@ -1067,6 +1261,88 @@ cudaError_t poisson_pass_f32(int pass, const PoissonPlan &pp, const Chan &c, dou
     if (!poisson_f32_supported(pp) || pass == 1) return cudaErrorInvalidValue;
     if (pass == 0) EK_ROW_DISPATCH(pp.log2nx, fwd32(pp, c, small_channel(pp), s))
     EK_ROW_DISPATCH(pp.log2nx, inv32(pp, c, psi, write_f64, small_channel(pp), s))
+}
+
+namespace {
+
+// Threads a row pair and shared memory of the cluster's blocks.
+int cluster_row_threads(const PoissonPlan &pp) {
+    if (use_r16(pp)) return pp.nx >> 4;
+    int t = 32;
+    while (t < CL_THREADS && 4 * t < pp.nx) t *= 2;
+    return t;
+}
+size_t cluster_smem(const PoissonPlan &pp, bool f32) {
+    const int per = CL_THREADS / cluster_row_threads(pp);
+    return (size_t)per * pp.nx * (f32 ? sizeof(float2) : (use_r16(pp) ? 1 : 2) * sizeof(double2));
+}
+// The kernel of a plan: nx = 16 to 256, or a length of the mixed form in FP64.
+const void *cluster_kernel(const PoissonPlan &pp, bool f32) {
+    if (!use_r16(pp)) return f32 ? nullptr : (const void *)solve_cluster_f64<0>;
+    switch (pp.log2nx) {
+#define EK_CASE(K) \
+    case K: return f32 ? (const void *)solve_cluster_f32<K> : (const void *)solve_cluster_f64<K>;
+        EK_CASE(4) EK_CASE(5) EK_CASE(6) EK_CASE(7) EK_CASE(8)
+#undef EK_CASE
+        default: return nullptr;
+    }
+}
+
+}  // namespace
+
+int poisson_cluster_blocks(const PoissonPlan &pp, bool f32) {
+    // microseconds a step on B200, one launch against three: 16 x 101 FP64 10.4 against
+    // 14.0, 64 x 64 12.4 against 12.6 (FP32 13.0 against 14.4), 64 x 128 12.8
+    // against 12.3; 512 x 33 16.9 against 14.4; mixed lengths 10 x 101 11.5
+    // against 13.5, 100 x 100 14.7 against 16.1, 300 x 60 16.2 against 18.2
+    const size_t most = use_r16(pp) ? (size_t)8192 : (size_t)16384;
+    if ((size_t)pp.nx * pp.ny > most || tridiag_modes(pp.n, pp.nx, f32) == 0) return 0;
+    const void *fn = cluster_kernel(pp, f32);
+    const size_t smem = cluster_smem(pp, f32);
+    if (!fn || smem > 200 * 1024) return 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    for (int blocks = 16; blocks >= 8; blocks /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(CL_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {(unsigned)blocks, 1, 1};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) return blocks;
+        (void)cudaGetLastError();
+    }
+    return 0;
+}
+
+cudaError_t poisson_cluster(const PoissonPlan &pp, const Chan &c, bool f32, const double *rhs, double *psi, bool write_f64,
+                            int blocks, cudaStream_t s) {
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim = {(unsigned)blocks, 1, 1};
+    const dim3 g(blocks), t(CL_THREADS);
+    const size_t smem = cluster_smem(pp, f32);
+    const int M = tridiag_modes(pp.n, pp.nx, f32), T = cluster_row_threads(pp);
+    const Radices f = use_r16(pp) ? Radices{} : radices(pp.nx);
+    if (!use_r16(pp)) return launch_attrs(at, 2, solve_cluster_f64<0>, g, t, smem, s, pp, f, T, c, rhs, psi, M);
+    switch (pp.log2nx) {
+#define EK_CASE(K)                                                                                                  \
+    case K:                                                                                                         \
+        return f32 ? launch_attrs(at, 2, solve_cluster_f32<K>, g, t, smem, s, pp, c, psi, write_f64, M)             \
+                   : launch_attrs(at, 2, solve_cluster_f64<K>, g, t, smem, s, pp, f, T, c, rhs, psi, M);
+        EK_CASE(4) EK_CASE(5) EK_CASE(6) EK_CASE(7) EK_CASE(8)
+#undef EK_CASE
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 int batch_row_block(int nx_max) { return nx_max <= 1024 ? 64 : 256; }

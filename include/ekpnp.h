@@ -295,7 +295,9 @@ int ek_poisson_noalloc(const ek_params *p, const double *cp, const double *cn,
 
 /* ---- profiling (CUDA events on the context's stream) ------------------
  * Phases of a step: 0 = fused LBM kernel, 1 = Poisson pass A (row FFTs),
- * 2 = pass B (tridiagonal y-solve), 3 = pass C (inverse row FFTs).
+ * 2 = pass B (tridiagonal y-solve), 3 = pass C (inverse row FFTs).  With
+ * profiling on every phase is a kernel by itself; a channel of a few thousand
+ * nodes otherwise runs phases 1 to 3 in one launch, to the same bits.
  * ek_profile_enable(ctx, 1) resets and starts per-launch timing;
  * ek_profile_read waits for the stream and returns, per phase, the summed
  * kernel milliseconds and the launch count since the last enable. */

@@ -69,3 +69,24 @@ def test_chained_steps_equal_single_steps(nx, ny, storage):
     a, b = run(p, init, [24]), run(p, init, [1] * 24)
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 4), (16, 401), (32, 33), (64, 128), (128, 17), (256, 31), (2, 9), (10, 101), (97, 12),
+                                   (100, 150), (128, 65), (512, 12)])
+@pytest.mark.parametrize("storage", [0, 1, 2], ids=["f64", "f32", "f16"])
+def test_one_launch_solve_equals_the_passes(nx, ny, storage):
+    """A small channel's Poisson solve in one launch gives the bits of the
+    three passes (which profiling runs by themselves), at both sides of the
+    node count up to which it is taken."""
+    import ekpnp
+    p, init = start(nx, ny, storage)
+    out = []
+    for profile in (False, True):
+        with ekpnp.Channel(p) as ch:
+            ch.set_fields(**init)
+            ch.init_equilibrium()
+            ch.profile(profile)
+            ch.step(12)
+            out.append(ch.get_fields())
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
