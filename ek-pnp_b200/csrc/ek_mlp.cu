@@ -10,8 +10,8 @@
 //              waits), tcgen05.ld and a fused epilogue (bias, SiLU, SiLU
 //              derivative, BF16 and transposed BF16 stores).
 //   training   per iteration: batch gather, 4 forward GEMMs, MSE loss and its
-//              gradient, 3 backward-data and 4 weight-gradient GEMMs, bias
-//              gradients, Adam on FP32 master weights, BF16 weight casts --
+//              gradient, 3 backward-data GEMMs with 4 weight-gradient GEMMs and
+//              bias gradients beside them, Adam on FP32 master weights, BF16 casts --
 //              16 launches, captured once in a CUDA graph and replayed.
 // Weights are used in BF16 with FP32 accumulation; the FP32 master copy, the
 // Adam moments and the gradients live in one flat buffer laid out per layer
@@ -368,7 +368,6 @@ __global__ void bias_grads(const BiasSeg s, int B) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     int l = 0, n = w;
     while (l < NL && n >= s.rows[l]) n -= s.rows[l++];
-    ek::pdl_wait();
     if (l >= NL) return;
     const bf16 *r = s.dzt[l] + (size_t)n * B;
     float acc = 0.0f;
@@ -379,8 +378,8 @@ __global__ void bias_grads(const BiasSeg s, int B) {
 
 // Adam on the flat FP32 parameters, four a thread; step count t = *step + 1.
 // The two bias corrections (FP64 powers) are computed by two threads of the
-// block before the wait for the gradients (*step was advanced by the previous
-// iteration's last kernel): in every thread they were half the kernel's time.
+// block: in every thread they were half the kernel's time. An ordinary launch:
+// it waits for both streams of the backward pass.
 __global__ void __launch_bounds__(256) adam_update(float4 *__restrict__ p, const float4 *__restrict__ g,
                                                    float4 *__restrict__ m, float4 *__restrict__ v, int64_t n4, float lr,
                                                    float b1, float b2, float eps, const int64_t *__restrict__ step) {
@@ -390,7 +389,6 @@ __global__ void __launch_bounds__(256) adam_update(float4 *__restrict__ p, const
         corr[threadIdx.x >> 5] = (float)(1.0 - pow((double)(threadIdx.x ? b2 : b1), t));
     }
     __syncthreads();
-    ek::pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n4) return;
     const float c1 = corr[0], c2 = corr[1];
@@ -458,6 +456,8 @@ __global__ void __launch_bounds__(256) cast_weights(const CastSeg s, int64_t *__
 struct ek_mlp {
     int B = 256;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;              // weight and bias gradients, beside the backward chain
+    cudaEvent_t ready[4] = {}, joined = nullptr;  // delta of layer 3, 2, 1, 0 written; the gradients done
     int64_t nparam = 0;
     int64_t off_w[NL], off_b[NL];
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // flat FP32
@@ -524,9 +524,14 @@ int tile_columns(int m, int n) {
     return 16;
 }
 
+// pdl: programmatic launch; an ordinary one where another stream is waited for too.
 template <int EPI>
-cudaError_t gemm(const GemmArgs &a, cudaStream_t s) {
+cudaError_t gemm(const GemmArgs &a, cudaStream_t s, bool pdl = true) {
     const size_t smem = (size_t)a.zoff + (EPI == EPI_BWD_HIDDEN ? epi_f32_bytes(a.nt) : 0);
+    if (!pdl) {
+        mlp_gemm<EPI><<<dim3(a.m / TM, a.n / a.nt), GT, smem, s>>>(a);
+        return cudaGetLastError();
+    }
     return ek::launch_pdl(mlp_gemm<EPI>, dim3(a.m / TM, a.n / a.nt), dim3(GT), smem, s, a);
 }
 
@@ -582,13 +587,23 @@ int backward(ek_mlp *q, bool counted) {
     EK_MCUDA(ek::launch_pdl(mse_grad, dim3(B / 32, OUT / 64), dim3(256), 0, q->stream, q->y, q->t, B, q->dy, q->dyt,
                             q->loss, counted ? q->step : nullptr, counted ? q->base : nullptr),
              "loss kernel");
+    // The weight and bias gradients run on a second stream beside the chain of
+    // deltas: no kernel of the chain reads them, none of them fills more than a
+    // fraction of the SMs, and each costs a launch's latency when it is waited
+    // for (an iteration of 256 rows on B200: 66 us one after the other, 55 us
+    // so). Adam waits for both streams.
+    auto fork = [&](int i) -> cudaError_t {
+        cudaError_t e = cudaEventRecord(q->ready[i], q->stream);
+        return e == cudaSuccess ? cudaStreamWaitEvent(q->side, q->ready[i], 0) : e;
+    };
+    EK_MCUDA(fork(0), "gradient stream");
     // layer 3: dW3 = dY^T H2, dZ2 = (dY W3) * silu'(Z2)
     {
         GemmArgs a;
         EK_MCUDA(gemm_args(a, q->dyt, B, q->ht[2], B, OUT, HID, B, q->err, q->wait_cycles), "operand maps");
         a.c = q->g + q->off_w[3];
         a.ldc = HID;
-        EK_MCUDA(gemm<EPI_F32>(a, q->stream), "weight-gradient GEMM");
+        EK_MCUDA(gemm<EPI_F32>(a, q->side, false), "weight-gradient GEMM");
     }
     const bf16 *up = q->dy;
     int ldup = OUT;
@@ -603,13 +618,14 @@ int backward(ek_mlp *q, bool counted) {
         a.ht = q->dzt[l];
         a.ldht = B;
         EK_MCUDA(gemm<EPI_BWD_HIDDEN>(a, q->stream), "backward GEMM");
+        EK_MCUDA(fork(3 - l), "gradient stream");
         // dW_l = dZ_l^T H_{l-1} (H_{-1} = X)
         const bf16 *hin_t = l > 0 ? q->ht[l - 1] : q->xt;
         GemmArgs w;
         EK_MCUDA(gemm_args(w, q->dzt[l], B, hin_t, B, HID, DIM_IN[l], B, q->err, q->wait_cycles), "operand maps");
         w.c = q->g + q->off_w[l];
         w.ldc = DIM_IN[l];
-        EK_MCUDA(gemm<EPI_F32>(w, q->stream), "weight-gradient GEMM");
+        EK_MCUDA(l > 0 ? gemm<EPI_F32>(w, q->side, false) : gemm<EPI_F32>(w, q->stream), "weight-gradient GEMM");
         up = q->dz[l];
         ldup = HID;
     }
@@ -621,8 +637,10 @@ int backward(ek_mlp *q, bool counted) {
         s.rows[l] = DIM_OUT[l];
         rows += DIM_OUT[l];
     }
-    EK_MCUDA(ek::launch_pdl(bias_grads, dim3((rows * 32 + 255) / 256), dim3(256), 0, q->stream, s, B),
-             "bias gradients");
+    bias_grads<<<(rows * 32 + 255) / 256, 256, 0, q->side>>>(s, B);
+    EK_MCUDA(cudaGetLastError(), "bias gradients");
+    EK_MCUDA(cudaEventRecord(q->joined, q->side), "gradient stream");
+    EK_MCUDA(cudaStreamWaitEvent(q->stream, q->joined, 0), "gradient stream");
     q->launches += 9;
     return EK_OK;
 }
@@ -651,9 +669,9 @@ int train_iteration(ek_mlp *q, float lr) {
     if (rc == EK_OK) rc = backward(q, true);
     if (rc != EK_OK) return rc;
     const int64_t n4 = q->nparam / 4;  // every layer's weights and biases come in fours
-    EK_MCUDA(ek::launch_pdl(adam_update, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, q->stream, (float4 *)q->p,
-                            (const float4 *)q->g, (float4 *)q->m, (float4 *)q->v, n4, lr, 0.9f, 0.999f, 1e-8f, q->step),
-             "Adam");
+    adam_update<<<(unsigned)((n4 + 255) / 256), 256, 0, q->stream>>>((float4 *)q->p, (const float4 *)q->g, (float4 *)q->m,
+                                                                    (float4 *)q->v, n4, lr, 0.9f, 0.999f, 1e-8f, q->step);
+    EK_MCUDA(cudaGetLastError(), "Adam");
     ++q->launches;
     return cast_all(q, true);
 }
@@ -729,6 +747,10 @@ int ek_mlp_create(int32_t batch, uint64_t seed, ek_mlp **out) {
         al.push_back({(void **)&q->dzt[l], (size_t)B * HID * 2});
     }
     cudaError_t e = cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&q->side, cudaStreamNonBlocking);
+    for (cudaEvent_t &ev : q->ready)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&q->joined, cudaEventDisableTiming);
     for (auto &a : al) {
         if (e == cudaSuccess) e = cudaMalloc(a.p, a.bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(*a.p, 0, a.bytes, q->stream);
@@ -758,6 +780,7 @@ int ek_mlp_create(int32_t batch, uint64_t seed, ek_mlp **out) {
 int ek_mlp_destroy(ek_mlp *q) {
     if (!q) return ek::ctx_fail(EK_ERR_INVALID, "null MLP");
     if (q->stream) cudaStreamSynchronize(q->stream);
+    if (q->side) cudaStreamSynchronize(q->side);
     if (q->graph) cudaGraphExecDestroy(q->graph);
     void *bufs[] = {q->p, q->g, q->m, q->v, q->x, q->xt, q->t, q->y, q->dy, q->dyt, q->step, q->base, q->err,
                     q->xs, q->ts, q->idx, q->loss, q->ey};
@@ -772,6 +795,10 @@ int ek_mlp_destroy(ek_mlp *q) {
         for (void *b : b2)
             if (b) cudaFree(b);
     }
+    for (cudaEvent_t ev : q->ready)
+        if (ev) cudaEventDestroy(ev);
+    if (q->joined) cudaEventDestroy(q->joined);
+    if (q->side) cudaStreamDestroy(q->side);
     if (q->stream) cudaStreamDestroy(q->stream);
     delete q;
     return EK_OK;

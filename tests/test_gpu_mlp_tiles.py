@@ -46,3 +46,32 @@ def test_forward_rows(rows):
     # the bar of test_forward_and_gradients_match_oracle
     assert np.linalg.norm(y - ref) < 5e-3 * np.linalg.norm(ref)
     assert np.array_equal(small, again)
+
+
+# the weight gradients run beside the deltas: whatever the overlap, gradients
+# asked for again (outside a graph) and a training run started again (a graph)
+# give the same bits, apart from the loss (summed by atomics)
+@pytest.mark.parametrize("batch", [128, 256, 1024])
+def test_gradient_streams_repeat(batch):
+    import ekpnp.mlp as em
+    import mlp_oracle as mo
+    r = np.random.default_rng(batch)
+    x = r.uniform(-1, 1, (batch, 4)).astype(np.float32)
+    t = r.standard_normal((batch, 512)).astype(np.float32)
+    runs = []
+    for _ in range(2):
+        with em.Mlp(batch=batch, seed=11) as net:
+            p = net.params
+            grads = [net.gradients(x, t)[0] for _ in range(4)]
+            net.set_data(x, t)
+            net.train(40, 1e-3)
+            runs.append((grads, net.params))
+    first = runs[0][0][0]
+    for grads, _ in runs:
+        assert all(np.array_equal(g, first) for g in grads)
+    assert np.array_equal(runs[0][1], runs[1][1])
+    _, ref = mo.loss_and_gradients(p.astype(np.float64), x.astype(np.float64), t.astype(np.float64))
+    # the bar of test_forward_and_gradients_match_oracle
+    for ws, _, bs in em.layer_slices():
+        for part in (ws, bs):
+            assert np.linalg.norm(first[part] - ref[part]) < 2e-2 * np.linalg.norm(ref[part])
