@@ -52,8 +52,12 @@ constexpr int REFS_TPB = 256;
 // queue[1] counts the blocks that found the list empty; the last of them
 // puts both back to zero for the next launch (every other block has made its
 // last claim by then), so the queue needs no reset between launches or graph
-// replays.
-constexpr int TILE_CHUNK = 4;
+// replays.  Runs of two: the second tile's rows were half read by the first,
+// while runs of four left narrow channels too few runs for one wave of blocks
+// (128 channels of 16 columns, ~2000 tiles for 592 blocks, on B200: 46 us a
+// launch in runs of four, 33 of two, 33 of one; 64 channels up to 512 wide, a
+// step: 367, 364, 372 us).
+constexpr int TILE_CHUNK = 2;
 
 template <typename S, bool FIRST, bool EE, int TXB, int MINB>
 __global__ void __launch_bounds__(TXB, MINB)
