@@ -71,6 +71,9 @@ ChanF make_chanf(const Chan &c) {
 namespace {
 
 constexpr int TPB = 128;
+// FP16 channels of at least this many nodes, not narrower than a block, prefetch (prefetch_rows)
+constexpr size_t PREFETCH_NODES = (size_t)1 << 20;
+constexpr int PREFETCH_AHEAD = 148;  // blocks
 // Blocks per SM the register allocation must allow: 4 blocks of 128 threads,
 // 128 registers, which the update of two nodes a thread takes without
 // spilling; 512 threads then have 54 loads of populations in flight each.
@@ -78,10 +81,34 @@ constexpr int TPB = 128;
 #define EK_LBM_MIN_BLOCKS 4
 #endif
 
+// The populations of the block `ahead` blocks on (one row of each of
+// the 27 planes, a plane a thread) into L2: that block's loads then wait for L2
+// and not for DRAM.  FP16 storage only: its 54 loads a thread bring half the
+// bytes of FP32's, so 16 warps an SM don't keep enough of them in flight.
+// One block per SM ahead is a quarter of a wave: at 592 ahead and more the rows
+// come too early and leave L2 again.  B200, FP16 4096 x 1024, a pass of 20 steps:
+// 3.93 ms; 74 ahead 3.78, 148 3.73, 222 3.72, 592 3.76, 1184 4.02.
+// FP32 4096 x 1024: 4.12, 148 ahead 4.11, 592 4.55.
+template <typename S>
+__device__ __forceinline__ void prefetch_rows(const ChanF &k, const S *__restrict__ src, int ahead) {
+    const int p = threadIdx.x;
+    if (p >= 27) return;
+    const int b = blockIdx.y * gridDim.x + blockIdx.x + ahead, y = b / gridDim.x;
+    const int x = (b - y * gridDim.x) * 2 * blockDim.x;
+    if (y >= k.ny || x >= k.nxp) return;
+    const S *a = src + (size_t)p * k.plane + (size_t)y * k.nxp + x;
+    // rows are padded to 32 columns: 16-byte addresses and sizes
+    const uint32_t bytes = (uint32_t)min(2 * (int)blockDim.x, k.nxp - x) * sizeof(S);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(bytes) : "memory");
+}
+
 template <typename S, bool FIRST, bool EE>
 __global__ void __launch_bounds__(TPB, EK_LBM_MIN_BLOCKS)
 step_shifted(const ChanF k, const S *__restrict__ src, S *__restrict__ dst, double *__restrict__ fields, bool mom,
-             int sbuf, bool wait) {
+             int sbuf, bool wait, int ahead) {
+    if constexpr (sizeof(S) == 2) {
+        if (ahead > 0) prefetch_rows(k, src, ahead);
+    }
     const int x = 2 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= k.nx || y >= k.ny) return;
     node_shifted<S, FIRST, EE, float2>(k, src, dst, fields, x, y, mom, sbuf, wait);
@@ -117,12 +144,16 @@ cudaError_t step_typed(const ChanF &k, const void *src, void *dst, double *field
     const S *a = (const S *)src;
     S *b = (S *)dst;
     const bool wait = chain != CHAIN_NONE, pdl = chain == CHAIN_NEXT;
+    // both buffers of 2^20 nodes are 113 MB: below that L2 holds them (512 x 600 FP16,
+    // a step: 33.0 us, 33.1 with the prefetch; 1024 x 1024: 64.5, 64.0)
+    int ahead = 0;
+    if (sizeof(S) == 2 && t.y == 1 && (size_t)k.nx * k.ny >= PREFETCH_NODES) ahead = PREFETCH_AHEAD;
     if (first) {
-        if (ee) return launch_chain(pdl, step_shifted<S, true, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
-        return launch_chain(pdl, step_shifted<S, true, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+        if (ee) return launch_chain(pdl, step_shifted<S, true, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait, ahead);
+        return launch_chain(pdl, step_shifted<S, true, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait, ahead);
     }
-    if (ee) return launch_chain(pdl, step_shifted<S, false, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
-    return launch_chain(pdl, step_shifted<S, false, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait);
+    if (ee) return launch_chain(pdl, step_shifted<S, false, true>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait, ahead);
+    return launch_chain(pdl, step_shifted<S, false, false>, g, t, 0, s, k, a, b, fields, mom, sbuf, wait, ahead);
 }
 
 __global__ void __launch_bounds__(256) row_refs(const Chan c, const double *__restrict__ fields, int qf, int qp,

@@ -90,3 +90,22 @@ def test_one_launch_solve_equals_the_passes(nx, ny, storage):
             out.append(ch.get_fields())
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+# at and around 2^20 nodes, with partial last blocks (odd widths, one column over) and the last rows
+@pytest.mark.parametrize("nx,ny", [(1024, 1023), (1024, 1024), (1025, 1033), (131, 8100), (8192, 130)])
+def test_prefetching_step_equals_the_pipelined_one(nx, ny):
+    """The large FP16 step that prefetches later blocks' rows gives the bits of
+    the TMA-fed kernel."""
+    import ekpnp
+    p, init = start(nx, ny, 2)
+    out = []
+    for form in ("plain", "tma"):
+        with ekpnp.Channel(p) as ch:
+            ch.set_lbm_kernel(form)
+            ch.set_fields(**init)
+            ch.init_equilibrium()
+            ch.step(6)
+            out.append(ch.get_fields())
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
