@@ -48,6 +48,8 @@ struct ek_ctx {
     ek::Rates *rates_dev = nullptr;
     ek::Rates rates{};
     ek::PoissonPlan pp{};
+    float *pivf_alloc = nullptr;     // what pp.pivf and pp.specf point into
+    float2 *specf_alloc = nullptr;
     int cluster[2] = {0, 0};              // blocks of the one-launch solve, FP64 and FP32 form (0: separate passes)
     ek::Chan chan{};
     int64_t steps = 0;

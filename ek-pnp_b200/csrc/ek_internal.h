@@ -274,8 +274,8 @@ struct PoissonPlan {
     // FP32 form (shifted storage): modes >= 1 in FP32, the zero mode in FP64
     // (column 0 of spec); null where the form is not set up
     float2 *twf;                // FP32 row transforms: per-pass twiddle tables (< nx entries)
-    float *pivf;                // n x mp pivots, FP32
-    float2 *specf;              // n x mp spectrum, FP32
+    float *pivf;                // n x mp pivots, FP32 (mode 1 starts a sector)
+    float2 *specf;              // n x mp spectrum, FP32 (the same from nx = 32 on)
     double *rowmean;            // n row means of the last solve: the offset removed before the FP32 FFT
     int *rowmean_ok;            // set by the first solve's pass C; before it pass A takes exact means
     // Field planes of the shifted-storage step (every shifted context; the
