@@ -297,7 +297,7 @@ int upload(T **dst, const std::vector<T> &v, cudaStream_t s) {
     return EK_OK;
 }
 
-// LBM + three Poisson passes; the FP32 form's column solve is two kernels.
+// LBM + three Poisson passes.
 int launches_per_step(const ek_batch *) { return 4; }
 
 void release_graph(ek_batch *b) {
