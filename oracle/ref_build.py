@@ -218,7 +218,7 @@ def build_all_shims(names=None) -> list:
 
 
 def available() -> bool:
-    return os.path.isdir(REF_DIR) and shutil.which(NVCC) is not None
+    return os.path.isfile(os.path.join(REF_DIR, "main.cu")) and shutil.which(NVCC) is not None
 
 
 if __name__ == "__main__":
