@@ -50,6 +50,7 @@ __device__ __forceinline__ int brev(int i, int lg) { return (int)(__brev((unsign
 // term by term, one output a thread: nx r products instead of the nx^2 of
 // the direct transform, which took 211 us (inverse 263) at 1000 x 257 on B200
 // against 10 (9) us here.  All roots are powers of the nx-th root from the table.
+constexpr int MIXED_MAX_NX = 2048;  // longest (ek_create, ek_poisson_noalloc)
 struct Radices {
     int n;
     int r[11];  // nx <= 2048 = 4^5 2
@@ -1377,11 +1378,15 @@ cudaError_t row_limits(F *f, size_t smem) {
 }
 }  // namespace
 
-// Only the kernels of this length: an attribute call loads its kernel.
+// Only the kernels of this length: an attribute call loads its kernel.  A limit
+// belongs to the kernel, not to the plan: it is the same whatever plan sets it,
+// so that plans of several lengths can be alive together (the mixed form's
+// kernels serve all its lengths and take that of the longest).
 cudaError_t poisson_set_smem_limits(const PoissonPlan &pp) {
     if (use_r16(pp)) EK_ROW_DISPATCH(pp.log2nx, limits(pp.specf != nullptr))
-    const cudaError_t e = row_limits(fwd_rows, poisson_smem_bytes_f64(pp.nx));
-    return e == cudaSuccess ? row_limits(inv_rows, poisson_smem_bytes_f64(pp.nx)) : e;
+    const size_t most = poisson_smem_bytes_f64(MIXED_MAX_NX);
+    const cudaError_t e = row_limits(fwd_rows, most);
+    return e == cudaSuccess ? row_limits(inv_rows, most) : e;
 }
 
 cudaError_t batch_set_smem_limits(int block) {
