@@ -1273,6 +1273,10 @@ int cluster_row_threads(const PoissonPlan &pp) {
     while (t < CL_THREADS && 4 * t < pp.nx) t *= 2;
     return t;
 }
+// The most that any plan asks for: 512 threads of 16 FP64 points (two buffers of
+// mixed length: 64 KB).  The kernels' limit, whatever plan sets it: one kernel
+// serves all mixed lengths, several of which may be alive.
+constexpr size_t CLUSTER_SMEM = (size_t)CL_THREADS * 16 * sizeof(double2);
 size_t cluster_smem(const PoissonPlan &pp, bool f32) {
     const int per = CL_THREADS / cluster_row_threads(pp);
     return (size_t)per * pp.nx * (f32 ? sizeof(float2) : (use_r16(pp) ? 1 : 2) * sizeof(double2));
@@ -1300,8 +1304,8 @@ int poisson_cluster_blocks(const PoissonPlan &pp, bool f32) {
     if ((size_t)pp.nx * pp.ny > most || tridiag_modes(pp.n, pp.nx, f32) == 0) return 0;
     const void *fn = cluster_kernel(pp, f32);
     const size_t smem = cluster_smem(pp, f32);
-    if (!fn || smem > 200 * 1024) return 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (!fn || smem > CLUSTER_SMEM) return 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;

@@ -32,8 +32,11 @@ def same(got, want):
         assert np.array_equal(got[k], want[k]), k
 
 
-# above the node count up to which a channel solves in one launch: the row passes
-@pytest.mark.parametrize("a,b", [((2047, 12), (10, 1700)), ((1000, 257), (6, 3000))])
+# the row passes (above 16384 nodes), and the solve in one launch (below): 1000 x
+# 16 and 100 x 150 ask for 64,000 and 51,200 bytes of shared memory there, 300 x 50
+# for 38,400, 10 x 101 for 5,120
+@pytest.mark.parametrize("a,b", [((2047, 12), (10, 1700)), ((1000, 257), (6, 3000)), ((1000, 16), (10, 101)),
+                                 ((100, 150), (10, 101)), ((300, 50), (10, 101)), ((2047, 12), (10, 101))])
 @pytest.mark.parametrize("storage", [0, 1], ids=["f64", "f32"])
 def test_two_lengths_alive(a, b, storage):
     """Steps of two channels in turn, the longer rows' channel created first
