@@ -357,8 +357,9 @@ cudaError_t launch_batch_residual(const Chan *chans, double *const *fields, doub
 // Record an error message for ek_last_error() (ek_api.cu).
 void set_last_error(const char *msg);
 // Shared-memory attributes of the row kernels: of one plan's length (its sizes and
-// specf set), of a batch's.
+// specf set), of all FP64 passes (ek_poisson_noalloc), of a batch's.
 cudaError_t poisson_set_smem_limits(const PoissonPlan &pp);
+cudaError_t poisson_load_f64();
 cudaError_t batch_set_smem_limits(int block);
 
 }  // namespace ek

@@ -21,8 +21,9 @@
 // and clears the spectrum region it uses before use.
 //
 // First call on a device: the call looks up the device addresses of the arrays
-// (cudaGetSymbolAddress, once per device, with that device current) and
-// caches them together with the identity of the device's current context.
+// (cudaGetSymbolAddress, once per device, with that device current),
+// caches them together with the identity of the device's current context and
+// loads every kernel that a later call may launch.
 // Make that first call before any stream capture begins.  After
 // cudaDeviceReset the library's module is loaded again into a new context and
 // the arrays move; the next call sees the new context and looks the addresses
@@ -95,31 +96,6 @@ cudaError_t current_ctx_id(unsigned long long *id) {
     return cudaSuccess;
 }
 
-// Device addresses of the arrays for the current device: looked up on the
-// first call and again whenever the device's context has changed.
-cudaError_t scratch_for(int dev, Scratch *out) {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    Scratch &s = g_scratch[dev];
-    unsigned long long id = 0;
-    const cudaError_t have = current_ctx_id(&id);
-    const bool checkable = have != cudaErrorNotSupported;  // no driver entry point: no check
-    if (s.ready && checkable && (have != cudaSuccess || s.ctx_id != id)) s.ready = false;
-    if (!s.ready) {
-        cudaError_t e;
-        if ((e = cudaGetSymbolAddress((void **)&s.spec, g_na_spec)) != cudaSuccess) return e;
-        if ((e = cudaGetSymbolAddress((void **)&s.piv, g_na_piv)) != cudaSuccess) return e;
-        if ((e = cudaGetSymbolAddress((void **)&s.rhs, g_na_rhs)) != cudaSuccess) return e;
-        if ((e = cudaGetSymbolAddress((void **)&s.tw, g_na_tw)) != cudaSuccess) return e;
-        if ((e = cudaGetSymbolAddress((void **)&s.wall, g_na_wall)) != cudaSuccess) return e;
-        // the lookups above made the device's context current if it was not
-        if (checkable && (e = current_ctx_id(&id)) != cudaSuccess) return e;
-        s.ctx_id = id;
-        s.ready = true;
-    }
-    *out = s;
-    return cudaSuccess;
-}
-
 // Twiddles exp(-2 pi i k/nx) and the uniform wall rows.
 __global__ void na_tables(int nx, double zlo, double zhi, double2 *tw, double *wall) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nx; k += gridDim.x * blockDim.x) {
@@ -171,6 +147,45 @@ __global__ void na_efield(int nx, int ny, double dx, double dy, const double *__
     const size_t r = (size_t)y * nx;
     ex[r + x] = 0.5 * (psi[r + xm] - psi[r + xp]) / dx;
     ey[r + x] = 0.5 * (psi[(size_t)(yc - 1) * nx + x] - psi[(size_t)(yc + 1) * nx + x]) / dy;
+}
+
+// Every kernel a call may launch: loading one takes device memory, which the calls
+// after the first must not (the first at 256 x 64, then 1024 x 40: 2 MB less free).
+cudaError_t load_kernels() {
+    const void *fns[] = {(const void *)na_tables, (const void *)na_pivots, (const void *)na_rhs, (const void *)na_efield};
+    cudaFuncAttributes at;
+    for (const void *f : fns) {
+        const cudaError_t e = cudaFuncGetAttributes(&at, f);
+        if (e != cudaSuccess) return e;
+    }
+    return poisson_load_f64();
+}
+
+// Device addresses of the arrays for the current device: looked up, and the
+// kernels loaded, on the first call and again whenever the device's context has
+// changed.
+cudaError_t scratch_for(int dev, Scratch *out) {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    Scratch &s = g_scratch[dev];
+    unsigned long long id = 0;
+    const cudaError_t have = current_ctx_id(&id);
+    const bool checkable = have != cudaErrorNotSupported;  // no driver entry point: no check
+    if (s.ready && checkable && (have != cudaSuccess || s.ctx_id != id)) s.ready = false;
+    if (!s.ready) {
+        cudaError_t e;
+        if ((e = cudaGetSymbolAddress((void **)&s.spec, g_na_spec)) != cudaSuccess) return e;
+        if ((e = cudaGetSymbolAddress((void **)&s.piv, g_na_piv)) != cudaSuccess) return e;
+        if ((e = cudaGetSymbolAddress((void **)&s.rhs, g_na_rhs)) != cudaSuccess) return e;
+        if ((e = cudaGetSymbolAddress((void **)&s.tw, g_na_tw)) != cudaSuccess) return e;
+        if ((e = cudaGetSymbolAddress((void **)&s.wall, g_na_wall)) != cudaSuccess) return e;
+        if ((e = load_kernels()) != cudaSuccess) return e;
+        // the lookups above made the device's context current if it was not
+        if (checkable && (e = current_ctx_id(&id)) != cudaSuccess) return e;
+        s.ctx_id = id;
+        s.ready = true;
+    }
+    *out = s;
+    return cudaSuccess;
 }
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
@@ -225,7 +240,6 @@ extern "C" int ek_poisson_noalloc(const ek_params *p, const double *cp, const do
     pp.tw = sc.tw;
     pp.piv = sc.piv;
     pp.spec = sc.spec;
-    if ((e = poisson_set_smem_limits(pp)) != cudaSuccess) return na_fail(EK_ERR_CUDA, cudaGetErrorString(e));
     Chan c{};
     c.nx = nx;
     c.ny = ny;

@@ -1393,6 +1393,22 @@ cudaError_t poisson_set_smem_limits(const PoissonPlan &pp) {
     return e == cudaSuccess ? row_limits(inv_rows, most) : e;
 }
 
+// Every kernel of the FP64 passes, whatever the channel: loaded, limits set.
+cudaError_t poisson_load_f64() {
+    cudaError_t e = cudaSuccess;
+#define EK_CASE(K) \
+    if (e == cudaSuccess) e = RowLaunch<K>::limits(false);
+    EK_ROW_CASES(EK_CASE)
+#undef EK_CASE
+    const size_t most = poisson_smem_bytes_f64(MIXED_MAX_NX);
+    if (e == cudaSuccess) e = row_limits(fwd_rows, most);
+    if (e == cudaSuccess) e = row_limits(inv_rows, most);
+    cudaFuncAttributes at;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, tridiag);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, tridiag_part);
+    return e;
+}
+
 cudaError_t batch_set_smem_limits(int block) {
     const size_t smem = (size_t)block * 16 * sizeof(float2);
     cudaError_t e;

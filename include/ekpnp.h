@@ -285,7 +285,8 @@ int ek_field_pointers(ek_ctx *ctx, double **out8, int32_t *pitch);
  * and ny <= 65535; larger channels return EK_ERR_TOO_LARGE before any work
  * is queued.  All calls on a GPU share the scratch: calls that overlap on the
  * GPU race, so order them on one stream.  The first call on a device looks up
- * the scratch addresses; make it before any stream capture.  After
+ * the scratch addresses and loads every kernel (which takes device memory, later
+ * calls of whatever size take none); make it before any stream capture.  After
  * cudaDeviceReset the next call looks them up again (also outside a capture).
  * A launch error pending from the caller's earlier work is cleared on entry;
  * on EK_ERR_CUDA part of the call may be queued and psi, ex, ey are undefined.
