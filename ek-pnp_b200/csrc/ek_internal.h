@@ -38,6 +38,32 @@ __device__ __forceinline__ void pdl_wait() {
 #endif
 }
 
+// Loads of what the kernel just before in the stream wrote.  A chained kernel starts
+// while that one still runs, so these values are not constant over its lifetime:
+// the read-only path (__ldg, a const __restrict__ parameter) is not for them, and
+// nothing may move their loads above pdl_wait().  Volatile statements stay in order,
+// wait included.
+__device__ __forceinline__ double ld_fresh(const double *p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_fresh(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_fresh(const float2 *p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_fresh(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 // Field-plane bytes (right-hand side + psi of every channel stepped together)
 // that the evict_last stores may pin, out of the 126 MB L2: above it the
 // planes are stored the ordinary way.

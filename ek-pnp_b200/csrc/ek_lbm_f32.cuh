@@ -187,6 +187,22 @@ template <typename S> struct Row<float2, S> {
     }
     static __device__ __forceinline__ void put(S *p, const RowAt &r, float2 v) { st_pair(at(p, r.x), v); }
 };
+// The same of psi's fluctuation plane, which the kernel before writes (ld_fresh).
+template <typename V> struct PsiRow;
+template <> struct PsiRow<float> {
+    static __device__ __forceinline__ float own(const float *p, const RowAt &r) { return ld_fresh(at(p, r.x)); }
+    static __device__ __forceinline__ float left(const float *p, const RowAt &r) { return ld_fresh(at(p, r.xm)); }
+    static __device__ __forceinline__ float right(const float *p, const RowAt &r) { return ld_fresh(at(p, r.xp)); }
+};
+template <> struct PsiRow<float2> {
+    static __device__ __forceinline__ float2 own(const float *p, const RowAt &r) { return ld_fresh((const float2 *)at(p, r.x)); }
+    static __device__ __forceinline__ float2 left(const float *p, const RowAt &r) {
+        return make_float2(ld_fresh(at(p, r.xm)), ld_fresh(at(p, r.x)));
+    }
+    static __device__ __forceinline__ float2 right(const float *p, const RowAt &r) {
+        return make_float2(ld_fresh(at(p, r.xr)), ld_fresh(at(p, r.xp)));
+    }
+};
 // Per-x arrays without padding (wall frames, lifting): element by element.
 template <typename V> struct PerX;
 template <> struct PerX<float> {
@@ -432,13 +448,13 @@ __device__ __forceinline__ void efield_shifted(const ChanF &k, const double *__r
 // gpu_efield / gpu_bc (poisson.cu:145-174).
 template <typename V>
 __device__ __forceinline__ void efield_f32(const ChanF &k, const Cols &c, int y, V *ex, V *ex_tot, V *ey) {
-    using R = Row<V, float>;
+    using R = PsiRow<V>;
     const RowAt r = row_at(c, y, k.nxp);
     const V dx = vsub(R::left(k.psif, r), R::right(k.psif, r));
     *ex = vscale(k.half_inv_dxf, dx);
     *ex_tot = vaxpy(k.half_inv_dxf, dx, bc<V>(k.ext_xf));
     const int yc = y == 0 ? 1 : (y == k.ny - 1 ? k.ny - 2 : y);
-    const float eym = (float)((__ldg(k.psim + yc - 1) - __ldg(k.psim + yc + 1)) * k.half_inv_dy);
+    const float eym = (float)((ld_fresh(k.psim + yc - 1) - ld_fresh(k.psim + yc + 1)) * k.half_inv_dy);
     const V dn = R::own(k.psif, row_at(c, yc - 1, k.nxp)), up = R::own(k.psif, row_at(c, yc + 1, k.nxp));
     *ey = vaxpy(k.half_inv_dyf, vsub(dn, up), bc<V>(eym));
 }

@@ -154,12 +154,13 @@ __device__ __forceinline__ double by_cs2_cfl(double v, const Chan &c) {
 
 // Field E at a node from psi: central differences with periodic x, and the
 // wall rows take the adjacent row's Ey (gpu_efield + gpu_bc, poisson.cu:145-174).
-__device__ __forceinline__ void efield_at(const double *__restrict__ psi, const Chan &c, int x,
+// psi: of the kernel before (ld_fresh).
+__device__ __forceinline__ void efield_at(const double *psi, const Chan &c, int x,
                                           int y, int xm, int xp, double *ex, double *ey) {
     const size_t r = (size_t)y * c.nxp;
-    *ex = div_by(0.5 * (__ldg(psi + r + xm) - __ldg(psi + r + xp)), c.dx, c.inv.dx);
+    *ex = div_by(0.5 * (ld_fresh(psi + r + xm) - ld_fresh(psi + r + xp)), c.dx, c.inv.dx);
     const int yc = y == 0 ? 1 : (y == c.ny - 1 ? c.ny - 2 : y);
-    *ey = div_by(0.5 * (__ldg(psi + (size_t)(yc - 1) * c.nxp + x) - __ldg(psi + (size_t)(yc + 1) * c.nxp + x)), c.dy,
+    *ey = div_by(0.5 * (ld_fresh(psi + (size_t)(yc - 1) * c.nxp + x) - ld_fresh(psi + (size_t)(yc + 1) * c.nxp + x)), c.dy,
                  c.inv.dy);
 }
 

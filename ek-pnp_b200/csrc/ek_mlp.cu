@@ -321,7 +321,7 @@ __global__ void pad_inputs(const float4 *__restrict__ x, int n, int rows, uint4 
 // 32 x 64 tile, transposed through shared memory so that both results are
 // stored in runs (one row a block with scattered transposed stores: 5.3 us
 // against 3.3 us at 256 rows, B200).
-__global__ void __launch_bounds__(256) mse_grad(const float *__restrict__ y, const float *__restrict__ t, int B,
+__global__ void __launch_bounds__(256) mse_grad(const float *y, const float *__restrict__ t, int B,
                                                 bf16 *__restrict__ dy, bf16 *__restrict__ dyt,
                                                 double *__restrict__ loss, const int64_t *__restrict__ step,
                                                 const int64_t *__restrict__ base) {
@@ -330,12 +330,20 @@ __global__ void __launch_bounds__(256) mse_grad(const float *__restrict__ y, con
     const int b0 = blockIdx.x * 32, j0 = blockIdx.y * 64;
     const float scale = 2.0f / ((float)B * (float)OUT);
     double acc = 0.0;
+    // the thread's 8 elements: targets (of the gather, kernels ago) before the wait,
+    // outputs (of the kernel before) after it, all of them before the first store
+    const size_t o0 = (size_t)(b0 + (threadIdx.x >> 6)) * OUT + j0 + (threadIdx.x & 63);
+    float tv[8], yv[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) tv[e] = __ldg(t + o0 + (size_t)(e * 4) * OUT);
     ek::pdl_wait();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) yv[e] = ek::ld_fresh(y + o0 + (size_t)(e * 4) * OUT);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const int r = e * 4 + (threadIdx.x >> 6), c = threadIdx.x & 63;
-        const size_t o = (size_t)(b0 + r) * OUT + j0 + c;
-        const float d = y[o] - t[o];
+        const size_t o = o0 + (size_t)(e * 4) * OUT;
+        const float d = yv[e] - tv[e];
         acc += (double)d * (double)d;
         const bf16 g = __float2bfloat16_rn(scale * d);
         dy[o] = g;
@@ -661,9 +669,9 @@ int cast_all(ek_mlp *q, bool advance) {
 }
 
 int train_iteration(ek_mlp *q, float lr) {
-    EK_MCUDA(ek::launch_pdl(gather_batch, dim3(q->B), dim3(256), 0, q->stream, q->xs, q->ts, q->idx, q->step, q->base,
-                            q->B, q->x, q->xt, q->t),
-             "batch gather");
+    // an ordinary launch: it reads the step count that the iteration before ends with
+    gather_batch<<<q->B, 256, 0, q->stream>>>(q->xs, q->ts, q->idx, q->step, q->base, q->B, q->x, q->xt, q->t);
+    EK_MCUDA(cudaGetLastError(), "batch gather");
     ++q->launches;
     int rc = forward(q);
     if (rc == EK_OK) rc = backward(q, true);

@@ -163,13 +163,13 @@ __device__ double2 *mixed_fft(double2 *a, double2 *b, int nx, const Radices &f, 
 
 // Pass A of any length: row pair (2 pair + 1, 2 pair + 2) of the right-hand side
 // -> spectra, by threads t < T of a group (z: 2 nx points of shared memory).
-__device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Radices &f, const double *__restrict__ rhs,
+__device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Radices &f, const double *rhs,
                                                  int nxp, int pair, bool live, double2 *z0, int t, int T, int ns = 0) {
     const int nx = pp.nx, j0 = 2 * pair, j1 = j0 + 1;
     const bool two = live && j1 < pp.n;
     const double *r0 = rhs + (size_t)(j0 + 1) * nxp;
     const double *r1 = rhs + (size_t)(j1 + 1) * nxp;
-    for (int x = t; x < nx; x += T) z0[x] = make_double2(live ? r0[x] : 0.0, two ? r1[x] : 0.0);
+    for (int x = t; x < nx; x += T) z0[x] = make_double2(live ? ld_fresh(r0 + x) : 0.0, two ? ld_fresh(r1 + x) : 0.0);
     const double2 *z = mixed_fft<false>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
     if (!live) return;
     // unpack the two real-input spectra: A = (Z[m] + conj Z[-m])/2, B = (Z[m] - conj Z[-m])/(2i)
@@ -182,7 +182,7 @@ __device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Ra
 }
 
 __global__ void __launch_bounds__(PTPB)
-fwd_rows(const PoissonPlan pp, const Radices f, const double *__restrict__ rhs, int nxp) {
+fwd_rows(const PoissonPlan pp, const Radices f, const double *rhs, int nxp) {
     extern __shared__ double2 sm[];
     pdl_wait();
     fwd_rows_any_len(pp, f, rhs, nxp, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
@@ -285,7 +285,7 @@ template <int K> struct RowCfg {
 // block) below pair_end: right-hand side -> spectra.  The first radix-16 pass
 // runs on the values as loaded.
 template <int K>
-__device__ __forceinline__ void fwd_rows_f64_k(const PoissonPlan &pp, const double *__restrict__ rhs, int nxp, int pair_base,
+__device__ __forceinline__ void fwd_rows_f64_k(const PoissonPlan &pp, const double *rhs, int nxp, int pair_base,
                                                int pair_end, double2 *sm, int ns = 0) {
     using S = fft16::Shape<K>;
     constexpr int N = S::N, T = S::T;
@@ -296,7 +296,7 @@ __device__ __forceinline__ void fwd_rows_f64_k(const PoissonPlan &pp, const doub
     const double *r0 = rhs + (size_t)(j0 + 1) * nxp + t, *r1 = r0 + nxp;
     double2 x[16];
 #pragma unroll
-    for (int v = 0; v < 16; ++v) x[v] = make_double2(live ? __ldg(r0 + v * T) : 0.0, two ? __ldg(r1 + v * T) : 0.0);
+    for (int v = 0; v < 16; ++v) x[v] = make_double2(live ? ld_fresh(r0 + v * T) : 0.0, two ? ld_fresh(r1 + v * T) : 0.0);
     fft16::fwd_pass_store<K, 1>(x, s, t, p, pp.tw);
     fft16::rows_sync(ns);
     fft16::fwd_rest<K, 2>(s, t, p, pp.tw, ns);
@@ -347,7 +347,7 @@ __device__ __forceinline__ void inv_rows_f64_k(const PoissonPlan &pp, int nxp, d
 
 template <int K>
 __global__ void __launch_bounds__(RowCfg<K>::block, 512 / RowCfg<K>::block)
-fwd_rows_f64(const PoissonPlan pp, const double *__restrict__ rhs, int nxp) {
+fwd_rows_f64(const PoissonPlan pp, const double *rhs, int nxp) {
     extern __shared__ double2 sm[];
     pdl_wait();
     fwd_rows_f64_k<K>(pp, rhs, nxp, blockIdx.x * RowCfg<K>::per, (pp.n + 1) / 2, sm);
@@ -422,7 +422,7 @@ __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan
         const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            const float4 u = live ? __ldg(q0 + v) : none, w = two ? __ldg(q1 + v) : none;
+            const float4 u = live ? ld_fresh(q0 + v) : none, w = two ? ld_fresh(q1 + v) : none;
             x[4 * v] = make_float2(u.x, w.x);
             x[4 * v + 1] = make_float2(u.y, w.y);
             x[4 * v + 2] = make_float2(u.z, w.z);
@@ -431,8 +431,8 @@ __device__ __forceinline__ void fwd_rows_f32_k(const PoissonPlan &pp, const Chan
     } else {
 #pragma unroll
         for (int v = 0; v < 16; ++v)
-            x[v] = make_float2(live ? __ldg(pp.rhsf + (r0 + (unsigned)(v * T))) : 0.0f,
-                               two ? __ldg(pp.rhsf + (r1 + (unsigned)(v * T))) : 0.0f);
+            x[v] = make_float2(live ? ld_fresh(pp.rhsf + (r0 + (unsigned)(v * T))) : 0.0f,
+                               two ? ld_fresh(pp.rhsf + (r1 + (unsigned)(v * T))) : 0.0f);
     }
     auto less_offset = [&](bool sum) {
 #pragma unroll
@@ -794,9 +794,10 @@ __device__ __forceinline__ double2 rn_sub_mul(double2 v, double2 d, double c) {
 
 // One block of the partitioned solve on a spectrum of type C (pivots R), with
 // segments of at most LMAX rows.  Rows past the end carry zero pivots and values,
-// which pass zero on in either direction, so the sweeps need no row test.
+// which pass zero on in either direction, so the sweeps need no row test.  spec, of
+// the kernel before, is not __restrict__: the wait is in here.
 template <int LMAX, typename R, typename C>
-__device__ __forceinline__ void tridiag_part_len(const R *__restrict__ piv, C *__restrict__ spec, int n, int nx,
+__device__ __forceinline__ void tridiag_part_len(const R *__restrict__ piv, C *spec, int n, int nx,
                                                  size_t mp, R dy2, int M, int m_base, typename SharedOf<R>::type &sh) {
     const int mlast = nx / 2;
     const int tid = threadIdx.x, mode = tid & (M - 1), S = TB_THREADS / M, seg = tid / M;
@@ -858,7 +859,7 @@ __device__ __forceinline__ void tridiag_part_len(const R *__restrict__ piv, C *_
 // The form for the segments' length: a sweep unrolled to 16 rows costs a channel
 // of 7 rows a segment more than twice its arithmetic (FP64 most of all).
 template <typename R, typename C>
-__device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *__restrict__ spec, int n, int nx,
+__device__ __forceinline__ void tridiag_part_gen(const R *__restrict__ piv, C *spec, int n, int nx,
                                                  size_t mp, R dy2, int M, int m_base, typename SharedOf<R>::type &sh) {
     const int S = TB_THREADS / M, L = (n + S - 1) / S;
     if (L <= 4) tridiag_part_len<4, R, C>(piv, spec, n, nx, mp, dy2, M, m_base, sh);
@@ -1034,7 +1035,7 @@ solve_cluster_f32(const PoissonPlan pp, const Chan c, double *__restrict__ psi, 
 // threads a row pair).
 template <int K>
 __global__ void __launch_bounds__(CL_THREADS, 1)
-solve_cluster_f64(const PoissonPlan pp, const Radices f, int T, const Chan c, const double *__restrict__ rhs,
+solve_cluster_f64(const PoissonPlan pp, const Radices f, int T, const Chan c, const double *rhs,
                   double *__restrict__ psi, int M) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ ClusterShared sh;
