@@ -26,6 +26,8 @@
 //          row 1's rest populations after they were overwritten in place).
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "ek_internal.h"
 
 namespace ek {
@@ -42,10 +44,21 @@ constexpr int STEP_BLOCKS = 4;
 // twenty-odd instructions.  A node divides by the constants some thirty times,
 // and the chain of them was most of a small channel's launch: without
 // them 10 x 101 takes 15.3 us a step, not 17.6, and 4096 x 1024 442 us, not 489
-// (B200).  A non-finite a gives a NaN.
+// (B200).  For constants from 2^-500 to 2^500 (recips_ok): then the reciprocal is
+// normal, and the remainder of any a from 2^-969 on is exact (smaller ones, of no
+// weight beside populations of order one, may lose their last bit); a quotient
+// that overflows, in a run that has blown up, is a NaN and not an infinity.
+// PLAIN divides: other constants, and the fields a caller reads.
+template <bool PLAIN>
 __device__ __forceinline__ double div_by(double a, double b, double ib) {
+    if (PLAIN) return a / b;
     const double q = __dmul_rn(a, ib);
     return __fma_rn(__fma_rn(-b, q, a), ib, q);
+}
+bool recips_ok(const Chan &c) {
+    for (double b : {c.cs2, c.cfl, c.dx, c.dy, std::fabs(c.eps)})
+        if (!(b >= 0x1p-500 && b <= 0x1p500)) return false;
+    return true;
 }
 
 __device__ __forceinline__ double sum9(const double t[9]) {
@@ -113,10 +126,11 @@ __device__ __forceinline__ void equilibria(double dens, double tux, double tuy, 
 }
 
 // Guo forcing populations (LBM.cu:556-572); e_i = c_i/CFL.
+template <bool PLAIN>
 __device__ __forceinline__ void guo_pops(double ux, double uy, double fx, double fy, const Chan &c, double s[9]) {
     const double coe0 = c.inv.w0_cs2, coes = c.inv.ws_cs2, coed = c.inv.wd_cs2;
     const double ci = c.inv.cfl;
-    const double qx = div_by((ci * ux) * ci, c.cs2, c.inv.cs2), qy = div_by((ci * uy) * ci, c.cs2, c.inv.cs2);
+    const double qx = div_by<PLAIN>((ci * ux) * ci, c.cs2, c.inv.cs2), qy = div_by<PLAIN>((ci * uy) * ci, c.cs2, c.inv.cs2);
     s[0] = coe0 * (-ux * fx - uy * fy);
     s[1] = coes * (((ci - ux) + qx) * fx - uy * fy);
     s[2] = coes * (-ux * fx + ((ci - uy) + qy) * fy);
@@ -148,19 +162,21 @@ __device__ __forceinline__ void relax(const double t[9], const double e[9], doub
 }
 
 // v / cs2 / cfl
+template <bool PLAIN>
 __device__ __forceinline__ double by_cs2_cfl(double v, const Chan &c) {
-    return div_by(div_by(v, c.cs2, c.inv.cs2), c.cfl, c.inv.cfl);
+    return div_by<PLAIN>(div_by<PLAIN>(v, c.cs2, c.inv.cs2), c.cfl, c.inv.cfl);
 }
 
 // Field E at a node from psi: central differences with periodic x, and the
 // wall rows take the adjacent row's Ey (gpu_efield + gpu_bc, poisson.cu:145-174).
 // psi: of the kernel before (ld_fresh).
+template <bool PLAIN>
 __device__ __forceinline__ void efield_at(const double *psi, const Chan &c, int x,
                                           int y, int xm, int xp, double *ex, double *ey) {
     const size_t r = (size_t)y * c.nxp;
-    *ex = div_by(0.5 * (ld_fresh(psi + r + xm) - ld_fresh(psi + r + xp)), c.dx, c.inv.dx);
+    *ex = div_by<PLAIN>(0.5 * (ld_fresh(psi + r + xm) - ld_fresh(psi + r + xp)), c.dx, c.inv.dx);
     const int yc = y == 0 ? 1 : (y == c.ny - 1 ? c.ny - 2 : y);
-    *ey = div_by(0.5 * (ld_fresh(psi + (size_t)(yc - 1) * c.nxp + x) - ld_fresh(psi + (size_t)(yc + 1) * c.nxp + x)), c.dy,
+    *ey = div_by<PLAIN>(0.5 * (ld_fresh(psi + (size_t)(yc - 1) * c.nxp + x) - ld_fresh(psi + (size_t)(yc + 1) * c.nxp + x)), c.dy,
                  c.inv.dy);
 }
 
@@ -198,7 +214,7 @@ __device__ __forceinline__ void gather_f64(const Chan &c, const double *__restri
 // wall's row-1 pull.  `moments` is a run-time flag: as a template parameter it
 // gave two bodies whose multiply-adds the compiler fused differently, so a
 // step that wrote the moments could round differently from one that did not.
-template <bool FIRST, bool EXPLICIT_E, typename I>
+template <bool FIRST, bool EXPLICIT_E, bool PLAIN, typename I>
 __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_raw[9], double tt_raw[9],
                                          const double *__restrict__ src, double *__restrict__ dst,
                                          double *__restrict__ fields, int x, int y, bool moments) {
@@ -231,15 +247,15 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
         Ex = __ldg(fields + F_EX * pl + o);
         Ey = __ldg(fields + F_EY * pl + o);
     } else {
-        efield_at(fields + F_PSI * pl, c, x, y, xm, xp, &Ex, &Ey);
+        efield_at<PLAIN>(fields + F_PSI * pl, c, x, y, xm, xp, &Ex, &Ey);
     }
     double forcex = 0.0, forcey = 0.0;
     if (c.flags & EK_FLAG_FORCE) {  // the expression commented out at LBM.cu:388-389
         forcex = c.f_charge * (charge - temp) * (Ex + c.ext_x) + c.exf;
         forcey = c.f_charge * (charge - temp) * Ey;
     }
-    double ux = rhoinv * (div_by(ft[1] + ft[5] + ft[8] - (ft[3] + ft[6] + ft[7]), c.cfl, c.inv.cfl) + forcex * c.dt * 0.5);
-    double uy = rhoinv * (div_by(ft[2] + ft[5] + ft[6] - (ft[4] + ft[7] + ft[8]), c.cfl, c.inv.cfl) + forcey * c.dt * 0.5);
+    double ux = rhoinv * (div_by<PLAIN>(ft[1] + ft[5] + ft[8] - (ft[3] + ft[6] + ft[7]), c.cfl, c.inv.cfl) + forcex * c.dt * 0.5);
+    double uy = rhoinv * (div_by<PLAIN>(ft[2] + ft[5] + ft[6] - (ft[4] + ft[7] + ft[8]), c.cfl, c.inv.cfl) + forcey * c.dt * 0.5);
     if (lo) {
         // lower wall: minus the velocity of row 1 (LBM.cu:402-443)
         double fm[9];
@@ -247,8 +263,8 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
         if (FIRST) own9(sf, pl, o1, fm);
         else pull9(sf, pl, nxp, x, 1, xm, xp, 0, 2, fm);
         const double rhoinvm = 1.0 / sum9(fm);
-        ux = -rhoinvm * (div_by(fm[1] + fm[5] + fm[8] - (fm[3] + fm[6] + fm[7]), c.cfl, c.inv.cfl) + forcex * c.dt * 0.5);
-        uy = -rhoinvm * (div_by(fm[2] + fm[5] + fm[6] - (fm[4] + fm[7] + fm[8]), c.cfl, c.inv.cfl) + forcey * c.dt * 0.5);
+        ux = -rhoinvm * (div_by<PLAIN>(fm[1] + fm[5] + fm[8] - (fm[3] + fm[6] + fm[7]), c.cfl, c.inv.cfl) + forcex * c.dt * 0.5);
+        uy = -rhoinvm * (div_by<PLAIN>(fm[2] + fm[5] + fm[6] - (fm[4] + fm[7] + fm[8]), c.cfl, c.inv.cfl) + forcey * c.dt * 0.5);
     }
     if (moments) {
         fields[F_RHO * pl + o] = rho;
@@ -259,27 +275,27 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
     }
     if (!lo && !hi) {
         // Poisson right-hand side with the Dirichlet lifting (poisson.cu:228-241)
-        double v = div_by(-c.f_charge * (charge - temp), c.eps, c.inv.eps);
+        double v = div_by<PLAIN>(-c.f_charge * (charge - temp), c.eps, c.inv.eps);
         if (y == 1) v = v - c.zlo[x] / c.dy / c.dy;
         if (y == c.ny - 2) v = v - c.zhi[x] / c.dy / c.dy;
         fields[F_RHS * pl + o] = v;
     }
 
     // ion equilibria in the drift velocities u + K E (LBM.cu:479-552)
-    const double omusq = 1.0 - div_by(0.5 * (ux * ux + uy * uy), c.cs2, c.inv.cs2);
-    const double omusq_c = 1.0 - div_by(0.5 * ((ux + c.mob_p * Ex) * (ux + c.mob_p * Ex) + (uy + c.mob_p * Ey) * (uy + c.mob_p * Ey)),
+    const double omusq = 1.0 - div_by<PLAIN>(0.5 * (ux * ux + uy * uy), c.cs2, c.inv.cs2);
+    const double omusq_c = 1.0 - div_by<PLAIN>(0.5 * ((ux + c.mob_p * Ex) * (ux + c.mob_p * Ex) + (uy + c.mob_p * Ey) * (uy + c.mob_p * Ey)),
                                          c.cs2, c.inv.cs2);
-    const double omusq_cn = 1.0 - div_by(0.5 * ((ux + c.mob_n * Ex) * (ux + c.mob_n * Ex) + (uy + c.mob_n * Ey) * (uy + c.mob_n * Ey)),
+    const double omusq_cn = 1.0 - div_by<PLAIN>(0.5 * ((ux + c.mob_n * Ex) * (ux + c.mob_n * Ex) + (uy + c.mob_n * Ey) * (uy + c.mob_n * Ey)),
                                          c.cs2, c.inv.cs2);
     {
         double e[9], out[9];
-        equilibria(charge, by_cs2_cfl(ux + c.mob_p * Ex, c), by_cs2_cfl(uy + c.mob_p * Ey, c),
+        equilibria(charge, by_cs2_cfl<PLAIN>(ux + c.mob_p * Ex, c), by_cs2_cfl<PLAIN>(uy + c.mob_p * Ey, c),
                    omusq_c, omusq_c, e);
         relax(ht, e, c.r.wcp, c.r.wcm, out);
         double *dh = dst + 9 * pl;
 #pragma unroll
         for (int d = 0; d < 9; ++d) dh[d * pl + o] = out[d];
-        equilibria(temp, by_cs2_cfl(ux + c.mob_n * Ex, c), by_cs2_cfl(uy + c.mob_n * Ey, c),
+        equilibria(temp, by_cs2_cfl<PLAIN>(ux + c.mob_n * Ex, c), by_cs2_cfl<PLAIN>(uy + c.mob_n * Ey, c),
                    omusq_cn, (c.flags & EK_FLAG_REST_QUIRK) ? omusq : omusq_cn, e);
         relax(tt, e, c.r.wtp, c.r.wtm, out);
         double *dt_ = dst + 18 * pl;
@@ -309,8 +325,8 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
     }
     // fluid: equilibrium, Guo source, TRT (LBM.cu:468-803)
     double e[9], fpop[9];
-    equilibria(rho, by_cs2_cfl(ux, c), by_cs2_cfl(uy, c), omusq, omusq, e);
-    guo_pops(ux, uy, forcex, forcey, c, fpop);
+    equilibria(rho, by_cs2_cfl<PLAIN>(ux, c), by_cs2_cfl<PLAIN>(uy, c), omusq, omusq, e);
+    guo_pops<PLAIN>(ux, uy, forcex, forcey, c, fpop);
     const double sp = c.r.sp, sm = c.r.sm, dt = c.dt;
     double src9[9];
     src9[0] = sp * fpop[0];
@@ -330,7 +346,7 @@ __device__ __forceinline__ void node_f64(const Chan &c, double ft[9], double ht_
     for (int d = 0; d < 9; ++d) df[d * pl + o] = out[d] + dt * src9[d];
 }
 
-template <bool FIRST, bool EXPLICIT_E, typename I>
+template <bool FIRST, bool EXPLICIT_E, bool PLAIN, typename I>
 __global__ void __launch_bounds__(TPB, STEP_BLOCKS)
 step_f64(const Chan c, const double *__restrict__ src, double *__restrict__ dst,
          double *__restrict__ fields, bool moments, bool wait) {
@@ -340,7 +356,7 @@ step_f64(const Chan c, const double *__restrict__ src, double *__restrict__ dst,
     double ft[9], ht[9], tt[9];
     gather_f64<FIRST, I>(c, src, x, y, ft, ht, tt);
     if (wait) pdl_wait();  // the populations are in flight; psi comes from the kernel before (StepChain)
-    node_f64<FIRST, EXPLICIT_E, I>(c, ft, ht, tt, src, dst, fields, x, y, moments);
+    node_f64<FIRST, EXPLICIT_E, PLAIN, I>(c, ft, ht, tt, src, dst, fields, x, y, moments);
 }
 
 __global__ void rates_kernel(ek_params p, Rates *out) {
@@ -381,7 +397,7 @@ init_f64(const Chan c, double *__restrict__ pops, const double *__restrict__ fie
         Ex = fields[F_EX * pl + o];
         Ey = fields[F_EY * pl + o];
     } else {
-        efield_at(fields + F_PSI * pl, c, x, y, xm, xp, &Ex, &Ey);
+        efield_at<true>(fields + F_PSI * pl, c, x, y, xm, xp, &Ex, &Ey);
     }
     const double omusq = 1.0 - 0.5 * (ux * ux + uy * uy) / c.cs2;
     const double omusq_c = 1.0 - 0.5 * ((ux + c.mob_p * Ex) * (ux + c.mob_p * Ex) + (uy + c.mob_p * Ey) * (uy + c.mob_p * Ey)) / c.cs2;
@@ -406,7 +422,7 @@ __global__ void __launch_bounds__(TPB) efield_f64(const Chan c, double *__restri
     if (x >= c.nx) return;
     const int xm = x == 0 ? c.nx - 1 : x - 1, xp = x + 1 == c.nx ? 0 : x + 1;
     double Ex, Ey;
-    efield_at(fields + F_PSI * c.plane, c, x, y, xm, xp, &Ex, &Ey);
+    efield_at<true>(fields + F_PSI * c.plane, c, x, y, xm, xp, &Ex, &Ey);
     const size_t o = (size_t)y * c.nxp + x;
     fields[F_EX * c.plane + o] = Ex;
     fields[F_EY * c.plane + o] = Ey;
@@ -447,10 +463,11 @@ cudaError_t launch_step_f64(const Chan &c, const double *src, double *dst, doubl
     const dim3 t(tx, TPB / tx), g((c.nx + tx - 1) / tx, (c.ny + TPB / tx - 1) / (TPB / tx));
     const bool wait = chain != CHAIN_NONE, pdl = chain == CHAIN_NEXT;
     // 32-bit offsets while the 27 population planes fit 2^32 elements
-    const bool i32 = (size_t)27 * c.plane < ((size_t)1 << 32);
-#define EK_STEP(F, E)                                                                                               \
-    return i32 ? launch_chain(pdl, step_f64<F, E, uint32_t>, g, t, 0, s, c, src, dst, fields, moments, wait)    \
-               : launch_chain(pdl, step_f64<F, E, size_t>, g, t, 0, s, c, src, dst, fields, moments, wait)
+    const bool i32 = (size_t)27 * c.plane < ((size_t)1 << 32), plain = !recips_ok(c);
+#define EK_STEP(F, E)                                                                                                      \
+    return plain ? launch_chain(pdl, step_f64<F, E, true, size_t>, g, t, 0, s, c, src, dst, fields, moments, wait)     \
+           : i32 ? launch_chain(pdl, step_f64<F, E, false, uint32_t>, g, t, 0, s, c, src, dst, fields, moments, wait)  \
+                 : launch_chain(pdl, step_f64<F, E, false, size_t>, g, t, 0, s, c, src, dst, fields, moments, wait)
     switch ((first ? 2 : 0) | (explicit_e ? 1 : 0)) {
         case 0: EK_STEP(false, false);
         case 1: EK_STEP(false, true);
