@@ -161,8 +161,36 @@ __device__ double2 *mixed_fft(double2 *a, double2 *b, int nx, const Radices &f, 
     return a;
 }
 
+// The same for a prime nx by itself: the one pass of nx terms.  In the mixed form's
+// kernel it took that kernel's registers (64 a thread against 40) and with them a
+// second wave of blocks: 257 x 1200 237 us a step against 191 (B200).
+template <bool INV>
+__device__ __forceinline__ double2 *prime_fft(const double2 *in, double2 *out, int nx, const double2 *__restrict__ tw, int t,
+                                              int T) {
+    __syncthreads();
+    for (int m = t; m < nx; m += T) {
+        double2 acc = in[0];
+        int idx = 0;
+        for (int q = 1; q < nx; ++q) {
+            idx += m;
+            if (idx >= nx) idx -= nx;
+            acc = cadd(acc, cmul(in[q], root<INV>(tw, idx)));
+        }
+        out[m] = acc;
+    }
+    __syncthreads();
+    return out;
+}
+template <bool INV, bool PRIME>
+__device__ __forceinline__ double2 *any_fft(double2 *a, double2 *b, int nx, const Radices &f, const double2 *__restrict__ tw,
+                                            int t, int T, int ns) {
+    if constexpr (PRIME) return prime_fft<INV>(a, b, nx, tw, t, T);
+    else return mixed_fft<INV>(a, b, nx, f, tw, t, T, ns);
+}
+
 // Pass A of any length: row pair (2 pair + 1, 2 pair + 2) of the right-hand side
 // -> spectra, by threads t < T of a group (z: 2 nx points of shared memory).
+template <bool PRIME = false>
 __device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Radices &f, const double *rhs,
                                                  int nxp, int pair, bool live, double2 *z0, int t, int T, int ns = 0) {
     const int nx = pp.nx, j0 = 2 * pair, j1 = j0 + 1;
@@ -170,7 +198,7 @@ __device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Ra
     const double *r0 = rhs + (size_t)(j0 + 1) * nxp;
     const double *r1 = rhs + (size_t)(j1 + 1) * nxp;
     for (int x = t; x < nx; x += T) z0[x] = make_double2(live ? ld_fresh(r0 + x) : 0.0, two ? ld_fresh(r1 + x) : 0.0);
-    const double2 *z = mixed_fft<false>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
+    const double2 *z = any_fft<false, PRIME>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
     if (!live) return;
     // unpack the two real-input spectra: A = (Z[m] + conj Z[-m])/2, B = (Z[m] - conj Z[-m])/(2i)
     double2 *s0 = pp.spec + (size_t)j0 * pp.mp, *s1 = pp.spec + (size_t)j1 * pp.mp;
@@ -181,11 +209,12 @@ __device__ __forceinline__ void fwd_rows_any_len(const PoissonPlan &pp, const Ra
     }
 }
 
+template <bool PRIME>
 __global__ void __launch_bounds__(PTPB)
 fwd_rows(const PoissonPlan pp, const Radices f, const double *rhs, int nxp) {
     extern __shared__ double2 sm[];
     pdl_wait();
-    fwd_rows_any_len(pp, f, rhs, nxp, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
+    fwd_rows_any_len<PRIME>(pp, f, rhs, nxp, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
 }
 
 // Pass B: one thread per x-mode, Thomas sweep over the n interior rows.
@@ -230,6 +259,7 @@ __device__ __forceinline__ void write_walls(double *__restrict__ psi, const doub
 }
 
 // Pass C of any length: spectra of a row pair -> psi rows.
+template <bool PRIME = false>
 __device__ __forceinline__ void inv_rows_any_len(const PoissonPlan &pp, const Radices &f, int nxp, double *__restrict__ psi,
                                                  int pair, bool live, double2 *z0, int t, int T, int ns = 0) {
     const int nx = pp.nx, j0 = 2 * pair, j1 = j0 + 1;
@@ -242,7 +272,7 @@ __device__ __forceinline__ void inv_rows_any_len(const PoissonPlan &pp, const Ra
         z0[m] = make_double2(a.x - b.y, a.y + b.x);
         if (m != 0 && 2 * m != nx) z0[nx - m] = make_double2(a.x + b.y, -a.y + b.x);
     }
-    const double2 *z = mixed_fft<true>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
+    const double2 *z = any_fft<true, PRIME>(z0, z0 + nx, nx, f, pp.tw, t, T, ns);
     if (!live) return;
     const double inv = 1.0 / (double)nx;
     double *p0 = psi + (size_t)(j0 + 1) * nxp, *p1 = psi + (size_t)(j1 + 1) * nxp;
@@ -252,12 +282,13 @@ __device__ __forceinline__ void inv_rows_any_len(const PoissonPlan &pp, const Ra
     }
 }
 
+template <bool PRIME>
 __global__ void __launch_bounds__(PTPB)
 inv_rows(const PoissonPlan pp, const Radices f, const Chan c, double *__restrict__ psi) {
     extern __shared__ double2 sm[];
     pdl_wait();
     write_walls(psi, c.zlo, c.zhi, pp.nx, c.ny, c.nxp, blockIdx.x, gridDim.x, blockDim.x);
-    inv_rows_any_len(pp, f, c.nxp, psi, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
+    inv_rows_any_len<PRIME>(pp, f, c.nxp, psi, blockIdx.x, true, sm, threadIdx.x, blockDim.x);
 }
 
 // ---- radix-16 row transforms (power-of-two nx >= 16) -----------------------
@@ -1157,9 +1188,16 @@ Radices radices(int nx) {
         }
     return f;
 }
-// Threads of a mixed-form block: a butterfly of radix 4 a thread and pass.
+// Whether a length has a prime factor above 5, whose pass takes one thread an output.
+bool prime_radix(int nx) {
+    const Radices f = radices(nx);
+    return f.n > 0 && f.r[f.n - 1] > 5;
+}
+// Threads of a mixed-form block: a butterfly of radix 4 a thread and pass; with a
+// prime radix, whose pass outlasts the others, one output a thread (131 x 400 in 32
+// threads 83 us a step on B200, in 160 41).
 int mixed_threads(int nx) {
-    const int t = (nx / 4 + 31) / 32 * 32;
+    const int t = ((prime_radix(nx) ? nx : nx / 4) + 31) / 32 * 32;
     return t < 32 ? 32 : (t > PTPB ? PTPB : t);
 }
 
@@ -1238,10 +1276,19 @@ cudaError_t poisson_pass_f64_at(int pass, const PoissonPlan &pp, const Chan &c, 
     const Radices f = radices(pp.nx);
     const dim3 grid((pp.n + 1) / 2), block(mixed_threads(pp.nx));
     const size_t smem = poisson_smem_bytes_f64(pp.nx);
+    if (f.n == 1 && f.r[0] > 5) {
+        // Long blocks that fill the GPU are launched the ordinary way: scheduled early
+        // they pile up on the SMs that the kernel before leaves first.  B200, us a
+        // step, chained against ordinary: 131 x 200 27.6, 27.2; 131 x 400 38.8, 33.4;
+        // 449 x 400 243, 181; but 131 x 101 22.1, 26.2 and 113 x 300 26.4, 29.2.
+        const bool chain = pdl && !(pp.nx > 128 && (pp.n + 1) / 2 > 74);
+        if (pass == 0) return launch_chain(chain, fwd_rows<true>, grid, block, smem, s, pp, f, rhs, c.nxp);
+        return launch_chain(chain, inv_rows<true>, grid, block, smem, s, pp, f, c, psi);
+    }
     if (pass == 0)
-        return pdl ? launch_chain(true, fwd_rows, grid, block, smem, s, pp, f, rhs, c.nxp)
-                   : launch_pdl(fwd_rows, grid, block, smem, s, pp, f, rhs, c.nxp);
-    return launch_chain(pdl, inv_rows, grid, block, smem, s, pp, f, c, psi);
+        return pdl ? launch_chain(true, fwd_rows<false>, grid, block, smem, s, pp, f, rhs, c.nxp)
+                   : launch_pdl(fwd_rows<false>, grid, block, smem, s, pp, f, rhs, c.nxp);
+    return launch_chain(pdl, inv_rows<false>, grid, block, smem, s, pp, f, c, psi);
 }
 
 int poisson_tridiag_modes(int n, int nx) { return tridiag_modes(n, nx, true); }
@@ -1270,8 +1317,9 @@ namespace {
 // Threads a row pair and shared memory of the cluster's blocks.
 int cluster_row_threads(const PoissonPlan &pp) {
     if (use_r16(pp)) return pp.nx >> 4;
+    const int per = prime_radix(pp.nx) ? 1 : 4;  // points a thread (mixed_threads)
     int t = 32;
-    while (t < CL_THREADS && 4 * t < pp.nx) t *= 2;
+    while (t < CL_THREADS && per * t < pp.nx) t *= 2;
     return t;
 }
 // The most that any plan asks for: 512 threads of 16 FP64 points (two buffers of
@@ -1303,6 +1351,11 @@ int poisson_cluster_blocks(const PoissonPlan &pp, bool f32) {
     // against 13.5, 100 x 100 14.7 against 16.1, 300 x 60 16.2 against 18.2
     const size_t most = use_r16(pp) ? (size_t)8192 : (size_t)16384;
     if ((size_t)pp.nx * pp.ny > most || tridiag_modes(pp.n, pp.nx, f32) == 0) return 0;
+    // a prime radix makes the row pairs the solve's bulk, which 16 SMs hold while each
+    // has one of them or 256 of their points: 113 x 60 22.7 us against 23.5, 131 x 33
+    // 0.81 of the passes' time, 131 x 48 1.05, 251 x 60 1.46
+    const int share = ((pp.n + 1) / 2 + 15) / 16;  // row pairs a block
+    if (!use_r16(pp) && prime_radix(pp.nx) && share > 1 && share * pp.nx > 256) return 0;
     const void *fn = cluster_kernel(pp, f32);
     const size_t smem = cluster_smem(pp, f32);
     if (!fn || smem > CLUSTER_SMEM) return 0;
@@ -1381,6 +1434,13 @@ cudaError_t row_limits(F *f, size_t smem) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, ROW_SMEM_PERCENT);
     return e;
 }
+cudaError_t mixed_limits() {
+    const size_t most = poisson_smem_bytes_f64(MIXED_MAX_NX);
+    cudaError_t e = row_limits(fwd_rows<false>, most);
+    if (e == cudaSuccess) e = row_limits(fwd_rows<true>, most);
+    if (e == cudaSuccess) e = row_limits(inv_rows<false>, most);
+    return e == cudaSuccess ? row_limits(inv_rows<true>, most) : e;
+}
 }  // namespace
 
 // Only the kernels of this length: an attribute call loads its kernel.  A limit
@@ -1389,9 +1449,7 @@ cudaError_t row_limits(F *f, size_t smem) {
 // kernels serve all its lengths and take that of the longest).
 cudaError_t poisson_set_smem_limits(const PoissonPlan &pp) {
     if (use_r16(pp)) EK_ROW_DISPATCH(pp.log2nx, limits(pp.specf != nullptr))
-    const size_t most = poisson_smem_bytes_f64(MIXED_MAX_NX);
-    const cudaError_t e = row_limits(fwd_rows, most);
-    return e == cudaSuccess ? row_limits(inv_rows, most) : e;
+    return mixed_limits();
 }
 
 // Every kernel of the FP64 passes, whatever the channel: loaded, limits set.
@@ -1401,9 +1459,7 @@ cudaError_t poisson_load_f64() {
     if (e == cudaSuccess) e = RowLaunch<K>::limits(false);
     EK_ROW_CASES(EK_CASE)
 #undef EK_CASE
-    const size_t most = poisson_smem_bytes_f64(MIXED_MAX_NX);
-    if (e == cudaSuccess) e = row_limits(fwd_rows, most);
-    if (e == cudaSuccess) e = row_limits(inv_rows, most);
+    if (e == cudaSuccess) e = mixed_limits();
     cudaFuncAttributes at;
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, tridiag);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, tridiag_part);
