@@ -1000,8 +1000,8 @@ __global__ void __launch_bounds__(TB_THREADS, 2) tridiag_modes_f32(const Poisson
 // ---- a small channel's whole solve in one launch ------------------------------
 //
 // One cluster of up to 16 blocks runs passes A, B and C with the cluster's
-// barrier between them: three launches' boundaries cost a channel of a few
-// thousand nodes more than the passes' work.  Each block takes an equal share of
+// barrier between them: three launches' boundaries cost a channel of a thousand
+// nodes more than the passes' work.  Each block takes an equal share of
 // the row pairs, then every gridDim.x-th group of modes; the spectrum goes
 // through L2.  The arithmetic is that of the separate passes, group for group, so
 // the bits are theirs.  On larger channels 16 SMs are too few
@@ -1062,8 +1062,8 @@ solve_cluster_f32(const PoissonPlan pp, const Chan c, double *__restrict__ psi, 
         }
 }
 
-// FP64: K = log2 nx of the radix-16 transforms, 0 for any other length (T
-// threads a row pair).
+// FP64: K = 4 for nx = 16 (radix-16 transforms), 0 for the mixed lengths (T threads a
+// row pair).
 template <int K>
 __global__ void __launch_bounds__(CL_THREADS, 1)
 solve_cluster_f64(const PoissonPlan pp, const Radices f, int T, const Chan c, const double *rhs,
@@ -1330,35 +1330,46 @@ size_t cluster_smem(const PoissonPlan &pp, bool f32) {
     const int per = CL_THREADS / cluster_row_threads(pp);
     return (size_t)per * pp.nx * (f32 ? sizeof(float2) : (use_r16(pp) ? 1 : 2) * sizeof(double2));
 }
-// The kernel of a plan: nx = 16 to 256, or a length of the mixed form in FP64.
+// The kernel of a plan (poisson_cluster_blocks): FP64 nx = 16 or a length of the mixed
+// form, FP32 nx = 16 to 128.
 const void *cluster_kernel(const PoissonPlan &pp, bool f32) {
-    if (!use_r16(pp)) return f32 ? nullptr : (const void *)solve_cluster_f64<0>;
+    if (!f32) return use_r16(pp) ? (const void *)solve_cluster_f64<4> : (const void *)solve_cluster_f64<0>;
     switch (pp.log2nx) {
-#define EK_CASE(K) \
-    case K: return f32 ? (const void *)solve_cluster_f32<K> : (const void *)solve_cluster_f64<K>;
-        EK_CASE(4) EK_CASE(5) EK_CASE(6) EK_CASE(7) EK_CASE(8)
-#undef EK_CASE
-        default: return nullptr;
+        case 4: return (const void *)solve_cluster_f32<4>;
+        case 5: return (const void *)solve_cluster_f32<5>;
+        case 6: return (const void *)solve_cluster_f32<6>;
+        default: return (const void *)solve_cluster_f32<7>;
     }
 }
 
 }  // namespace
 
 int poisson_cluster_blocks(const PoissonPlan &pp, bool f32) {
-    // microseconds a step on B200, one launch against three: 16 x 101 FP64 10.4 against
-    // 14.0, 64 x 64 12.4 against 12.6 (FP32 13.0 against 14.4), 64 x 128 12.8
-    // against 12.3; 512 x 33 16.9 against 14.4; mixed lengths 10 x 101 11.5
-    // against 13.5, 100 x 100 14.7 against 16.1, 300 x 60 16.2 against 18.2
+    // Time of a step with one launch over that with three, FP64 on B200 unless said
+    // (44 lengths by 6 to 4000 rows, up to 20,000 nodes):
+    // * each block holds its row pairs in one round: 2 x 400 0.89, 2 x 700 1.08, 2 x 4000
+    //   1.58, 30 x 500 0.94, 27 x 700 1.22
+    // * not with column segments of 5 to 8 rows: 10 x 256 0.91, 10 x 300 1.07; 50 x 128
+    //   0.88, 50 x 200 1.07, 50 x 300 0.91; 64 x 200 FP32 1.00, 64 x 300 1.11
+    // * powers of two: FP64 at 16 columns (16 x 128 0.84, 32 x 128 1.04, 64 x 128 1.07, 256
+    //   x 64 1.06), FP32 up to 128 (16 x 128 0.93, 128 x 64 0.98, 256 x 33 1.04, 256 x 12
+    //   1.12)
+    // * other lengths up to 1024: 10 x 101 0.89, 300 x 48 0.88, 1000 x 12 0.98, 1500 x 6
+    //   1.02, 2000 x 6 1.11
+    // * a prime radix makes the row pairs the solve's bulk, which 16 SMs hold while each
+    //   has one of them or 256 of their points: 113 x 64 0.91, 131 x 33 0.81, 131 x 48 1.05,
+    //   251 x 64 1.46
+    const int M = tridiag_modes(pp.n, pp.nx, f32);
     const size_t most = use_r16(pp) ? (size_t)8192 : (size_t)16384;
-    if ((size_t)pp.nx * pp.ny > most || tridiag_modes(pp.n, pp.nx, f32) == 0) return 0;
-    // a prime radix makes the row pairs the solve's bulk, which 16 SMs hold while each
-    // has one of them or 256 of their points: 113 x 60 22.7 us against 23.5, 131 x 33
-    // 0.81 of the passes' time, 131 x 48 1.05, 251 x 60 1.46
+    if ((size_t)pp.nx * pp.ny > most || M == 0) return 0;
     const int share = ((pp.n + 1) / 2 + 15) / 16;  // row pairs a block
+    const int L = (pp.n + TB_THREADS / M - 1) / (TB_THREADS / M);
+    if (share > CL_THREADS / cluster_row_threads(pp) || (L > 4 && L <= 8)) return 0;
+    if (pp.nx > (use_r16(pp) ? (f32 ? 128 : 16) : 1024)) return 0;
     if (!use_r16(pp) && prime_radix(pp.nx) && share > 1 && share * pp.nx > 256) return 0;
     const void *fn = cluster_kernel(pp, f32);
     const size_t smem = cluster_smem(pp, f32);
-    if (!fn || smem > CLUSTER_SMEM) return 0;
+    if (smem > CLUSTER_SMEM) return 0;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -1392,16 +1403,16 @@ cudaError_t poisson_cluster(const PoissonPlan &pp, const Chan &c, bool f32, cons
     const size_t smem = cluster_smem(pp, f32);
     const int M = tridiag_modes(pp.n, pp.nx, f32), T = cluster_row_threads(pp);
     const Radices f = use_r16(pp) ? Radices{} : radices(pp.nx);
-    if (!use_r16(pp)) return launch_attrs(at, 2, solve_cluster_f64<0>, g, t, smem, s, pp, f, T, c, rhs, psi, M);
+    if (!f32)
+        return launch_attrs(at, 2, use_r16(pp) ? solve_cluster_f64<4> : solve_cluster_f64<0>, g, t, smem, s, pp, f, T, c, rhs,
+                            psi, M);
+#define EK_CASE(K) \
+    case K: return launch_attrs(at, 2, solve_cluster_f32<K>, g, t, smem, s, pp, c, psi, write_f64, M);
     switch (pp.log2nx) {
-#define EK_CASE(K)                                                                                                  \
-    case K:                                                                                                         \
-        return f32 ? launch_attrs(at, 2, solve_cluster_f32<K>, g, t, smem, s, pp, c, psi, write_f64, M)             \
-                   : launch_attrs(at, 2, solve_cluster_f64<K>, g, t, smem, s, pp, f, T, c, rhs, psi, M);
-        EK_CASE(4) EK_CASE(5) EK_CASE(6) EK_CASE(7) EK_CASE(8)
-#undef EK_CASE
+        EK_CASE(4) EK_CASE(5) EK_CASE(6) EK_CASE(7)
         default: return cudaErrorInvalidValue;
     }
+#undef EK_CASE
 }
 
 int batch_row_block(int nx_max) { return nx_max <= 1024 ? 64 : 256; }
