@@ -63,10 +63,8 @@ __device__ __forceinline__ C w16(C z) {
         // forward m = 4: -i z; m = 12: +i z; inverse the other way round
         constexpr bool minus_i = (m == 4) != INV;
         return minus_i ? mk(z.y, -z.x) : mk(-z.y, z.x);
-    } else if constexpr ((m & 1) == 0) {
-        static_assert(m & 1, "the odd multiples of pi/4 are rot45's");
-        return z;
     } else {
+        static_assert(m & 1, "the odd multiples of pi/4 are rot45's");
         constexpr double cs[8] = {1.0, C1, R2, S1, 0.0, -S1, -R2, -C1};   // cos(pi j/8), j < 8
         constexpr double sn[8] = {0.0, S1, R2, C1, 1.0, C1, R2, S1};      // sin(pi j/8), j < 8
         constexpr R c = (R)(m < 8 ? cs[m] : -cs[m - 8]);
@@ -171,13 +169,6 @@ struct Shape {
         return o;
     }
 };
-
-// Entries of the twiddle tables of a 2^K-point transform (< 2^K).
-__host__ __device__ constexpr int table_size(int K) {
-    int o = 0;
-    for (int b = K - 4; b >= 1; b -= 4) o += 15 << b;
-    return o;
-}
 
 // Pass twiddle of the table, loaded with an L2 evict_last policy: the tables
 // (32 KB at nx = 4096) are read by every block of every solve, and between

@@ -74,18 +74,6 @@ inline bool keep_l2_fits(size_t bytes) { return bytes <= KEEP_L2_BYTES; }
 // right-hand side written by the LBM step, psi written by the inverse row
 // pass): with keep set they carry an L2 evict_last policy, so the plane
 // stays in L2 while the step's populations stream through it.
-__device__ __forceinline__ void st_field(double *p, double v, bool keep) {
-#if defined(__CUDA_ARCH__)
-    if (keep) {
-        unsigned long long pol;
-        asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-        asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol) : "memory");
-        return;
-    }
-#endif
-    *p = v;
-}
-
 __device__ __forceinline__ void st_field_f(float *p, float v, bool keep) {
 #if defined(__CUDA_ARCH__)
     if (keep) {
@@ -316,7 +304,7 @@ struct PoissonPlan {
     float *psif;
     double *psim;
     double zlo_mean, zhi_mean;  // x-means of the wall potentials (psim of the wall rows)
-    int keep_l2;                // psi stores ask L2 to keep the plane (see st_field)
+    int keep_l2;                // psi stores ask L2 to keep the plane (see st_field_f)
 };
 // pass 0: row FFTs, 1: tridiagonal column solve, 2: inverse row FFTs + walls
 cudaError_t poisson_pass_f64(int pass, const PoissonPlan &pp, const Chan &c, double *fields, cudaStream_t s);

@@ -125,9 +125,6 @@ __device__ __forceinline__ float2 vrcp(float2 a) { return make_float2(1.0f / a.x
 // a + k b, a k for a scalar k
 template <typename V> __device__ __forceinline__ V vaxpy(float k, V b, V a) { return vfma(bc<V>(k), b, a); }
 template <typename V> __device__ __forceinline__ V vscale(float k, V a) { return vmul(bc<V>(k), a); }
-template <typename V> struct Width;
-template <> struct Width<float> { static constexpr int n = 1; };
-template <> struct Width<float2> { static constexpr int n = 2; };
 
 // Columns of a thread's nodes: x, and where its pulls and differences look --
 // xm left of the first node, xr right of the first (the second node itself,

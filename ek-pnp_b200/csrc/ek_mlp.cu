@@ -480,7 +480,6 @@ struct ek_mlp {
     float *xs = nullptr, *ts = nullptr;
     int64_t nrows = 0;
     int *idx = nullptr;
-    int64_t idx_cap = 0;            // iterations the index buffer holds
     double *loss = nullptr;
     int64_t *step = nullptr, *base = nullptr;
     int64_t host_step = 0;
@@ -873,7 +872,6 @@ int ek_mlp_train(ek_mlp *q, int32_t iters, float lr, double *loss_out) {
     if (!q->idx) {
         EK_MCUDA(cudaMalloc(&q->idx, CHUNK * q->B * sizeof(int)), "index buffer");
         EK_MCUDA(cudaMalloc(&q->loss, CHUNK * sizeof(double)), "loss buffer");
-        q->idx_cap = CHUNK;
     }
     if (q->graph && q->graph_lr != lr) {
         cudaGraphExecDestroy(q->graph);
@@ -992,7 +990,7 @@ int ek_mlp_forward(ek_mlp *q, const float *x, int64_t n, float *y) {
         int ldin = INP;
         for (int l = 0; l < 3; ++l) {
             GemmArgs a;
-        EK_MCUDA(gemm_args(a, in, ldin, q->wb[l], DIM_IN[l], rows, HID, DIM_IN[l], q->err, q->wait_cycles), "operand maps");
+            EK_MCUDA(gemm_args(a, in, ldin, q->wb[l], DIM_IN[l], rows, HID, DIM_IN[l], q->err, q->wait_cycles), "operand maps");
             a.bias = q->p + q->off_b[l];
             a.h = q->eh[l & 1];
             a.ldh = HID;
