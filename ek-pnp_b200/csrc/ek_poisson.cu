@@ -1188,6 +1188,8 @@ Radices radices(int nx) {
         }
     return f;
 }
+// A prime length above 5: the kernel of its own (prime_fft).
+bool prime_length(const Radices &f) { return f.n == 1 && f.r[0] > 5; }
 // Whether a length has a prime factor above 5, whose pass takes one thread an output.
 bool prime_radix(int nx) {
     const Radices f = radices(nx);
@@ -1276,7 +1278,7 @@ cudaError_t poisson_pass_f64_at(int pass, const PoissonPlan &pp, const Chan &c, 
     const Radices f = radices(pp.nx);
     const dim3 grid((pp.n + 1) / 2), block(mixed_threads(pp.nx));
     const size_t smem = poisson_smem_bytes_f64(pp.nx);
-    if (f.n == 1 && f.r[0] > 5) {
+    if (prime_length(f)) {
         // Long blocks that fill the GPU are launched the ordinary way: scheduled early
         // they pile up on the SMs that the kernel before leaves first.  B200, us a
         // step, chained against ordinary: 131 x 200 27.6, 27.2; 131 x 400 38.8, 33.4;
@@ -1445,12 +1447,11 @@ cudaError_t row_limits(F *f, size_t smem) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, ROW_SMEM_PERCENT);
     return e;
 }
+template <bool PRIME>
 cudaError_t mixed_limits() {
     const size_t most = poisson_smem_bytes_f64(MIXED_MAX_NX);
-    cudaError_t e = row_limits(fwd_rows<false>, most);
-    if (e == cudaSuccess) e = row_limits(fwd_rows<true>, most);
-    if (e == cudaSuccess) e = row_limits(inv_rows<false>, most);
-    return e == cudaSuccess ? row_limits(inv_rows<true>, most) : e;
+    const cudaError_t e = row_limits(fwd_rows<PRIME>, most);
+    return e == cudaSuccess ? row_limits(inv_rows<PRIME>, most) : e;
 }
 }  // namespace
 
@@ -1460,7 +1461,7 @@ cudaError_t mixed_limits() {
 // kernels serve all its lengths and take that of the longest).
 cudaError_t poisson_set_smem_limits(const PoissonPlan &pp) {
     if (use_r16(pp)) EK_ROW_DISPATCH(pp.log2nx, limits(pp.specf != nullptr))
-    return mixed_limits();
+    return prime_length(radices(pp.nx)) ? mixed_limits<true>() : mixed_limits<false>();
 }
 
 // Every kernel of the FP64 passes, whatever the channel: loaded, limits set.
@@ -1470,7 +1471,8 @@ cudaError_t poisson_load_f64() {
     if (e == cudaSuccess) e = RowLaunch<K>::limits(false);
     EK_ROW_CASES(EK_CASE)
 #undef EK_CASE
-    if (e == cudaSuccess) e = mixed_limits();
+    if (e == cudaSuccess) e = mixed_limits<false>();
+    if (e == cudaSuccess) e = mixed_limits<true>();
     cudaFuncAttributes at;
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, tridiag);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, tridiag_part);
