@@ -1,7 +1,8 @@
 // ek_internal.h -- shared definitions of libekpnp's kernels and C ABI.
 //
 // Device memory of one channel (all planes ny rows x nxp columns, nxp = nx
-// rounded up to 32 so every row starts 256-byte aligned):
+// rounded up to 32, rows of FP64 256-byte aligned; 16 for nx <= 16, where a row of
+// FP16 starts 32-byte aligned):
 //   pops[2]   27 planes each, ping-pong: species-major (fluid f, c+ h, c- t),
 //             then direction 0..8 in the reference numbering (LBM.cu:831-834).
 //             Between steps a buffer holds POST-collision populations; the next
@@ -28,9 +29,9 @@ namespace ek {
 // and the visibility of its writes, then lets the next kernel be scheduled
 // in turn.  A kernel launched the ordinary way passes pdl_wait() at once.
 // Used for a channel's one-wave row transform after the LBM step (measured
-// at 4096 x 1024: -2.6 us a step); on the many-wave LBM kernel the per-block
-// wait cost ~40 us a step, and next to the column pass's fork/join events it
-// cost more than it saved (the batched passes run many waves: not used there).
+// at 4096 x 1024: -2.6 us a step) and for every kernel of a small channel's step
+// (launch_chain); on the many-wave LBM kernel of a large channel the per-block
+// wait cost ~40 us a step (the batched passes run many waves: not used there).
 __device__ __forceinline__ void pdl_wait() {
 #if defined(__CUDA_ARCH__)
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -155,7 +156,12 @@ cudaError_t launch_chain(bool chain, void (*kern)(Exp...), dim3 grid, dim3 block
     return launch_attrs(at, 2, kern, grid, block, smem, s, std::forward<Act>(args)...);
 }
 // Channels of at most this many nodes: every kernel of a step is about one
-// wave of blocks, and the step a chain of launch latencies.
+// wave of blocks, and the step a chain of launch latencies.  Time of a step chained
+// over that with ordinary launches (pass A always early), FP64 and FP32 on B200: 256 x
+// 128 0.69, 0.69; 1000 x 257 0.83, 0.83; 512 x 512 0.82, 0.79.  Above the line powers of
+// two still gain (512 x 1024 0.89, 0.85; 1024 x 1024 0.96, 0.93; 2048 x 2000 1.02,
+// 1.02), but mixed lengths, whose blocks then wait in the others' place, lose: 1000 x
+// 500 1.05, 1.05; 1500 x 800 1.13, 1.16.
 constexpr size_t PDL_NODES = (size_t)1 << 18;
 // The LBM kernel of a step: by itself (many waves of blocks); of a small
 // channel, letting pass A be scheduled early; the same, itself scheduled while

@@ -76,14 +76,15 @@ constexpr size_t PREFETCH_NODES = (size_t)1 << 20;
 constexpr int PREFETCH_AHEAD = 148;  // blocks
 // Blocks per SM the register allocation must allow: 4 blocks of 128 threads,
 // 128 registers, which the update of two nodes a thread takes without
-// spilling; 512 threads then have 54 loads of populations in flight each.
+// spilling; 512 threads then have 45 loads of populations in flight each (a
+// species' three pairs in place and twelve single neighbours).
 #ifndef EK_LBM_MIN_BLOCKS
 #define EK_LBM_MIN_BLOCKS 4
 #endif
 
 // The populations of the block `ahead` blocks on (one row of each of
 // the 27 planes, a plane a thread) into L2: that block's loads then wait for L2
-// and not for DRAM.  FP16 storage only: its 54 loads a thread bring half the
+// and not for DRAM.  FP16 storage only: its 45 loads a thread bring half the
 // bytes of FP32's, so 16 warps an SM don't keep enough of them in flight.
 // One block per SM ahead is a quarter of a wave: at 592 ahead and more the rows
 // come too early and leave L2 again.  B200, FP16 4096 x 1024, a pass of 20 steps:

@@ -160,8 +160,8 @@ template <typename T> __device__ __forceinline__ const T *at(const T *base, uint
     return (const T *)((const char *)base + (size_t)(e * (uint32_t)sizeof(T)));
 }
 
-// Values of a plane's row at the thread's own columns (rows start 64-byte
-// aligned and are padded to a multiple of 32 elements, so the pair is one
+// Values of a plane's row at the thread's own columns (rows are
+// padded to 16 or to a multiple of 32 elements and start 32-byte aligned, so the pair is one
 // access), at their left neighbours and at their right ones.
 template <typename V, typename S> struct Row;
 template <typename S> struct Row<float, S> {

@@ -12,7 +12,7 @@
 // once per channel), for any ny, with no FFT in y:
 //   pass A  per pair of interior rows: real FFT in x (two rows packed as one
 //           complex row; register-blocked radix-16 passes for powers of two
-//           from 16 on, mixed radix otherwise) -> spec[j][m], m = 0..nx/2
+//           from 16 on, mixed radix otherwise, a direct sum for primes) -> spec[j][m], m = 0..nx/2
 //   pass B  per x-mode m: Thomas sweeps down the column, partitioned into row
 //           segments of at most 16 rows held in registers (one thread per
 //           mode for columns taller than 8192 rows)
@@ -49,7 +49,7 @@ __device__ __forceinline__ int brev(int i, int lg) { return (int)(__brev((unsign
 // 2, 3 and 5 are butterflies held by a thread; any other prime r is summed
 // term by term, one output a thread: nx r products instead of the nx^2 of
 // the direct transform, which took 211 us (inverse 263) at 1000 x 257 on B200
-// against 10 (9) us here.  All roots are powers of the nx-th root from the table.
+// against 10.4 (8.4) us here.  All roots are powers of the nx-th root from the table.
 constexpr int MIXED_MAX_NX = 2048;  // longest (ek_create, ek_poisson_noalloc)
 struct Radices {
     int n;

@@ -298,7 +298,8 @@ int ek_poisson_noalloc(const ek_params *p, const double *cp, const double *cn,
  * Phases of a step: 0 = fused LBM kernel, 1 = Poisson pass A (row FFTs),
  * 2 = pass B (tridiagonal y-solve), 3 = pass C (inverse row FFTs).  With
  * profiling on every phase is a kernel by itself; a channel of a few thousand
- * nodes otherwise runs phases 1 to 3 in one launch, to the same bits.
+ * nodes otherwise runs phases 1 to 3 in one launch where that is the faster
+ * form, to the same bits.
  * ek_profile_enable(ctx, 1) resets and starts per-launch timing;
  * ek_profile_read waits for the stream and returns, per phase, the summed
  * kernel milliseconds and the launch count since the last enable. */
@@ -375,8 +376,8 @@ int ek_batch_sync(ek_batch *b);
 int ek_batch_step_count(const ek_batch *b, int64_t *out);
 int ek_batch_launch_count(const ek_batch *b, int64_t *out);
 /* Block shapes of the batched LBM kernel, indices 0 .. EK_BATCH_SHAPES-1:
- * threads per block, the widest tile (a tile is min(width, nx) columns by
- * threads / min(width, nx) rows) and the blocks per SM that the kernel's
+ * threads per block, the widest tile (a tile is min(width, nx) columns, two a
+ * thread, by 2 threads / min(width, nx) rows) and the blocks per SM that the kernel's
  * register allocation allows.  Every shape gives the same bits. */
 #define EK_BATCH_SHAPES 6
 int ek_batch_shape_info(int32_t index, int32_t *threads, int32_t *width, int32_t *blocks_per_sm);
